@@ -25,6 +25,12 @@ struct CpDims {
   int off[TFX_MAX_ORDER];
 };
 
+}  // namespace tfx
+
+#include "mttkrp_f32.cuh"
+
+namespace tfx {
+
 template <class T, int TS>
 __global__ void __launch_bounds__(TFX_THREADS) k_mttkrp(const T* __restrict__ Tt, const T* __restrict__ W, CpDims sh,
                                                         int l, int ksplit, T* __restrict__ part) {
@@ -375,6 +381,8 @@ extern "C" size_t tfx_mttkrp_scratch_bytes(int dtype, int L, const int* dims, in
   const size_t es = dtype == TFX_F64 ? 8 : 4;
   if (mttkrp_short(dims[mode], R))  // partials, then the row-major factors
     return al256((size_t)mttkrp_short_splits(K) * dims[mode] * R * es) + (size_t)S * R * es;
+  CpDims sh;
+  if (dtype == TFX_F32 && !cpdims(sh, L, dims, R)) return mf32::plan(sh, mode, nsm()).total();
   return (size_t)mttkrp_splits(K, dims[mode], R, dtype) * dims[mode] * R * es;
 }
 
@@ -423,6 +431,16 @@ extern "C" int tfx_mttkrp(int dtype, const void* T, int L, const int* dims, int 
       k_sum_parts<double><<<rb, 256, 0, st0>>>((const double*)scratch, n, ks, (double*)out);
     }
     return done("mttkrp_sum");
+  }
+  // (a caller's scratch below what mttkrp_f32 asks for takes the general kernel)
+  if (dtype == TFX_F32) {
+    const mf32::Plan p = mf32::plan(sh, mode, nsm());
+    if (p.total() <= scratch_bytes && ((uintptr_t)scratch & 15) == 0) {
+      if (cudaError_t e = mf32::run(p, (const float*)T, (const float*)W, sh, mode, (float*)out, scratch, st0))
+        return tfx_set_cuda_error(e, "mttkrp_f32");
+      tfx_count_launch(3);
+      return TFX_STATUS_OK;
+    }
   }
   int ks = mttkrp_splits(K, D, R, dtype);
   ks = (int)std::min<size_t>((size_t)ks, scratch_bytes / ((size_t)D * R * es));
