@@ -16,18 +16,7 @@
 
 #include "tfx_capi_internal.h"
 #include "tfx_common.cuh"
-
-namespace tfx {
-
-struct CpDims {
-  int L, R;
-  int d[TFX_MAX_ORDER];
-  int off[TFX_MAX_ORDER];
-};
-
-}  // namespace tfx
-
-#include "mttkrp_f32.cuh"
+#include "mttkrp_gemm.cuh"
 
 namespace tfx {
 
@@ -382,8 +371,8 @@ extern "C" size_t tfx_mttkrp_scratch_bytes(int dtype, int L, const int* dims, in
   if (mttkrp_short(dims[mode], R))  // partials, then the row-major factors
     return al256((size_t)mttkrp_short_splits(K) * dims[mode] * R * es) + (size_t)S * R * es;
   CpDims sh;
-  if (dtype == TFX_F32 && !cpdims(sh, L, dims, R)) return mf32::plan(sh, mode, nsm()).total();
-  return (size_t)mttkrp_splits(K, dims[mode], R, dtype) * dims[mode] * R * es;
+  if (cpdims(sh, L, dims, R)) return 0;
+  return mg::plan((int)es, sh, mode, mode + 1, nsm()).total();
 }
 
 extern "C" int tfx_mttkrp(int dtype, const void* T, int L, const int* dims, int R, const void* W, int mode, void* out,
@@ -432,15 +421,17 @@ extern "C" int tfx_mttkrp(int dtype, const void* T, int L, const int* dims, int 
     }
     return done("mttkrp_sum");
   }
-  // (a caller's scratch below what mttkrp_f32 asks for takes the general kernel)
-  if (dtype == TFX_F32) {
-    const mf32::Plan p = mf32::plan(sh, mode, nsm());
-    if (p.total() <= scratch_bytes && ((uintptr_t)scratch & 15) == 0) {
-      if (cudaError_t e = mf32::run(p, (const float*)T, (const float*)W, sh, mode, (float*)out, scratch, st0))
-        return tfx_set_cuda_error(e, "mttkrp_f32");
-      tfx_count_launch(3);
-      return TFX_STATUS_OK;
-    }
+  // (a caller's scratch below what the GEMM asks for takes the general kernel)
+  const mg::Plan gp = mg::plan((int)es, sh, mode, mode + 1, nsm());
+  if (gp.total() <= scratch_bytes && ((uintptr_t)scratch & 15) == 0) {
+    int nl = 0;
+    const cudaError_t e =
+        dtype == TFX_F32
+            ? mg::run(gp, (const float*)T, (const float*)W, sh, (float*)out, true, scratch, st0, &nl)
+            : mg::run(gp, (const double*)T, (const double*)W, sh, (double*)out, true, scratch, st0, &nl);
+    if (e != cudaSuccess) return tfx_set_cuda_error(e, "mttkrp");
+    tfx_count_launch(nl);
+    return TFX_STATUS_OK;
   }
   int ks = mttkrp_splits(K, D, R, dtype);
   ks = (int)std::min<size_t>((size_t)ks, scratch_bytes / ((size_t)D * R * es));

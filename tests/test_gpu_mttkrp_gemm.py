@@ -1,5 +1,5 @@
-"""The FP32 MTTKRP (``mttkrp``, GaussNewton.py:411-423) at the edges of its
-tiles and plans, against the same product in FP64."""
+"""The MTTKRP (``mttkrp``, GaussNewton.py:411-423) at the edges of its tiles and
+plans, in FP32 and FP64, against the same product in FP64."""
 import numpy as np
 import pytest
 import torch
@@ -14,16 +14,17 @@ SHAPES = [((17, 5, 7), 1), ((33, 31, 32), 8), ((32, 33, 64), 9), ((128, 20, 36),
           ((18, 19, 20, 21), 7), ((17, 3, 18, 2, 19), 12), ((20, 700, 90), 24), ((30, 1, 40), 6)]
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
 @pytest.mark.parametrize("dims,R", SHAPES)
-def test_mttkrp_f32_edges(dims, R):
+def test_mttkrp_edges(dims, R, dtype):
     import tensorfox_gb300 as tfx
     g = torch.Generator(device="cuda").manual_seed(sum(dims) + R)
     L = len(dims)
     # an offset of one element: the tensor's base is not 16-byte aligned
     for shift in (0, 1):
-        buf = torch.randn(int(np.prod(dims)) + shift, device="cuda", generator=g)
+        buf = torch.randn(int(np.prod(dims)) + shift, device="cuda", generator=g, dtype=dtype)
         T = buf[shift:].view(dims)
-        W = [torch.randn((d, R), device="cuda", generator=g) for d in dims]
+        W = [torch.randn((d, R), device="cuda", generator=g, dtype=dtype) for d in dims]
         s = "abcde"[:L]
         for l in range(L):
             rest = [m for m in range(L) if m != l]
@@ -31,7 +32,9 @@ def test_mttkrp_f32_edges(dims, R):
             ref = torch.einsum(eq, T.double(), *[W[m].double() for m in rest])
             mag = torch.einsum(eq, T.double().abs(), *[W[m].double().abs() for m in rest])
             out = tfx.mttkrp(T, W, l).double()
-            # FP32 sums of K products of L factors: at most (K + L) roundings of
-            # 2^-24 of the sum of magnitudes, K capped by the split's chain
-            n = min(int(np.prod([dims[m] for m in rest])), 4096) + L + 64
-            assert torch.all((out - ref).abs() <= n * 2.0 ** -24 * mag + 1e-30), (l, shift)
+            # sums of K products of L factors: at most (K + L) roundings of the
+            # sum of magnitudes (FP32: K capped by the split's chain); the FP64
+            # reference has as many
+            K = int(np.prod([dims[m] for m in rest]))
+            n, u = (min(K, 4096) + L + 64, 2.0 ** -24) if dtype == torch.float32 else (2 * (K + L), 2.0 ** -53)
+            assert torch.all((out - ref).abs() <= n * u * mag + 1e-30), (l, shift)
