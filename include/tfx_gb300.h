@@ -213,6 +213,11 @@ int tfx_tensor_norms(int dtype, const void* T, long long N, double* out2, void* 
 size_t tfx_mttkrp_scratch_bytes(int dtype, int L, const int* dims, int R, int mode);
 int tfx_mttkrp(int dtype, const void* T, int L, const int* dims, int R, const void* W, int mode, void* out, void* scratch,
                size_t scratch_bytes, void* stream);
+/* The same product for every mode at once, out in the flat layout (the modes are
+ * cut in two halves, so the tensor is read twice instead of L times). */
+size_t tfx_mttkrp_all_scratch_bytes(int dtype, int L, const int* dims, int R);
+int tfx_mttkrp_all(int dtype, const void* T, int L, const int* dims, int R, const void* W, void* out, void* scratch,
+                   size_t scratch_bytes, void* stream);
 int tfx_cp_full(int dtype, int L, const int* dims, int R, const void* W, void* out, void* stream);
 /* The same product T_(l) KR_l of an FP32 tensor on the 5th-generation tensor
  * cores (GaussNewton.py:401-427 compute_grad's contraction, 411-423): the

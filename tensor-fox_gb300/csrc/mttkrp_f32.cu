@@ -46,6 +46,7 @@ __device__ __forceinline__ float2 unpack2(f2 v) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
   return f;
 }
+__device__ __forceinline__ void add2(f2& c, f2 a) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(c) : "l"(a)); }
 __device__ __forceinline__ void fma2(f2& c, f2 a, f2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
 
 template <int TN, int WM, bool LAST, bool FOLD>
@@ -155,13 +156,13 @@ __global__ void __launch_bounds__(NT, Cfg<TN, WM, LAST, FOLD>::CTAS)
     }
   };
 
-  f2 acc[4][TN / 2], sum[4][FOLD ? TN / 2 : 1];
+  f2 acc[4][TN / 2], sum[4][TN / 2];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < TN / 2; ++j) {
       acc[i][j] = 0ull;
-      if (FOLD) sum[i][j] = 0ull;
+      sum[i][j] = 0ull;
     }
 
 #pragma unroll
@@ -210,7 +211,15 @@ __global__ void __launch_bounds__(NT, Cfg<TN, WM, LAST, FOLD>::CTAS)
         }
       }
     }
-    if (FOLD && (++cc == nc || c + 1 == ce)) {
+    if (!FOLD) {  // a chunk's sums into the total: 32-step chains
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < TN / 2; ++j) {
+          add2(sum[i][j], acc[i][j]);
+          acc[i][j] = 0ull;
+        }
+    } else if (++cc == nc || c + 1 == ce) {
       if (cc == nc) cc = 0;
       const float* sp = A + C::ASZ + BK * C::BN;
 #pragma unroll
@@ -226,11 +235,10 @@ __global__ void __launch_bounds__(NT, Cfg<TN, WM, LAST, FOLD>::CTAS)
     }
     if (++stage == STAGES) stage = 0;
   }
-  if (FOLD)
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < TN / 2; ++j) acc[i][j] = sum[i][j];
+    for (int j = 0; j < TN / 2; ++j) acc[i][j] = sum[i][j];
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   if (C::WK > 1) {  // the k groups' sums, in order, into group 0
     __syncthreads();

@@ -7,7 +7,7 @@
 //   M[d, r] = sum_o KR_O[o, r] (sum_f T[d, o, f] KR_F[f, r]).
 // So the inner loop is a plain GEMM whose operands both arrive by cp.async, and
 // every dF steps the sums are scaled by KR_O's row and folded into a second set
-// (no fold when F holds every other mode).  Forming Khatri-Rao rows in the loop
+// (none in FP64 when F holds every other mode; FP32 then adds chunk by chunk).  Forming Khatri-Rao rows in the loop
 // instead cost as many instructions as the FMAs.
 #pragma once
 #include <cuda_runtime.h>
@@ -56,8 +56,7 @@ struct Plan {
 // F: every other mode if they lie together and the block stays within 8 MB;
 // else the one beside the rows, and those next to it while the chunks' padding
 // is above 1/8 and the block within 4096 rows.
-// Splits: one wave of the resident CTAs, in FP32 at least 4 chunks each and
-// without a fold at most 2048 steps (a longer FP32 chain loses digits).
+// Splits: one wave of the resident CTAs, in FP32 at least 4 chunks each.
 inline Plan plan(int es, const CpDims& sh, int g0, int g1, int sms) {
   Plan p;
   const int L = sh.L, R = sh.R;
@@ -106,7 +105,6 @@ inline Plan plan(int es, const CpDims& sh, int g0, int g1, int sms) {
   p.tilesM = (D + 32 * p.WM - 1) / (32 * p.WM);
   const long long nch = p.w.nO * p.w.nc, slots = (long long)sms * (f32 ? (p.TN > 8 ? 2 : 3) : (p.TN > 8 ? 4 : 6));
   long long ks = std::max<long long>(1, slots / (p.tilesM * p.nblk));
-  while (f32 && !p.fold && nch * BK / ks > 2048) ks *= 2;
   ks = std::max<long long>(1, std::min(ks, f32 ? nch / 4 : nch));
   p.ks = (int)std::min<long long>(ks, 32768);
   p.krF_bytes = (size_t)((p.rowsF * p.w.ldp * es + 255) & ~255LL);
@@ -152,6 +150,21 @@ __global__ void __launch_bounds__(32 * SG) k_sum(const T* __restrict__ part, lon
     if (!COL) out[e] = (T)t.value();
     else if (r < R) out[(size_t)r * D + d] = (T)t.value();
   }
+}
+
+// The same for few partials: one output a thread.
+template <class T, bool COL>
+__global__ void __launch_bounds__(256) k_sum_few(const T* __restrict__ part, long long D, int R, int ldp, int ks,
+                                                 T* __restrict__ out) {
+  const long long n = D * ldp, e = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (e >= n) return;
+  Acc<T> s;
+#pragma unroll 4
+  for (int k = 0; k < ks; ++k) s.add(__ldcs(part + (size_t)k * n + e));
+  const long long d = e / ldp;
+  const int r = (int)(e - d * ldp);
+  if (!COL) out[e] = (T)s.value();
+  else if (r < R) out[(size_t)r * D + d] = (T)s.value();
 }
 
 // KR_F as [column block][nF rows padded to chunks][BN] (zeros in the padding)
@@ -220,7 +233,16 @@ inline cudaError_t run(Plan p, const T* X, const T* W, const CpDims& sh, T* out,
   if ((e = gemm(p, X, krF, krO, direct ? out : part, st)) != cudaSuccess) return e;
   *launches += direct ? 2 : 3;
   if (direct) return cudaSuccess;
-  const unsigned sb = (unsigned)((p.w.D * p.w.ldp + 31) / 32);
+  const long long n = p.w.D * p.w.ldp;
+  // one thread an output where those fill the chip or the partials are few
+  // (147456 outputs of 2 partials: 12 us dealt to groups, 3 us this way)
+  if (p.ks <= 8 || n >= (1 << 20)) {
+    const unsigned sb = (unsigned)((n + 255) / 256);
+    if (col) k_sum_few<T, true><<<sb, 256, 0, st>>>(part, p.w.D, sh.R, p.w.ldp, p.ks, out);
+    else k_sum_few<T, false><<<sb, 256, 0, st>>>(part, p.w.D, sh.R, p.w.ldp, p.ks, out);
+    return cudaGetLastError();
+  }
+  const unsigned sb = (unsigned)((n + 31) / 32);
   if (col) k_sum<T, true><<<sb, 32 * SG, 0, st>>>(part, p.w.D, sh.R, p.w.ldp, p.ks, out);
   else k_sum<T, false><<<sb, 32 * SG, 0, st>>>(part, p.w.D, sh.R, p.w.ldp, p.ks, out);
   return cudaGetLastError();

@@ -50,6 +50,9 @@ def _declare():
     lib.tfx_mttkrp.argtypes = [I, P, I, ctypes.POINTER(ctypes.c_int), I, P, I, P, P, SZ, P]
     lib.tfx_mttkrp_scratch_bytes.restype = SZ
     lib.tfx_mttkrp_scratch_bytes.argtypes = [I, I, ctypes.POINTER(ctypes.c_int), I, I]
+    lib.tfx_mttkrp_all.argtypes = [I, P, I, ctypes.POINTER(ctypes.c_int), I, P, P, P, SZ, P]
+    lib.tfx_mttkrp_all_scratch_bytes.restype = SZ
+    lib.tfx_mttkrp_all_scratch_bytes.argtypes = [I, I, ctypes.POINTER(ctypes.c_int), I]
     lib.tfx_cp_full.argtypes = [I, I, ctypes.POINTER(ctypes.c_int), I, P, P, P]
     lib.tfx_cp_wp1.argtypes = [I, I, ctypes.POINTER(ctypes.c_int), I, P, P, P, P]
     lib.tfx_cp_wp1_scratch_bytes.restype = SZ
@@ -74,6 +77,26 @@ def mttkrp(T, factors, mode):
     _lib.check(lib.tfx_mttkrp(_dt(T), _vp(T), len(dims), _cint(dims), R, _vp(W), int(mode), _vp(out), _vp(scratch),
                               nb, _st()))
     return out.t()
+
+
+def mttkrp_all(T, W_flat, dims, R):
+    """The MTTKRPs of every mode in the flat layout (one ``tfx_mttkrp_all`` call)."""
+    lib = _declare()
+    cd = _cint(dims)
+    nb = int(lib.tfx_mttkrp_all_scratch_bytes(_dt(T), len(dims), cd, R))
+    scratch = torch.empty(nb, dtype=torch.uint8, device=T.device)
+    out = torch.empty_like(W_flat)
+    _lib.check(lib.tfx_mttkrp_all(_dt(T), _vp(T), len(dims), cd, R, _vp(W_flat), _vp(out), _vp(scratch), nb, _st()))
+    return out
+
+
+def _columns(flat, dims, R):
+    """The (d_l, R) matrices of a flat vector, as views."""
+    out, s = [], 0
+    for d in dims:
+        out.append(flat[s:s + d * R].view(R, d).t())
+        s += d * R
+    return out
 
 
 def cp_full(factors):
@@ -111,6 +134,10 @@ class CPReconstruct(torch.autograd.Function):
     def backward(ctx, G):
         factors = ctx.saved_tensors
         G = G.contiguous().to(factors[0].dtype)
+        if all(ctx.needs_input_grad) and len(factors) > 1:
+            dims = list(G.shape)
+            R = int(factors[0].shape[1])
+            return tuple(_columns(mttkrp_all(G, _flat(factors).to(G.dtype), dims, R), dims, R))
         return tuple(mttkrp(G, factors, l) if ctx.needs_input_grad[l] else None for l in range(len(factors)))
 
 

@@ -38,3 +38,34 @@ def test_mttkrp_edges(dims, R, dtype):
             K = int(np.prod([dims[m] for m in rest]))
             n, u = (min(K, 4096) + L + 64, 2.0 ** -24) if dtype == torch.float32 else (2 * (K + L), 2.0 ** -53)
             assert torch.all((out - ref).abs() <= n * u * mag + 1e-30), (l, shift)
+
+
+# cuts after the first, a middle and the last mode, halves of one and of several
+# modes, short modes (whose single product takes a group too)
+ALL_SHAPES = [((200, 31, 33), 20), ((31, 33, 200), 20), ((70, 75, 80), 50), ((40, 41, 3, 3), 64), ((3, 40, 41), 9),
+              ((21, 22, 23, 24), 12), ((9, 10, 11, 12, 13), 5), ((5, 6, 4, 5, 3, 4), 3), ((50, 60), 7), ((12, 2, 500), 66)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("dims,R", ALL_SHAPES)
+def test_mttkrp_all_modes(dims, R, dtype):
+    import tensorfox_gb300 as tfx
+    from tensorfox_gb300.autograd import mttkrp_all, _columns
+    g = torch.Generator(device="cuda").manual_seed(sum(dims) + R)
+    L = len(dims)
+    T = torch.randn(dims, device="cuda", generator=g, dtype=dtype)
+    W = [torch.randn((d, R), device="cuda", generator=g, dtype=dtype) for d in dims]
+    flat = torch.cat([w.t().reshape(-1) for w in W])
+    every = _columns(mttkrp_all(T, flat, list(dims), R), list(dims), R)
+    s = "abcdef"[:L]
+    for l in range(L):
+        rest = [m for m in range(L) if m != l]
+        eq = s + "," + ",".join(s[m] + "r" for m in rest) + "->" + s[l] + "r"
+        ref = torch.einsum(eq, T.double(), *[W[m].double() for m in rest])
+        mag = torch.einsum(eq, T.double().abs(), *[W[m].double().abs() for m in rest])
+        # the GEMM's chain, then the group's contraction: at most one rounding a
+        # product and a term
+        K = int(np.prod([dims[m] for m in rest]))
+        n, u = (min(K, 4096) + 2 * L + 64, 2.0 ** -24) if dtype == torch.float32 else (2 * (K + 2 * L), 2.0 ** -53)
+        for out in (every[l], tfx.mttkrp(T, W, l)):
+            assert torch.all((out.double() - ref).abs() <= n * u * mag + 1e-30), l
