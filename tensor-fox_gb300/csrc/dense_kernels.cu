@@ -1,8 +1,5 @@
 // Grid-level dense kernels of the compression (MLSVD) and full-tensor stages.
 //
-//   tfx_mode_gram      S_(l) S_(l)^T of a C-order tensor viewed as (P, D, Q)
-//                      (Compression.py:192-237: the Gram route replaces the
-//                      randomized SVD's streaming passes over the unfolding)
 //   tfx_gemm           strided batched C = alpha A B + beta C (TTM, subspace
 //                      products, decompression U_l W_l; TensorFox.py:573-574)
 //   tfx_orthonormalize CGS2 on the columns of a tall matrix (one CTA)
@@ -21,78 +18,6 @@
 #include "linalg.cuh"
 
 namespace tfx {
-
-// ---------------------------------------------------------------------------
-// mode Gram: partial[s][i][j] = sum_{k in split s} A(i,k) A(j,k),
-// A(i, k) = S[p*D*Q + i*Q + q] with k = p*Q + q; upper tile pairs only.
-// ---------------------------------------------------------------------------
-template <class T, int TS>
-__global__ void __launch_bounds__(TFX_THREADS) k_mode_gram(const T* __restrict__ S, long long P, int D, long long Q,
-                                                           int ksplit, T* __restrict__ part) {
-  using TL = Tile<TS, TS>;
-  __shared__ T sA[TFX_BK * TL::LDA];
-  __shared__ T sB[TFX_BK * TL::LDB];
-  const int nt = (D + TL::BM - 1) / TL::BM;
-  // tile pair index -> (bi, bj), bi <= bj
-  int t = blockIdx.x, bi = 0;
-  while (t >= nt - bi) {
-    t -= nt - bi;
-    ++bi;
-  }
-  const int bj = bi + t;
-  const int i0 = bi * TL::BM, j0 = bj * TL::BN;
-  const long long K = P * Q;
-  const long long kb = K * blockIdx.y / ksplit, ke = K * (blockIdx.y + 1) / ksplit;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  T acc[TS][TS];
-  tile_zero<T, TS, TS>(acc);
-  const bool kfast = Q > 1;
-  for (long long k0 = kb; k0 < ke; k0 += TFX_BK) {
-    const int kc = (int)min((long long)TFX_BK, ke - k0);
-    for (int e = tid; e < TFX_BK * TL::BM; e += TFX_THREADS) {
-      int kk, mm;
-      if (kfast) {
-        mm = e / TFX_BK;
-        kk = e - mm * TFX_BK;
-      } else {
-        kk = e / TL::BM;
-        mm = e - kk * TL::BM;
-      }
-      T va = T(0), vb = T(0);
-      if (kk < kc) {
-        const long long k = k0 + kk, p = k / Q, q = k - p * Q;
-        const long long base = p * (long long)D * Q + q;
-        if (i0 + mm < D) va = S[base + (long long)(i0 + mm) * Q];
-        if (j0 + mm < D) vb = S[base + (long long)(j0 + mm) * Q];
-      }
-      sA[kk * TL::LDA + mm] = va;
-      sB[kk * TL::LDB + mm] = vb;
-    }
-    __syncthreads();
-    tile_fma<T, TS, TS>(sA, sB, acc, kc);
-    __syncthreads();
-  }
-  T* out = part + (size_t)blockIdx.y * D * D;
-#pragma unroll
-  for (int u = 0; u < TS; ++u)
-#pragma unroll
-    for (int v = 0; v < TS; ++v) {
-      const int i = i0 + ty + 16 * u, j = j0 + tx + 16 * v;
-      if (i < D && j < D) out[(size_t)i * D + j] = acc[u][v];
-    }
-}
-
-template <class T, int BMt>
-__global__ void k_gram_reduce(const T* __restrict__ part, int D, int ksplit, T* __restrict__ G) {
-  const long long n = (long long)D * D;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(e / D), j = (int)(e - (long long)i * D);
-    const long long src = (i / BMt <= j / BMt) ? e : (long long)j * D + i;
-    double s = 0.0;
-    for (int k = 0; k < ksplit; ++k) s += (double)part[(size_t)k * n + src];
-    G[e] = (T)s;
-  }
-}
 
 // ---------------------------------------------------------------------------
 // strided batched GEMM: C[b](m,n) = alpha * sum_k A[b](m,k) B[b](k,n) + beta C
@@ -955,61 +880,20 @@ static int check_launch(const char* where) {
   return TFX_STATUS_OK;
 }
 
-extern "C" size_t tfx_mode_gram_scratch_bytes(int dtype, long long P, int D, long long Q) {
-  const int BM = 64;
-  const int nt = (D + BM - 1) / BM;
-  const long long tiles = (long long)nt * (nt + 1) / 2;
-  const long long K = P * Q;
-  long long ks = (4LL * num_sms() + tiles - 1) / tiles;
-  const long long kmax = (K + 255) / 256;
-  if (ks > kmax) ks = kmax;
-  if (ks < 1) ks = 1;
-  if (ks > 64) ks = 64;
-  return (size_t)ks * D * D * (dtype == TFX_F64 ? 8 : 4);
-}
-
-extern "C" int tfx_mode_gram(int dtype, const void* S, long long P, int D, long long Q, void* G, void* scratch,
-                             size_t scratch_bytes, void* stream) {
-  if (!S || !G || !scratch || P < 1 || D < 1 || Q < 1) return tfx_set_error(TFX_STATUS_ERR_ARG, "mode_gram args");
-  const size_t es = dtype == TFX_F64 ? 8 : 4;
-  const int BM = 64;
-  const int nt = (D + BM - 1) / BM;
-  const long long tiles = (long long)nt * (nt + 1) / 2;
-  int ks = (int)(scratch_bytes / ((size_t)D * D * es));
-  const size_t want = tfx_mode_gram_scratch_bytes(dtype, P, D, Q) / ((size_t)D * D * es);
-  if ((size_t)ks > want) ks = (int)want;
-  if (ks < 1) return tfx_set_error(TFX_STATUS_ERR_ARG, "mode_gram scratch too small");
-  cudaStream_t st = (cudaStream_t)stream;
-  dim3 grid((unsigned)tiles, (unsigned)ks);
-  const long long n = (long long)D * D;
-  const int rb = (int)std::min<long long>((n + 255) / 256, 4LL * num_sms());
-  if (dtype == TFX_F32) {
-    k_mode_gram<float, 4><<<grid, TFX_THREADS, 0, st>>>((const float*)S, P, D, Q, ks, (float*)scratch);
-    int s = check_launch("mode_gram");
-    if (s) return s;
-    k_gram_reduce<float, 64><<<rb, 256, 0, st>>>((const float*)scratch, D, ks, (float*)G);
-  } else {
-    k_mode_gram<double, 4><<<grid, TFX_THREADS, 0, st>>>((const double*)S, P, D, Q, ks, (double*)scratch);
-    int s = check_launch("mode_gram");
-    if (s) return s;
-    k_gram_reduce<double, 64><<<rb, 256, 0, st>>>((const double*)scratch, D, ks, (double*)G);
-  }
-  return check_launch("gram_reduce");
-}
-
 // ---------------------------------------------------------------------------
 // C = alpha A B + beta C for a short left factor (M <= 64 rows) and a long K:
 // the eigen-step's products (60 x 512 by 512 x 512, 60 x 512 by 512 x 60).  A
-// CTA owns SK_NB columns of C and every row; its 256 threads are 64 rows x 4
-// quarters of each K chunk, each accumulating SK_NB outputs, and the four
+// CTA owns NB columns of C and every row; its 256 threads are 64 rows x 4
+// quarters of each K chunk, each accumulating NB outputs, and the four
 // quarter sums are added in a fixed order at the end.  One output per thread
 // over all of K (the general kernel's smallest tile) leaves a 512-long
-// dependent chain per thread.
+// dependent chain per thread.  NB = 16 in FP32; 4 in FP64, whose pipe is the
+// bound: four times the CTAs, and warps past the last row do no FMAs (20 x 100 x
+// 100: 45 -> 8 us).
 // ---------------------------------------------------------------------------
-#define SK_NB 16
 #define SK_KC 128
 
-template <class T>
+template <class T, int SK_NB>
 __global__ void __launch_bounds__(256) k_gemm_skinny(const T* __restrict__ A, const T* __restrict__ B, T* C,
                                                      GemmArgs g) {
   extern __shared__ __align__(16) char sk_smem[];
@@ -1053,6 +937,7 @@ __global__ void __launch_bounds__(256) k_gemm_skinny(const T* __restrict__ A, co
     // (FP64) loads per k instead of 16
     using V = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
     constexpr int PV = 16 / sizeof(T);
+    if ((row & 32) >= M) continue;
 #pragma unroll 4
     for (int kk = 0; kk < SK_KC / 4; ++kk) {
       const T a = ar[kk];
@@ -1079,8 +964,8 @@ __global__ void __launch_bounds__(256) k_gemm_skinny(const T* __restrict__ A, co
   }
 }
 
-static size_t skinny_smem(size_t es) {
-  return (size_t)(64 * (SK_KC + 1) + SK_KC * SK_NB + 4 * 64 * SK_NB) * es;
+static size_t skinny_smem(size_t es, int nb) {
+  return (size_t)(64 * (SK_KC + 1) + SK_KC * nb + 4 * 64 * nb) * es;
 }
 
 extern "C" int tfx_gemm(int dtype, const void* A, const void* B, void* C, long long M, long long N, long long K,
@@ -1105,18 +990,19 @@ extern "C" int tfx_gemm(int dtype, const void* A, const void* B, void* C, long l
   g.alpha = alpha;
   g.beta = beta;
   cudaStream_t st = (cudaStream_t)stream;
-  if (batch == 1 && M <= 64 && K >= 32 && N <= 65535LL * SK_NB) {
-    const size_t sm = skinny_smem(dtype == TFX_F32 ? 4 : 8);
-    const unsigned grid = (unsigned)((N + SK_NB - 1) / SK_NB);
+  if (batch == 1 && M <= 64 && K >= 32 && N <= 65535LL * 16) {
+    const int nb = dtype == TFX_F32 ? 16 : 4;
+    const size_t sm = skinny_smem(dtype == TFX_F32 ? 4 : 8, nb);
+    const unsigned grid = (unsigned)((N + nb - 1) / nb);
     cudaError_t e;
     if (dtype == TFX_F32) {
-      e = cudaFuncSetAttribute(k_gemm_skinny<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      e = cudaFuncSetAttribute(k_gemm_skinny<float, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       if (e != cudaSuccess) return tfx_set_cuda_error(e, "gemm_skinny smem");
-      k_gemm_skinny<float><<<grid, 256, sm, st>>>((const float*)A, (const float*)B, (float*)C, g);
+      k_gemm_skinny<float, 16><<<grid, 256, sm, st>>>((const float*)A, (const float*)B, (float*)C, g);
     } else {
-      e = cudaFuncSetAttribute(k_gemm_skinny<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      e = cudaFuncSetAttribute(k_gemm_skinny<double, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       if (e != cudaSuccess) return tfx_set_cuda_error(e, "gemm_skinny smem");
-      k_gemm_skinny<double><<<grid, 256, sm, st>>>((const double*)A, (const double*)B, (double*)C, g);
+      k_gemm_skinny<double, 4><<<grid, 256, sm, st>>>((const double*)A, (const double*)B, (double*)C, g);
     }
     return check_launch("gemm_skinny");
   }
@@ -1144,6 +1030,117 @@ extern "C" int tfx_gemm(int dtype, const void* A, const void* B, void* C, long l
   return check_launch("gemm");
 }
 
+// ---------------------------------------------------------------------------
+// Mode product in FP64: out[p] (n x Q) = Ut (n x D) S[p] (D x Q); Q == 1: out
+// (P x n) = S (P x D) Ut^T.  Bound by the FP64 pipe, so no padded FMAs: a warp
+// holds 8 rows (q, or p) x 4 TN columns, one output a lane and column group,
+// over the valid k only.  WK = 4: the four warps share 8 rows and take a quarter
+// of each k chunk, where 32-row CTAs would leave SMs idle.  20 x 150 x 18330: 124
+// us; 542 us when 20 of the 64 rows of the short-left-factor GEMM did work.
+// ---------------------------------------------------------------------------
+constexpr int TD_BK = 32, TD_ST = TD_BK + 2, TD_NT = 128;
+
+__device__ __forceinline__ void cp_async_bytes(void* sdst, const void* gsrc, int bytes) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
+  if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gsrc) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gsrc) : "memory");
+}
+
+template <int TN, int WK>
+__global__ void __launch_bounds__(TD_NT) k_ttm_f64(const double* __restrict__ S, const double* __restrict__ Ut,
+                                                   double* __restrict__ out, int n, int D, long long Q, long long P,
+                                                   int vec_a, int vec_b) {
+  constexpr int BM = 32 / WK, BN = 4 * TN;
+  __shared__ __align__(16) double sA[2][32 * TD_ST];  // [k][BM] or, Q == 1, [row][TD_ST]
+  __shared__ __align__(16) double sB[2][BN * TD_ST];  // [column][TD_ST]
+  __shared__ double red[WK > 1 ? 3 * BN * 8 : 1];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lm = lane >> 2, ln = lane & 3;
+  const bool rowk = Q == 1;
+  const long long rows = rowk ? P : Q, m0 = (long long)blockIdx.x * BM;
+  const int n0 = blockIdx.z * BN, nn = min(BN, n - n0);
+  const int strip = WK > 1 ? 0 : ((warp + blockIdx.x) & 3);
+  const bool on = m0 + 8 * strip < rows;
+  const int nch = (D + TD_BK - 1) / TD_BK;
+  for (long long p = blockIdx.y; p < (rowk ? 1 : P); p += gridDim.y) {
+    const double* Sp = S + p * D * Q;
+    auto load = [&](int c, int b) {
+      const int k0 = c * TD_BK;
+      if (rowk) {
+        const int k = vec_a ? (tid & 15) * 2 : lane, mr = vec_a ? tid >> 4 : warp;
+        if (k0 + k < D)
+          for (int m = mr; m < BM; m += vec_a ? 8 : 4)
+            if (m0 + m < rows) cp_async_bytes(&sA[b][m * TD_ST + k], Sp + (m0 + m) * D + k0 + k, vec_a ? 16 : 8);
+      } else {
+        const int per = vec_a ? BM / 2 : BM, m = (tid % per) * (vec_a ? 2 : 1);
+        if (m0 + m < rows)
+          for (int k = tid / per; k < TD_BK; k += TD_NT / per)
+            if (k0 + k < D) cp_async_bytes(&sA[b][k * BM + m], Sp + (long long)(k0 + k) * Q + m0 + m, vec_a ? 16 : 8);
+      }
+      const int k = vec_b ? (tid & 15) * 2 : lane;
+      if (k0 + k < D)
+        for (int j = vec_b ? tid >> 4 : warp; j < nn; j += vec_b ? 8 : 4)
+          cp_async_bytes(&sB[b][j * TD_ST + k], Ut + (long long)(n0 + j) * D + k0 + k, vec_b ? 16 : 8);
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    double acc[TN];
+#pragma unroll
+    for (int g = 0; g < TN; ++g) acc[g] = 0.0;
+    __syncthreads();  // the previous p's readers are done
+    load(0, 0);
+    for (int c = 0; c < nch; ++c) {
+      const int b = c & 1;
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+      __syncthreads();
+      if (c + 1 < nch) load(c + 1, b ^ 1);
+      const int kc = min(TD_BK, D - c * TD_BK);
+      const int ke = WK > 1 ? min(kc, 8 * (warp + 1)) : kc;
+      if (on) {
+#pragma unroll 2
+        for (int k = WK > 1 ? 8 * warp : 0; k < ke; ++k) {
+          const int m = 8 * strip + lm;
+          const double a = rowk ? sA[b][m * TD_ST + k] : sA[b][k * BM + m];
+#pragma unroll
+          for (int g = 0; g < TN; ++g)
+            if (4 * g < nn) acc[g] = fma(a, sB[b][(4 * g + ln) * TD_ST + k], acc[g]);
+        }
+      }
+    }
+    if (WK > 1) {  // the quarters' sums, in order
+      if (warp > 0)
+#pragma unroll
+        for (int g = 0; g < TN; ++g) red[((warp - 1) * TN + g) * 32 + lane] = acc[g];
+      __syncthreads();
+      if (warp == 0)
+#pragma unroll
+        for (int g = 0; g < TN; ++g)
+#pragma unroll
+          for (int q = 0; q < 3; ++q) acc[g] += red[(q * TN + g) * 32 + lane];
+      if (warp > 0) continue;
+    }
+    const long long m = m0 + 8 * strip + lm;
+    if (m < rows) {
+#pragma unroll
+      for (int g = 0; g < TN; ++g) {
+        const int j = 4 * g + ln;
+        if (j < nn) out[rowk ? m * n + n0 + j : (p * n + n0 + j) * Q + m] = acc[g];
+      }
+    }
+  }
+}
+
+template <int TN>
+static void launch_ttm_f64(const double* S, long long P, int D, long long Q, const double* Ut, int n, double* out,
+                           cudaStream_t st) {
+  const long long rows = Q == 1 ? P : Q, batch = Q == 1 ? 1 : P;
+  const int nblk = (n + 4 * TN - 1) / (4 * TN);
+  const int va = ((uintptr_t)S & 15) == 0 && (Q == 1 ? D : Q) % 2 == 0, vb = ((uintptr_t)Ut & 15) == 0 && D % 2 == 0;
+  const unsigned by = (unsigned)std::min<long long>(batch, 65535);
+  if ((rows + 31) / 32 * batch * nblk >= 2LL * num_sms())
+    k_ttm_f64<TN, 1><<<dim3((unsigned)((rows + 31) / 32), by, nblk), TD_NT, 0, st>>>(S, Ut, out, n, D, Q, P, va, vb);
+  else
+    k_ttm_f64<TN, 4><<<dim3((unsigned)((rows + 7) / 8), by, nblk), TD_NT, 0, st>>>(S, Ut, out, n, D, Q, P, va, vb);
+}
+
 extern "C" int tfx_ttm(int dtype, const void* S, long long P, int D, long long Q, const void* Ut, int n, void* out,
                        void* stream) {
   if (!S || !Ut || !out || P < 1 || D < 1 || Q < 1 || n < 1) return tfx_set_error(TFX_STATUS_ERR_ARG, "ttm args");
@@ -1164,6 +1161,14 @@ extern "C" int tfx_ttm(int dtype, const void* S, long long P, int D, long long Q
     else
       k_ttm_f32<4><<<grid, 32 * nw, 0, st>>>((const float*)Ut, (const float*)S, (float*)out, n, D, Q, P);
     return check_launch("ttm");
+  }
+  if (dtype == TFX_F64 && (Q == 1 || Q >= 8) && (Q == 1 ? P : Q) <= 0x7fffffffLL) {
+    const int per = (n + (n + 31) / 32 - 1) / ((n + 31) / 32);  // columns a block, at most 32
+    if (per <= 8) launch_ttm_f64<2>((const double*)S, P, D, Q, (const double*)Ut, n, (double*)out, st);
+    else if (per <= 16) launch_ttm_f64<4>((const double*)S, P, D, Q, (const double*)Ut, n, (double*)out, st);
+    else if (per <= 24) launch_ttm_f64<6>((const double*)S, P, D, Q, (const double*)Ut, n, (double*)out, st);
+    else launch_ttm_f64<8>((const double*)S, P, D, Q, (const double*)Ut, n, (double*)out, st);
+    return check_launch("ttm_f64");
   }
   // general shapes: strided batched GEMM, batched over p (Q >= 16) or over q
   long long sd[9];
@@ -1555,6 +1560,9 @@ static int noalloc_scratch_address(void** out) {
   *out = g_noalloc_addr[dev];
   return TFX_STATUS_OK;
 }
+
+extern "C" int tfx_mode_gram(int dtype, const void* S, long long P, int D, long long Q, void* G, void* scratch,
+                             size_t scratch_bytes, void* stream);
 
 extern "C" size_t tfx_mode_gram_noalloc_capacity_bytes(void) { return TFX_NOALLOC_SCRATCH_BYTES; }
 
