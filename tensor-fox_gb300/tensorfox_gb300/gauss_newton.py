@@ -50,14 +50,20 @@ def advance_rng(options, iterations):
             np.random.randint(1 + it ** 0.4, 2 + it ** 0.9)
 
 
-def auto_cluster(dims, R):
-    """CTAs per problem (one thread-block cluster): about one CTA per 1.2 million
-    multiply-adds of per-iteration MTTKRP work, at most 16 and at most R (every
-    CTA owns whole factor columns).  Measured on the 50^3, R=50 core of a
-    512^3 problem: 16 CTAs beat 10 and 8 despite the uneven column split."""
+def auto_cluster(dims, R, problems=1):
+    """CTAs per problem (one thread-block cluster): at most R, since every CTA
+    owns whole factor columns, and 16, or 8 where the core has fewer than 1e5
+    multiply-adds a product (the step from 8 to 16 then gains nothing).  One
+    CTA's own SM bounds small problems, in FP64 by its FP64 pipe.  Ten
+    iterations, one CTA against the cluster chosen: 10^3 R 10 FP64 3.8 -> 1.6 ms,
+    FP32 1.04 -> 0.71; 30^3 R 30 FP64 28.7 -> 3.7, FP32 4.3 -> 0.96 (two CTAs:
+    15.8 and 2.4); 4^3 R 4 FP32 0.65 -> 0.64.  ``problems`` solved in one launch
+    share the GPU's 152 SMs: no more CTAs than those, but about one CTA per 1.2
+    million multiply-adds of per-iteration MTTKRP work."""
     n = int(np.prod(dims))
-    work = n * R * len(dims)
-    return int(max(1, min(16, R, work // 1200000)))
+    alone = 16 if n * R >= 100000 else 8
+    share = max(152 // problems, n * R * len(dims) // 1200000)
+    return int(max(1, min(16, R, alone, share)))
 
 
 def _cluster_candidates(c, R):
