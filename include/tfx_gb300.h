@@ -202,6 +202,9 @@ int tfx_flip_signs(int dtype, void* U, int D, int n, void* stream);
 size_t tfx_cp_residual_scratch_bytes(void);
 int tfx_cp_residual(int dtype, const void* T, int L, const int* dims, int R, const void* W, double* out, void* scratch,
                     void* stream);
+/* The same value in the working type (dtype), the fit loss of the autograd layer. */
+int tfx_cp_fit_loss(int dtype, const void* T, int L, const int* dims, int R, const void* W, void* out, void* scratch,
+                    void* stream);
 /* norm(T)^2 and sum|T| (TensorFox.py:503, GaussNewton.py:113) into out2[0..1]. */
 int tfx_tensor_norms(int dtype, const void* T, long long N, double* out2, void* scratch, void* stream);
 

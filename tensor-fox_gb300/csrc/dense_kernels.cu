@@ -847,14 +847,6 @@ __global__ void k_tensor_norms(const T* __restrict__ Tt, long long N, double* __
 }
 
 // fixed-order sum of `n` partials with stride `stride` into out[0..stride)
-__global__ void k_sum_partials(const double* __restrict__ partial, int n, int stride, double* __restrict__ out) {
-  if (threadIdx.x < stride) {
-    double s = 0.0;
-    for (int i = 0; i < n; ++i) s += partial[(size_t)i * stride + threadIdx.x];
-    out[threadIdx.x] = s;
-  }
-}
-
 }  // namespace tfx
 
 // ============================================================================
@@ -1275,11 +1267,6 @@ extern "C" int tfx_flip_signs(int dtype, void* U, int D, int n, void* stream) {
 
 extern "C" size_t tfx_cp_residual_scratch_bytes(void) { return (size_t)8 * (8 * 1024 + 8); }
 
-namespace tfx {
-__global__ void k_nan_if_flag(const int* err, double* out) {
-  if (*err) *out = nan("");
-}
-}  // namespace tfx
 int tfx_cp_residual_tc_launch(const float* T, const int* dims, int R, const float* W, double* partial,
                               int max_partials, int* err, int* nblocks, cudaStream_t st);
 
@@ -1290,7 +1277,7 @@ int tfx_cp_residual_tc_launch(const float* T, const int* dims, int R, const floa
 // walks every row tile of mode 0: the model tile (8 rows per warp, 8 x 8
 // outputs per lane as in k_ttm_f32) = W_0 (rows x R) KR^T (R x 256), and the
 // epilogue subtracts the streamed tensor tile and accumulates squares in
-// float-float.  Block partials are summed in FP64 by k_sum_partials.
+// float-float.  Block partials are summed in FP64 by k_final_sum.
 // ---------------------------------------------------------------------------
 constexpr int RES_BN = 256, RES_RMAX = 64;
 
@@ -1411,9 +1398,11 @@ __global__ void __launch_bounds__(256, 2) k_cp_residual_f32(const float* __restr
   }
 }
 
-extern "C" int tfx_cp_residual(int dtype, const void* T, int L, const int* dims, int R, const void* W, double* out,
-                               void* scratch, void* stream) {
-  if (!T || !dims || !W || !out || !scratch || L < 2 || L > TFX_MAX_ORDER || R < 1)
+// ||T - [[W]]||^2 into out (double) and out_t (the working type), either may be null
+template <class T>
+static int cp_residual(int dtype, const void* Tp, int L, const int* dims, int R, const void* W, double* out, T* out_t,
+                       void* scratch, void* stream) {
+  if (!Tp || !dims || !W || !(out || out_t) || !scratch || L < 2 || L > TFX_MAX_ORDER || R < 1)
     return tfx_set_error(TFX_STATUS_ERR_ARG, "cp_residual args");
   CpShape sh;
   sh.L = L;
@@ -1435,13 +1424,10 @@ extern "C" int tfx_cp_residual(int dtype, const void* T, int L, const int* dims,
     cudaError_t ce = cudaMemsetAsync(err, 0, sizeof(int), st);
     if (ce != cudaSuccess) return tfx_set_cuda_error(ce, "cp_residual flag");
     int nb = 0;
-    const int r = tfx_cp_residual_tc_launch((const float*)T, dims, R, (const float*)W, partial, 8 * 1024, err, &nb, st);
+    const int r = tfx_cp_residual_tc_launch((const float*)Tp, dims, R, (const float*)W, partial, 8 * 1024, err, &nb, st);
     if (r == TFX_STATUS_OK) {
-      k_sum_partials<<<1, 32, 0, st>>>(partial, nb, 1, out);
-      int c = check_launch("sum_partials");
-      if (c) return c;
-      k_nan_if_flag<<<1, 1, 0, st>>>(err, out);
-      return check_launch("cp_residual flag");
+      k_final_sum<T><<<1, 256, 0, st>>>(partial, nb, 1, err, out, out_t);
+      return check_launch("final_sum");
     }
     if (r != TFX_STATUS_ERR_UNSUPPORTED) return r;
   }
@@ -1453,22 +1439,38 @@ extern "C" int tfx_cp_residual(int dtype, const void* T, int L, const int* dims,
     const size_t smb = ((size_t)RES_RMAX * RES_BN + 64 * (RES_RMAX + 4)) * sizeof(float);
     cudaError_t e = cudaFuncSetAttribute(k_cp_residual_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
     if (e != cudaSuccess) return tfx_set_cuda_error(e, "cp_residual attr");
-    k_cp_residual_f32<<<blocks, 32 * nw, smb, st>>>((const float*)T, (const float*)W, sh, Q0, partial);
+    k_cp_residual_f32<<<blocks, 32 * nw, smb, st>>>((const float*)Tp, (const float*)W, sh, Q0, partial);
     int r = check_launch("cp_residual");
     if (r) return r;
-    k_sum_partials<<<1, 32, 0, st>>>(partial, blocks, 1, out);
-    return check_launch("sum_partials");
+    k_final_sum<T><<<1, 256, 0, st>>>(partial, blocks, 1, nullptr, out, out_t);
+    return check_launch("final_sum");
   }
   const long long tiles = ((dims[0] + 63) / 64) * ((Q0 + 63) / 64);
   const int blocks = (int)std::max<long long>(1, std::min<long long>(tiles, 8LL * num_sms()));
   if (dtype == TFX_F32)
-    k_cp_residual<float, 4><<<blocks, TFX_THREADS, 0, st>>>((const float*)T, (const float*)W, sh, partial);
+    k_cp_residual<float, 4><<<blocks, TFX_THREADS, 0, st>>>((const float*)Tp, (const float*)W, sh, partial);
   else
-    k_cp_residual<double, 4><<<blocks, TFX_THREADS, 0, st>>>((const double*)T, (const double*)W, sh, partial);
+    k_cp_residual<double, 4><<<blocks, TFX_THREADS, 0, st>>>((const double*)Tp, (const double*)W, sh, partial);
   int r = check_launch("cp_residual");
   if (r) return r;
-  k_sum_partials<<<1, 32, 0, st>>>(partial, blocks, 1, out);
-  return check_launch("sum_partials");
+  k_final_sum<T><<<1, 256, 0, st>>>(partial, blocks, 1, nullptr, out, out_t);
+  return check_launch("final_sum");
+}
+
+extern "C" int tfx_cp_residual(int dtype, const void* T, int L, const int* dims, int R, const void* W, double* out,
+                               void* scratch, void* stream) {
+  if (!out) return tfx_set_error(TFX_STATUS_ERR_ARG, "cp_residual args");
+  return cp_residual<float>(dtype, T, L, dims, R, W, out, nullptr, scratch, stream);
+}
+
+// The same in the working type (the fit loss's value), one launch less than a
+// conversion of the double.
+extern "C" int tfx_cp_fit_loss(int dtype, const void* T, int L, const int* dims, int R, const void* W, void* out,
+                               void* scratch, void* stream) {
+  if (!out) return tfx_set_error(TFX_STATUS_ERR_ARG, "cp_fit_loss args");
+  if (dtype == TFX_F64)
+    return cp_residual<double>(dtype, T, L, dims, R, W, (double*)out, nullptr, scratch, stream);
+  return cp_residual<float>(dtype, T, L, dims, R, W, nullptr, (float*)out, scratch, stream);
 }
 
 extern "C" int tfx_tensor_norms(int dtype, const void* T, long long N, double* out2, void* scratch, void* stream) {
@@ -1482,8 +1484,8 @@ extern "C" int tfx_tensor_norms(int dtype, const void* T, long long N, double* o
     k_tensor_norms<double><<<blocks, TFX_THREADS, 0, st>>>((const double*)T, N, partial);
   int r = check_launch("tensor_norms");
   if (r) return r;
-  k_sum_partials<<<1, 32, 0, st>>>(partial, blocks, 2, out2);
-  return check_launch("sum_partials");
+  k_final_sum<double><<<1, 256, 0, st>>>(partial, blocks, 2, nullptr, out2, nullptr);
+  return check_launch("final_sum");
 }
 
 // ============================================================================

@@ -302,7 +302,7 @@ using namespace tfx;
 
 // Called by tfx_cp_residual for FP32 third-order tensors; returns
 // TFX_STATUS_ERR_UNSUPPORTED when the shape is outside the kernel's range so the
-// caller uses its SIMT kernel.  out = sum of the per-CTA partials (k_sum_partials
+// caller uses its SIMT kernel.  out = sum of the per-CTA partials (k_final_sum
 // is launched by the caller on `partial`); *nblocks receives the partial count.
 int tfx_cp_residual_tc_launch(const float* T, const int* dims, int R, const float* W, double* partial,
                               int max_partials, int* err, int* nblocks, cudaStream_t st) {

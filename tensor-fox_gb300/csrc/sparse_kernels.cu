@@ -661,14 +661,6 @@ __global__ void __launch_bounds__(TFX_THREADS) k_sparse_ttmc(const int* __restri
     }
 }
 
-__global__ void k_sum_partials_sp(const double* __restrict__ partial, int n, double* __restrict__ out) {
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i < n; ++i) s += partial[i];
-    out[0] = s;
-  }
-}
-
 template <class T>
 __global__ void k_sum_split(const T* __restrict__ part, long long n, int ks, T* __restrict__ out) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -801,8 +793,8 @@ extern "C" int tfx_sparse_residual(int dtype, const int* idx32, const void* vals
     k_sparse_residual<double><<<blocks, 256, 0, st>>>(idx32, (const double*)vals, nnz, sh,
                                                       (const double* const*)Wrow_dev, partial);
   if (int s = launched("sparse_residual")) return s;
-  k_sum_partials_sp<<<1, 32, 0, st>>>(partial, blocks, out);
-  return launched("sum_partials");
+  k_final_sum<double><<<1, 256, 0, st>>>(partial, blocks, 1, nullptr, out, nullptr);
+  return launched("final_sum");
 }
 
 extern "C" size_t tfx_coo_gram_scratch_bytes(long long nnz, int d) {

@@ -447,7 +447,34 @@ __device__ __forceinline__ void tile_zero(T (&acc)[TM][TN]) {
     for (int v = 0; v < TN; ++v) acc[u][v] = T(0);
 }
 
-// Status codes shared with the C ABI.
+// The sum of n partials of `stride` interleaved values each, by one CTA of 256
+// threads: thread t takes partials t, t + 256, ..., warps and then the eight
+// warp sums are added in a fixed order.  out[j] (double) and, where given,
+// out_t (the first value in the working type); *err != 0 makes them NaN.  One
+// thread walking the partials took 4 us for 300 of them and 65 us for 1216.
+template <class T>
+__global__ void __launch_bounds__(256) k_final_sum(const double* __restrict__ partial, int n, int stride,
+                                                   const int* __restrict__ err, double* __restrict__ out,
+                                                   T* __restrict__ out_t) {
+  __shared__ double red[8];
+  for (int j = 0; j < stride; ++j) {
+    double s = 0.0;
+    for (int i = threadIdx.x; i < n; i += 256) s += partial[(size_t)i * stride + j];
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = red[0];
+#pragma unroll
+      for (int w = 1; w < 8; ++w) t += red[w];
+      if (err && *err) t = nan("");
+      if (out) out[j] = t;
+      if (out_t && j == 0) *out_t = (T)t;
+    }
+    __syncthreads();
+  }
+}
+
 // Bounded wait on phase `parity` of a shared-memory mbarrier (its 32-bit
 // shared address): at most `limit` polls with mbarrier.try_wait.parity.
 // Returns false when the wait ran out; the caller then records an error status
@@ -467,6 +494,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar_addr, uint32_t pa
   return false;
 }
 
+// Status codes shared with the C ABI.
 #define TFX_OK 0
 #define TFX_ERR_ARG 1
 #define TFX_ERR_NUMERIC 2
