@@ -73,56 +73,97 @@ __global__ void __launch_bounds__(TFX_THREADS) k_cp_full(const T* __restrict__ W
 }
 
 // Gramians of every mode, G_m = W_m^T W_m (FP64, compensated sums of the
-// working-type products): grid L * ceil(R*R / 256), one entry per thread.
+// working-type products).  A CTA takes a 16 x 16 block on or above the diagonal
+// of one Gramian: 32 rows of its 32 columns at a time through shared memory
+// (coalesced), four groups of threads a quarter of the rows each, added in
+// order.  512 rows, R = 50: 67 us with one thread an entry walking two columns.
 template <class T>
-__global__ void __launch_bounds__(TFX_THREADS) k_cp_grams(const T* __restrict__ W, CpDims sh,
-                                                          double* __restrict__ gram) {
-  const int R = sh.R, RR = R * R;
-  const int per = (RR + TFX_THREADS - 1) / TFX_THREADS;
-  const int m = blockIdx.x / per;
-  const int e = (blockIdx.x - m * per) * TFX_THREADS + threadIdx.x;
-  if (e >= RR) return;
-  const int a = e / R, b = e - a * R;
-  if (a > b) return;
-  const int d = sh.d[m];
-  const T* wa = W + sh.off[m] + a * d;
-  const T* wb = W + sh.off[m] + b * d;
-  Acc<T> s;
-  for (int i = 0; i < d; ++i) s.fma_(wa[i], wb[i]);
-  const double v = s.value();
-  gram[(size_t)m * RR + a * R + b] = v;
-  gram[(size_t)m * RR + b * R + a] = v;
+__global__ void __launch_bounds__(1024) k_cp_grams(const T* __restrict__ W, CpDims sh, double* __restrict__ gram) {
+  __shared__ T sa[16][129], sb[16][129];
+  __shared__ double red[3][256];
+  const int R = sh.R, RR = R * R, nb = (R + 15) / 16;
+  int t = blockIdx.x, ba = 0;
+  while (t >= nb - ba) {
+    t -= nb - ba;
+    ++ba;
+  }
+  const int a0 = ba * 16, b0 = (ba + t) * 16, m = blockIdx.y, d = sh.d[m];
+  const int tid = threadIdx.x, z = tid >> 8, a = (tid >> 4) & 15, b = tid & 15;
+  const T* w = W + sh.off[m];
+  Acc<T> s[2];
+  for (int i0 = 0; i0 < d; i0 += 128) {
+    __syncthreads();
+    for (int e = tid; e < 32 * 128; e += 1024) {
+      const int c = e >> 7, i = e & 127, col = c < 16 ? a0 + c : b0 + c - 16;
+      const T v = (col < R && i0 + i < d) ? w[(long long)col * d + i0 + i] : T(0);
+      if (c < 16) sa[c][i] = v;
+      else sb[c - 16][i] = v;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int i = 32 * z; i < 32 * z + 32; i += 2) {
+      s[0].fma_(sa[a][i], sb[b][i]);
+      s[1].fma_(sa[a][i + 1], sb[b][i + 1]);
+    }
+  }
+  double v = s[0].value() + s[1].value();
+  if (z > 0) red[z - 1][tid & 255] = v;
+  __syncthreads();
+  if (z == 0 && a0 + a < R && b0 + b < R && a0 + a <= b0 + b) {
+    v = ((v + red[0][tid]) + red[1][tid]) + red[2][tid];
+    gram[(size_t)m * RR + (a0 + a) * R + b0 + b] = v;
+    gram[(size_t)m * RR + (b0 + b) * R + a0 + a] = v;
+  }
+}
+
+static unsigned gram_blocks(int R) {
+  const unsigned nb = (R + 15) / 16;
+  return nb * (nb + 1) / 2;
 }
 
 // out_l = scale (W_l P1_l - M_l), P1_l = o_{m != l} G_m (ascending m, FP64,
 // rounded to the working type in shared memory); M == nullptr means M_l = 0.
-// Grid (L, ceil(max d / 32)), 32 rows per CTA.
+// Grid (ceil(max d / 16), L), 16 rows per CTA; four accumulators a thread, whose
+// compensated chains overlap.
 template <class T>
 __global__ void __launch_bounds__(TFX_THREADS) k_cp_wp1(const T* __restrict__ W, CpDims sh,
                                                         const double* __restrict__ gram, const T* __restrict__ M,
                                                         T scale, T* __restrict__ out) {
   extern __shared__ __align__(16) char smem[];
-  T* sP = (T*)smem;
-  const int l = blockIdx.x, L = sh.L, R = sh.R, RR = R * R, tid = threadIdx.x;
-  const int dl = sh.d[l], r0 = blockIdx.y * 32;
+  T* sP = (T*)smem;          // [R][R]
+  const int l = blockIdx.y, L = sh.L, R = sh.R, RR = R * R, tid = threadIdx.x;
+  T* sW = sP + RR;           // [R][16]
+  const int dl = sh.d[l], r0 = blockIdx.x * 16;
   if (r0 >= dl) return;
+#pragma unroll 4
   for (int e = tid; e < RR; e += TFX_THREADS) {
     double p = 1.0;
     for (int m = 0; m < L; ++m)
       if (m != l) p *= gram[(size_t)m * RR + e];
     sP[e] = (T)p;
   }
+  for (int e = tid; e < 16 * R; e += TFX_THREADS) {
+    const int q = e >> 4, i = e & 15;
+    sW[e] = r0 + i < dl ? W[sh.off[l] + (long long)q * dl + r0 + i] : T(0);
+  }
   __syncthreads();
-  const int nr = min(32, dl - r0);
-  for (int e = tid; e < 32 * R; e += TFX_THREADS) {
-    const int ii = e & 31, r = e >> 5;
-    if (ii >= nr) continue;
-    const int i = r0 + ii;
-    Acc<T> s;
-    for (int q = 0; q < R; ++q) s.fma_(W[sh.off[l] + q * dl + i], sP[q * R + r]);
-    const size_t o = (size_t)sh.off[l] + (size_t)r * dl + i;
-    if (M) s.add(-M[o]);
-    out[o] = scale * (T)s.value();
+  for (int e = tid; e < 16 * R; e += TFX_THREADS) {
+    const int i = e & 15, r = e >> 4;
+    if (r0 + i >= dl) continue;
+    Acc<T> s[4];
+    int q = 0;
+    for (; q + 4 <= R; q += 4)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) s[u].fma_(sW[(q + u) * 16 + i], sP[(q + u) * R + r]);
+    for (; q < R; ++q) s[0].fma_(sW[q * 16 + i], sP[q * R + r]);
+#pragma unroll
+    for (int u = 1; u < 4; ++u) {
+      s[0].add(s[u].hi_or_v());
+      if (sizeof(T) == 4) s[0].add((T)s[u].lo_or_0());
+    }
+    const size_t o = (size_t)sh.off[l] + (size_t)r * dl + r0 + i;
+    if (M) s[0].add(-M[o]);
+    out[o] = scale * (T)s[0].value();
   }
 }
 
@@ -192,22 +233,21 @@ extern "C" int tfx_cp_wp1(int dtype, int L, const int* dims, int R, const void* 
   cudaStream_t st = (cudaStream_t)stream;
   int maxd = 0;
   for (int l = 0; l < L; ++l) maxd = std::max(maxd, dims[l]);
-  const int gb = L * ((R * R + TFX_THREADS - 1) / TFX_THREADS);
-  const dim3 grid(L, (maxd + 31) / 32);
+  const dim3 gb(gram_blocks(R), L), grid((maxd + 15) / 16, L);
   const size_t es = dtype == TFX_F64 ? 8 : 4;
-  const size_t smb = (size_t)R * R * es;
-  if (smb > 200 * 1024) return tfx_set_error(TFX_STATUS_ERR_UNSUPPORTED, "cp_wp1: rank too large");
+  const size_t smb = (size_t)R * (R + 16) * es;
+  if ((size_t)R * R * es > 200 * 1024) return tfx_set_error(TFX_STATUS_ERR_UNSUPPORTED, "cp_wp1: rank too large");
   cudaError_t e = dtype == TFX_F32
                       ? cudaFuncSetAttribute(k_cp_wp1<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb)
                       : cudaFuncSetAttribute(k_cp_wp1<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
   if (e != cudaSuccess) return tfx_set_cuda_error(e, "cp_wp1 attribute");
   if (dtype == TFX_F32) {
-    k_cp_grams<float><<<gb, TFX_THREADS, 0, st>>>((const float*)W, sh, (double*)scratch);
+    k_cp_grams<float><<<gb, 1024, 0, st>>>((const float*)W, sh, (double*)scratch);
     if (int r = done("cp_grams")) return r;
     k_cp_wp1<float><<<grid, TFX_THREADS, smb, st>>>((const float*)W, sh, (const double*)scratch, nullptr, 1.f,
                                                     (float*)out);
   } else {
-    k_cp_grams<double><<<gb, TFX_THREADS, 0, st>>>((const double*)W, sh, (double*)scratch);
+    k_cp_grams<double><<<gb, 1024, 0, st>>>((const double*)W, sh, (double*)scratch);
     if (int r = done("cp_grams")) return r;
     k_cp_wp1<double><<<grid, TFX_THREADS, smb, st>>>((const double*)W, sh, (const double*)scratch, nullptr, 1.0,
                                                      (double*)out);
@@ -252,20 +292,20 @@ extern "C" int tfx_cp_fit_grad(int dtype, const void* T, int L, const int* dims,
   char* sc = (char*)scratch;
   int maxd = 0;
   for (int l = 0; l < L; ++l) maxd = std::max(maxd, dims[l]);
-  const size_t smb = (size_t)R * R * es;
-  if (smb > 200 * 1024) return tfx_set_error(TFX_STATUS_ERR_UNSUPPORTED, "cp_fit_grad: rank too large");
+  const size_t smb = (size_t)R * (R + 16) * es;
+  if ((size_t)R * R * es > 200 * 1024) return tfx_set_error(TFX_STATUS_ERR_UNSUPPORTED, "cp_fit_grad: rank too large");
   cudaError_t e = dtype == TFX_F32
                       ? cudaFuncSetAttribute(k_cp_wp1<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb)
                       : cudaFuncSetAttribute(k_cp_wp1<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
   if (e != cudaSuccess) return tfx_set_cuda_error(e, "cp_fit_grad attribute");
-  const int gb = L * ((R * R + TFX_THREADS - 1) / TFX_THREADS);
+  const dim3 gb(gram_blocks(R), L);
   if (dtype == TFX_F32)
-    k_cp_grams<float><<<gb, TFX_THREADS, 0, st>>>((const float*)W, sh, (double*)(sc + y.gram));
+    k_cp_grams<float><<<gb, 1024, 0, st>>>((const float*)W, sh, (double*)(sc + y.gram));
   else
-    k_cp_grams<double><<<gb, TFX_THREADS, 0, st>>>((const double*)W, sh, (double*)(sc + y.gram));
+    k_cp_grams<double><<<gb, 1024, 0, st>>>((const double*)W, sh, (double*)(sc + y.gram));
   if (int r = done("cp_grams")) return r;
   if (int r = tfx_mttkrp_all(dtype, T, L, dims, R, W, sc + y.M, sc + y.mtt, y.mtt_bytes, stream)) return r;
-  const dim3 grid(L, (maxd + 31) / 32);
+  const dim3 grid((maxd + 15) / 16, L);
   if (dtype == TFX_F32)
     k_cp_wp1<float><<<grid, TFX_THREADS, smb, st>>>((const float*)W, sh, (const double*)(sc + y.gram),
                                                     (const float*)(sc + y.M), 2.f, (float*)grad);
