@@ -216,11 +216,17 @@ int tfx_tensor_norms(int dtype, const void* T, long long N, double* out2, void* 
 size_t tfx_mttkrp_scratch_bytes(int dtype, int L, const int* dims, int R, int mode);
 int tfx_mttkrp(int dtype, const void* T, int L, const int* dims, int R, const void* W, int mode, void* out, void* scratch,
                size_t scratch_bytes, void* stream);
-/* The same product for every mode at once, out in the flat layout (the modes are
- * cut in two halves, so the tensor is read twice instead of L times). */
+/* The same product for every mode at once (the modes are cut in two halves, so
+ * the tensor is read twice instead of L times): out is a HOST array of L device
+ * pointers, d_l x R column-major or, with row_major, row-major; a null one is not
+ * wanted. */
 size_t tfx_mttkrp_all_scratch_bytes(int dtype, int L, const int* dims, int R);
-int tfx_mttkrp_all(int dtype, const void* T, int L, const int* dims, int R, const void* W, void* out, void* scratch,
-                   size_t scratch_bytes, void* stream);
+int tfx_mttkrp_all(int dtype, const void* T, int L, const int* dims, int R, const void* W, void* const* out,
+                   int row_major, void* scratch, size_t scratch_bytes, void* stream);
+/* The flat layout from factors as a caller has them: HOST arrays of L device
+ * pointers and of their row and column strides (elements). */
+int tfx_factors_pack(int dtype, int L, const int* dims, int R, const void* const* W, const long long* rs,
+                     const long long* cs, void* out, void* stream);
 int tfx_cp_full(int dtype, int L, const int* dims, int R, const void* W, void* out, void* stream);
 /* The same product T_(l) KR_l of an FP32 tensor on the 5th-generation tensor
  * cores (GaussNewton.py:401-427 compute_grad's contraction, 411-423): the
@@ -245,6 +251,12 @@ int tfx_cp_wp1(int dtype, int L, const int* dims, int R, const void* W, void* ou
 size_t tfx_cp_fit_grad_scratch_bytes(int dtype, int L, const int* dims, int R);
 int tfx_cp_fit_grad(int dtype, const void* T, int L, const int* dims, int R, const void* W, void* grad, void* scratch,
                     size_t scratch_bytes, void* stream);
+
+/* The same times the device scalar *gl (dtype), into a HOST array of L device
+ * pointers to contiguous d_l x R row-major matrices, null where not wanted;
+ * scratch: tfx_cp_fit_grad_scratch_bytes(). */
+int tfx_cp_fit_backward(int dtype, const void* T, int L, const int* dims, int R, const void* W, const void* gl,
+                        void* const* grads, void* scratch, size_t scratch_bytes, void* stream);
 
 /* ---- sparse (COO) ----------------------------------------------------------
  * TensorFox.py:476-481: int64 (nnz x L) coordinates -> int32 L x nnz; *err = 1

@@ -72,6 +72,35 @@ __global__ void __launch_bounds__(TFX_THREADS) k_cp_full(const T* __restrict__ W
   }
 }
 
+// The factors as a caller has them (any strides) into the flat column-major
+// layout: 32 x 32 tiles through shared memory, read along whichever stride is
+// the shorter.
+struct PackArgs {
+  const void* p[TFX_MAX_ORDER];
+  long long rs[TFX_MAX_ORDER], cs[TFX_MAX_ORDER];
+};
+
+template <class T>
+__global__ void __launch_bounds__(256) k_pack(const __grid_constant__ PackArgs a, const __grid_constant__ CpDims sh,
+                                              T* __restrict__ out) {
+  __shared__ T tile[32][33];
+  const int R = sh.R, nr = (R + 31) / 32;
+  int t = blockIdx.x, m = 0;
+  while (t >= (sh.d[m] + 31) / 32 * nr) t -= (sh.d[m++] + 31) / 32 * nr;
+  const int i0 = t / nr * 32, r0 = t % nr * 32, d = sh.d[m];
+  const T* w = (const T*)a.p[m];
+  const long long rs = a.rs[m], cs = a.cs[m];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const bool along_r = cs <= rs;
+  for (int u = y; u < 32; u += 8) {
+    const int i = along_r ? u : x, r = along_r ? x : u;
+    if (i0 + i < d && r0 + r < R) tile[i][r] = w[(i0 + i) * rs + (r0 + r) * cs];
+  }
+  __syncthreads();
+  for (int u = y; u < 32; u += 8)
+    if (i0 + x < d && r0 + u < R) out[sh.off[m] + (long long)(r0 + u) * d + i0 + x] = tile[x][u];
+}
+
 // Gramians of every mode, G_m = W_m^T W_m (FP64, compensated sums of the
 // working-type products).  A CTA takes a 16 x 16 block on or above the diagonal
 // of one Gramian: 32 rows of its 32 columns at a time through shared memory
@@ -121,20 +150,22 @@ static unsigned gram_blocks(int R) {
   return nb * (nb + 1) / 2;
 }
 
-// out_l = scale (W_l P1_l - M_l), P1_l = o_{m != l} G_m (ascending m, FP64,
-// rounded to the working type in shared memory); M == nullptr means M_l = 0.
-// Grid (ceil(max d / 16), L), 16 rows per CTA; four accumulators a thread, whose
-// compensated chains overlap.
+// out_l = scale (W_l P1_l - M_l) [times *gl], P1_l = o_{m != l} G_m (ascending
+// m, FP64, rounded to the working type in shared memory); M == nullptr means
+// M_l = 0; M and out in the same layout.  Grid (ceil(max d / 16), L), 16 rows per
+// CTA; four accumulators a thread, whose compensated chains overlap.
 template <class T>
-__global__ void __launch_bounds__(TFX_THREADS) k_cp_wp1(const T* __restrict__ W, CpDims sh,
+__global__ void __launch_bounds__(TFX_THREADS) k_cp_wp1(const T* __restrict__ W, const __grid_constant__ CpDims sh,
                                                         const double* __restrict__ gram, const T* __restrict__ M,
-                                                        T scale, T* __restrict__ out) {
+                                                        T scale, const T* __restrict__ gl,
+                                                        const __grid_constant__ mg::Outs out) {
   extern __shared__ __align__(16) char smem[];
   T* sP = (T*)smem;          // [R][R]
   const int l = blockIdx.y, L = sh.L, R = sh.R, RR = R * R, tid = threadIdx.x;
   T* sW = sP + RR;           // [R][16]
+  T* o = (T*)out.p[l];
   const int dl = sh.d[l], r0 = blockIdx.x * 16;
-  if (r0 >= dl) return;
+  if (r0 >= dl || !o) return;
 #pragma unroll 4
   for (int e = tid; e < RR; e += TFX_THREADS) {
     double p = 1.0;
@@ -148,7 +179,7 @@ __global__ void __launch_bounds__(TFX_THREADS) k_cp_wp1(const T* __restrict__ W,
   }
   __syncthreads();
   for (int e = tid; e < 16 * R; e += TFX_THREADS) {
-    const int i = e & 15, r = e >> 4;
+    const int i = out.rows ? e / R : e & 15, r = out.rows ? e - i * R : e >> 4;
     if (r0 + i >= dl) continue;
     Acc<T> s[4];
     int q = 0;
@@ -161,9 +192,11 @@ __global__ void __launch_bounds__(TFX_THREADS) k_cp_wp1(const T* __restrict__ W,
       s[0].add(s[u].hi_or_v());
       if (sizeof(T) == 4) s[0].add((T)s[u].lo_or_0());
     }
-    const size_t o = (size_t)sh.off[l] + (size_t)r * dl + r0 + i;
-    if (M) s[0].add(-M[o]);
-    out[o] = scale * (T)s[0].value();
+    const size_t at = out.rows ? (size_t)(r0 + i) * R + r : (size_t)r * dl + r0 + i;
+    if (M) s[0].add(-M[sh.off[l] + at]);
+    T v = scale * (T)s[0].value();
+    if (gl) v *= *gl;
+    o[at] = v;
   }
 }
 
@@ -172,8 +205,6 @@ __global__ void __launch_bounds__(TFX_THREADS) k_cp_wp1(const T* __restrict__ W,
 using namespace tfx;
 
 extern "C" size_t tfx_mttkrp_all_scratch_bytes(int dtype, int L, const int* dims, int R);
-extern "C" int tfx_mttkrp_all(int dtype, const void* T, int L, const int* dims, int R, const void* W, void* out,
-                              void* scratch, size_t scratch_bytes, void* stream);
 
 static int nsm() {
   static int n = 0;
@@ -224,40 +255,74 @@ extern "C" int tfx_cp_full(int dtype, int L, const int* dims, int R, const void*
   return done("cp_full");
 }
 
+extern "C" int tfx_factors_pack(int dtype, int L, const int* dims, int R, const void* const* W, const long long* rs,
+                                const long long* cs, void* out, void* stream) {
+  CpDims sh;
+  if (cpdims(sh, L, dims, R) || !W || !rs || !cs || !out) return tfx_set_error(TFX_STATUS_ERR_ARG, "factors_pack args");
+  PackArgs a;
+  long long nb = 0;
+  for (int l = 0; l < L; ++l) {
+    if (!W[l]) return tfx_set_error(TFX_STATUS_ERR_ARG, "factors_pack pointer");
+    a.p[l] = W[l];
+    a.rs[l] = rs[l];
+    a.cs[l] = cs[l];
+    nb += (long long)((dims[l] + 31) / 32) * ((R + 31) / 32);
+  }
+  if (dtype == TFX_F64) k_pack<double><<<(unsigned)nb, 256, 0, (cudaStream_t)stream>>>(a, sh, (double*)out);
+  else k_pack<float><<<(unsigned)nb, 256, 0, (cudaStream_t)stream>>>(a, sh, (float*)out);
+  return done("factors_pack");
+}
+
+// Gramians, then scale (W_l P1_l - M_l) [*gl] for every mode
+static int grams_and_wp1(int dtype, const CpDims& sh, const void* W, double* gram, const void* M, double scale,
+                         const void* gl, const mg::Outs& out, cudaStream_t st, const char* where) {
+  const int L = sh.L, R = sh.R;
+  const size_t es = dtype == TFX_F64 ? 8 : 4;
+  if ((size_t)R * R * es > 200 * 1024) return tfx_set_error(TFX_STATUS_ERR_UNSUPPORTED, where);
+  const size_t smb = (size_t)R * (R + 16) * es;
+  cudaError_t e = dtype == TFX_F32
+                      ? cudaFuncSetAttribute(k_cp_wp1<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb)
+                      : cudaFuncSetAttribute(k_cp_wp1<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
+  if (e != cudaSuccess) return tfx_set_cuda_error(e, "cp_wp1 attribute");
+  int maxd = 0;
+  for (int l = 0; l < L; ++l) maxd = std::max(maxd, sh.d[l]);
+  const dim3 gb(gram_blocks(R), L), grid((maxd + 15) / 16, L);
+  if (dtype == TFX_F32) {
+    k_cp_grams<float><<<gb, 1024, 0, st>>>((const float*)W, sh, gram);
+    k_cp_wp1<float><<<grid, TFX_THREADS, smb, st>>>((const float*)W, sh, gram, (const float*)M, (float)scale,
+                                                    (const float*)gl, out);
+  } else {
+    k_cp_grams<double><<<gb, 1024, 0, st>>>((const double*)W, sh, gram);
+    k_cp_wp1<double><<<grid, TFX_THREADS, smb, st>>>((const double*)W, sh, gram, (const double*)M, scale,
+                                                     (const double*)gl, out);
+  }
+  if ((e = cudaGetLastError()) != cudaSuccess) return tfx_set_cuda_error(e, "cp_wp1");
+  tfx_count_launch(2);
+  return TFX_STATUS_OK;
+}
+
+// a flat vector's blocks
+static mg::Outs flat_outs(const CpDims& sh, void* out, size_t es, int rows) {
+  mg::Outs o = {};
+  o.rows = rows;
+  for (int l = 0; l < sh.L; ++l) o.p[l] = (char*)out + (size_t)sh.off[l] * es;
+  return o;
+}
+
 extern "C" size_t tfx_cp_wp1_scratch_bytes(int L, int R) { return (size_t)L * R * R * 8; }
 
 extern "C" int tfx_cp_wp1(int dtype, int L, const int* dims, int R, const void* W, void* out, void* scratch,
                           void* stream) {
   CpDims sh;
   if (cpdims(sh, L, dims, R) || !W || !out || !scratch) return tfx_set_error(TFX_STATUS_ERR_ARG, "cp_wp1 args");
-  cudaStream_t st = (cudaStream_t)stream;
-  int maxd = 0;
-  for (int l = 0; l < L; ++l) maxd = std::max(maxd, dims[l]);
-  const dim3 gb(gram_blocks(R), L), grid((maxd + 15) / 16, L);
-  const size_t es = dtype == TFX_F64 ? 8 : 4;
-  const size_t smb = (size_t)R * (R + 16) * es;
-  if ((size_t)R * R * es > 200 * 1024) return tfx_set_error(TFX_STATUS_ERR_UNSUPPORTED, "cp_wp1: rank too large");
-  cudaError_t e = dtype == TFX_F32
-                      ? cudaFuncSetAttribute(k_cp_wp1<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb)
-                      : cudaFuncSetAttribute(k_cp_wp1<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
-  if (e != cudaSuccess) return tfx_set_cuda_error(e, "cp_wp1 attribute");
-  if (dtype == TFX_F32) {
-    k_cp_grams<float><<<gb, 1024, 0, st>>>((const float*)W, sh, (double*)scratch);
-    if (int r = done("cp_grams")) return r;
-    k_cp_wp1<float><<<grid, TFX_THREADS, smb, st>>>((const float*)W, sh, (const double*)scratch, nullptr, 1.f,
-                                                    (float*)out);
-  } else {
-    k_cp_grams<double><<<gb, 1024, 0, st>>>((const double*)W, sh, (double*)scratch);
-    if (int r = done("cp_grams")) return r;
-    k_cp_wp1<double><<<grid, TFX_THREADS, smb, st>>>((const double*)W, sh, (const double*)scratch, nullptr, 1.0,
-                                                     (double*)out);
-  }
-  return done("cp_wp1");
+  return grams_and_wp1(dtype, sh, W, (double*)scratch, nullptr, 1.0, nullptr,
+                       flat_outs(sh, out, dtype == TFX_F64 ? 8 : 4, 0), (cudaStream_t)stream,
+                       "cp_wp1: rank too large");
 }
 
 // grad_l = 2 (W_l P1_l - T_(l) KR_l) for every mode: the gradient of
-// ||T - [[W]]||^2 (twice GaussNewton.py:401-427's g), flat layout.  Scratch:
-// the Gramians, the MTTKRPs and the MTTKRP split-K partials.
+// ||T - [[W]]||^2 (twice GaussNewton.py:401-427's g).  Scratch: the Gramians, the
+// MTTKRPs and what those need.
 struct FitGradLayout {
   size_t gram, M, mtt, mtt_bytes, total;
 };
@@ -281,36 +346,38 @@ extern "C" size_t tfx_cp_fit_grad_scratch_bytes(int dtype, int L, const int* dim
   return fit_grad_layout(dtype, L, dims, R).total;
 }
 
+static int fit_grad(int dtype, const void* T, const CpDims& sh, const void* W, const void* gl, const mg::Outs& out,
+                    void* scratch, size_t scratch_bytes, cudaStream_t st) {
+  const FitGradLayout y = fit_grad_layout(dtype, sh.L, sh.d, sh.R);
+  if (scratch_bytes < y.total) return tfx_set_error(TFX_STATUS_ERR_ARG, "cp_fit_grad scratch too small");
+  const size_t es = dtype == TFX_F64 ? 8 : 4;
+  if ((size_t)sh.R * sh.R * es > 200 * 1024)
+    return tfx_set_error(TFX_STATUS_ERR_UNSUPPORTED, "cp_fit_grad: rank too large");
+  char* sc = (char*)scratch;
+  mg::Outs M = flat_outs(sh, sc + y.M, es, out.rows);
+  for (int l = 0; l < sh.L; ++l)
+    if (!out.p[l]) M.p[l] = nullptr;
+  if (int r = mg::all_modes(dtype, T, sh, W, M, sc + y.mtt, y.mtt_bytes, st)) return r;
+  return grams_and_wp1(dtype, sh, W, (double*)(sc + y.gram), sc + y.M, 2.0, gl, out, st,
+                       "cp_fit_grad: rank too large");
+}
+
 extern "C" int tfx_cp_fit_grad(int dtype, const void* T, int L, const int* dims, int R, const void* W, void* grad,
                                void* scratch, size_t scratch_bytes, void* stream) {
   CpDims sh;
   if (cpdims(sh, L, dims, R) || !T || !W || !grad || !scratch) return tfx_set_error(TFX_STATUS_ERR_ARG, "cp_fit_grad args");
-  const FitGradLayout y = fit_grad_layout(dtype, L, dims, R);
-  if (scratch_bytes < y.total) return tfx_set_error(TFX_STATUS_ERR_ARG, "cp_fit_grad scratch too small");
-  cudaStream_t st = (cudaStream_t)stream;
-  const size_t es = dtype == TFX_F64 ? 8 : 4;
-  char* sc = (char*)scratch;
-  int maxd = 0;
-  for (int l = 0; l < L; ++l) maxd = std::max(maxd, dims[l]);
-  const size_t smb = (size_t)R * (R + 16) * es;
-  if ((size_t)R * R * es > 200 * 1024) return tfx_set_error(TFX_STATUS_ERR_UNSUPPORTED, "cp_fit_grad: rank too large");
-  cudaError_t e = dtype == TFX_F32
-                      ? cudaFuncSetAttribute(k_cp_wp1<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb)
-                      : cudaFuncSetAttribute(k_cp_wp1<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
-  if (e != cudaSuccess) return tfx_set_cuda_error(e, "cp_fit_grad attribute");
-  const dim3 gb(gram_blocks(R), L);
-  if (dtype == TFX_F32)
-    k_cp_grams<float><<<gb, 1024, 0, st>>>((const float*)W, sh, (double*)(sc + y.gram));
-  else
-    k_cp_grams<double><<<gb, 1024, 0, st>>>((const double*)W, sh, (double*)(sc + y.gram));
-  if (int r = done("cp_grams")) return r;
-  if (int r = tfx_mttkrp_all(dtype, T, L, dims, R, W, sc + y.M, sc + y.mtt, y.mtt_bytes, stream)) return r;
-  const dim3 grid((maxd + 15) / 16, L);
-  if (dtype == TFX_F32)
-    k_cp_wp1<float><<<grid, TFX_THREADS, smb, st>>>((const float*)W, sh, (const double*)(sc + y.gram),
-                                                    (const float*)(sc + y.M), 2.f, (float*)grad);
-  else
-    k_cp_wp1<double><<<grid, TFX_THREADS, smb, st>>>((const double*)W, sh, (const double*)(sc + y.gram),
-                                                     (const double*)(sc + y.M), 2.0, (double*)grad);
-  return done("cp_fit_grad");
+  return fit_grad(dtype, T, sh, W, nullptr, flat_outs(sh, grad, dtype == TFX_F64 ? 8 : 4, 0), scratch, scratch_bytes,
+                  (cudaStream_t)stream);
+}
+
+extern "C" int tfx_cp_fit_backward(int dtype, const void* T, int L, const int* dims, int R, const void* W,
+                                   const void* gl, void* const* grads, void* scratch, size_t scratch_bytes,
+                                   void* stream) {
+  CpDims sh;
+  if (cpdims(sh, L, dims, R) || !T || !W || !gl || !grads || !scratch)
+    return tfx_set_error(TFX_STATUS_ERR_ARG, "cp_fit_backward args");
+  mg::Outs o = {};
+  o.rows = 1;
+  for (int l = 0; l < L; ++l) o.p[l] = grads[l];
+  return fit_grad(dtype, T, sh, W, gl, o, scratch, scratch_bytes, (cudaStream_t)stream);
 }

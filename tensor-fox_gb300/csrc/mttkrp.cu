@@ -148,7 +148,7 @@ constexpr int MY = 16;
 template <class T>
 __global__ void __launch_bounds__(32 * MY) k_modes(const T* __restrict__ X, const T* __restrict__ kr,
                                                    const __grid_constant__ CpDims sh, int g0, int g1, int only,
-                                                   unsigned D, int ldp, T* __restrict__ out) {
+                                                   unsigned D, int ldp, const __grid_constant__ Outs out) {
   __shared__ T hi[MY][32], lo[MY][32];
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
   const int c = blockIdx.y * 32 + x;
@@ -160,9 +160,11 @@ __global__ void __launch_bounds__(32 * MY) k_modes(const T* __restrict__ X, cons
       kp += (size_t)(D / sh.d[m]) * ldp;
       i -= sh.d[m++];
     }
+  T* o = (T*)out.p[m];
+  if (!o) return;
   const unsigned dm = sh.d[m], n = D / dm;
   unsigned inner = 1;
-  for (int o = m + 1; o < g1; ++o) inner *= sh.d[o];
+  for (int q = m + 1; q < g1; ++q) inner *= sh.d[q];
   Acc<T> s;
   if (c < ldp) {
     if (inner == n || inner == 1) {  // the first or the last mode: a fixed stride
@@ -188,7 +190,7 @@ __global__ void __launch_bounds__(32 * MY) k_modes(const T* __restrict__ X, cons
       t.add(hi[q][x]);
       if (sizeof(T) == 4) t.add(lo[q][x]);
     }
-    out[(only >= 0 ? 0 : sh.off[m]) + (size_t)c * dm + i] = (T)t.value();
+    o[out.rows ? (size_t)i * sh.R + c : (size_t)c * dm + i] = (T)t.value();
   }
 }
 
@@ -265,17 +267,21 @@ static int best_cut(int es, const CpDims& sh, int sms) {
   return least < one ? cut : 0;
 }
 
-// out: the column-major D x R product of one mode (only >= 0), or the flat
-// MTTKRPs, of which the group's modes are written
+// the group's modes (only >= 0: that one) into out
 template <class T>
-static cudaError_t run_group(const Group& g, const T* X, const T* W, const CpDims& sh, int only, T* out, char* scratch,
-                             cudaStream_t st, int* launches) {
+static cudaError_t run_group(const Group& g, const T* X, const T* W, const CpDims& sh, int only, const Outs& out,
+                             char* scratch, cudaStream_t st, int* launches) {
   const int g0 = g.p.g0, g1 = g.p.g1;
-  if (g1 - g0 == 1)
-    return run<T>(g.p, X, W, sh, only >= 0 ? out : out + sh.off[g0], true, scratch, st, launches);
+  bool any = false;
+  for (int m = g0; m < g1; ++m) any = any || (out.p[m] && (only < 0 || only == m));
+  if (!any) return cudaSuccess;
+  if (g1 - g0 == 1) {
+    const Out<T> o = {(T*)out.p[g0], out.rows ? sh.R : 1, out.rows ? 1 : sh.d[g0]};
+    return run<T>(g.p, X, W, sh, o, scratch, st, launches);
+  }
   T* XG = (T*)(scratch + g.p.total());
   T* kr = (T*)(scratch + g.p.total() + g.x_bytes);
-  cudaError_t e = run<T>(g.p, X, W, sh, XG, false, scratch, st, launches);
+  cudaError_t e = run<T>(g.p, X, W, sh, Out<T>{XG, 0, 0}, scratch, st, launches);
   if (e != cudaSuccess) return e;
   const unsigned D = (unsigned)g.p.w.D;
   long long rows = 0, idx = 0;
@@ -291,6 +297,13 @@ static cudaError_t run_group(const Group& g, const T* X, const T* W, const CpDim
                                                                                    out);
   *launches += 2;
   return cudaGetLastError();
+}
+
+static cudaError_t run_group(int dtype, const Group& g, const void* X, const void* W, const CpDims& sh, int only,
+                             const Outs& out, void* scratch, cudaStream_t st, int* launches) {
+  if (dtype == TFX_F64)
+    return run_group<double>(g, (const double*)X, (const double*)W, sh, only, out, (char*)scratch, st, launches);
+  return run_group<float>(g, (const float*)X, (const float*)W, sh, only, out, (char*)scratch, st, launches);
 }
 
 }  // namespace mg
@@ -347,11 +360,9 @@ extern "C" int tfx_mttkrp(int dtype, const void* T, int L, const int* dims, int 
   const mg::Group g = mg::best_single((int)es, sh, mode, nsm());
   if (g.total() <= scratch_bytes && ((uintptr_t)scratch & 15) == 0) {
     int nl = 0;
-    const cudaError_t e =
-        dtype == TFX_F32
-            ? mg::run_group<float>(g, (const float*)T, (const float*)W, sh, mode, (float*)out, (char*)scratch, st, &nl)
-            : mg::run_group<double>(g, (const double*)T, (const double*)W, sh, mode, (double*)out, (char*)scratch, st,
-                                    &nl);
+    mg::Outs o = {};
+    o.p[mode] = out;
+    const cudaError_t e = mg::run_group(dtype, g, T, W, sh, mode, o, scratch, st, &nl);
     if (e != cudaSuccess) return tfx_set_cuda_error(e, "mttkrp");
     tfx_count_launch(nl);
     return TFX_STATUS_OK;
@@ -390,35 +401,33 @@ extern "C" size_t tfx_mttkrp_all_scratch_bytes(int dtype, int L, const int* dims
     for (int l = 0; l < L; ++l) n = std::max(n, mg::best_single(es, sh, l, nsm()).total());
   else
     n = std::max(mg::group(es, sh, 0, s, -1, nsm()).total(), mg::group(es, sh, s, L, -1, nsm()).total());
-  return n;
+  return n + 256;  // to align within
 }
 
-extern "C" int tfx_mttkrp_all(int dtype, const void* T, int L, const int* dims, int R, const void* W, void* out,
-                              void* scratch, size_t scratch_bytes, void* stream) {
+int tfx::mg::all_modes(int dtype, const void* T, const CpDims& sh, const void* W, const Outs& out, void* scratch,
+                       size_t scratch_bytes, cudaStream_t st) {
+  const int es = dtype == TFX_F64 ? 8 : 4, s = best_cut(es, sh, nsm());
+  const size_t skip = (256 - ((uintptr_t)scratch & 255)) & 255;
+  scratch_bytes = scratch_bytes > skip ? scratch_bytes - skip : 0;
+  scratch = (char*)scratch + skip;
+  int nl = 0;
+  for (int h = 0; h < (s ? 2 : sh.L); ++h) {  // two halves, or mode by mode
+    const Group g = s ? group(es, sh, h ? s : 0, h ? sh.L : s, -1, nsm()) : best_single(es, sh, h, nsm());
+    if (g.total() > scratch_bytes) return tfx_set_error(TFX_STATUS_ERR_ARG, "mttkrp_all scratch too small");
+    const cudaError_t e = run_group(dtype, g, T, W, sh, s ? -1 : h, out, scratch, st, &nl);
+    if (e != cudaSuccess) return tfx_set_cuda_error(e, "mttkrp_all");
+  }
+  tfx_count_launch(nl);
+  return TFX_STATUS_OK;
+}
+
+extern "C" int tfx_mttkrp_all(int dtype, const void* T, int L, const int* dims, int R, const void* W, void* const* out,
+                              int row_major, void* scratch, size_t scratch_bytes, void* stream) {
   CpDims sh;
   if (cpdims(sh, L, dims, R) || !T || !W || !out || !scratch)
     return tfx_set_error(TFX_STATUS_ERR_ARG, "mttkrp_all args");
-  const int es = dtype == TFX_F64 ? 8 : 4, s = mg::best_cut(es, sh, nsm());
-  if (s == 0) {
-    for (int l = 0; l < L; ++l)
-      if (int r = tfx_mttkrp(dtype, T, L, dims, R, W, l, (char*)out + (size_t)sh.off[l] * es, scratch, scratch_bytes,
-                             stream))
-        return r;
-    return TFX_STATUS_OK;
-  }
-  cudaStream_t st = (cudaStream_t)stream;
-  for (int h = 0; h < 2; ++h) {
-    const mg::Group g = mg::group(es, sh, h ? s : 0, h ? L : s, -1, nsm());
-    if (g.total() > scratch_bytes || ((uintptr_t)scratch & 15) != 0)
-      return tfx_set_error(TFX_STATUS_ERR_ARG, "mttkrp_all scratch too small");
-    int nl = 0;
-    const cudaError_t e =
-        dtype == TFX_F32
-            ? mg::run_group<float>(g, (const float*)T, (const float*)W, sh, -1, (float*)out, (char*)scratch, st, &nl)
-            : mg::run_group<double>(g, (const double*)T, (const double*)W, sh, -1, (double*)out, (char*)scratch, st,
-                                    &nl);
-    if (e != cudaSuccess) return tfx_set_cuda_error(e, "mttkrp_all");
-    tfx_count_launch(nl);
-  }
-  return TFX_STATUS_OK;
+  mg::Outs o = {};
+  o.rows = row_major;
+  for (int l = 0; l < L; ++l) o.p[l] = out[l];
+  return mg::all_modes(dtype, T, sh, W, o, scratch, scratch_bytes, (cudaStream_t)stream);
 }

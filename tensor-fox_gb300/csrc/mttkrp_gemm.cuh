@@ -118,14 +118,33 @@ cudaError_t gemm_f32(const Plan& p, const float* T, const float* krF, const floa
 cudaError_t gemm_f64(const Plan& p, const double* T, const double* krF, const double* krO, double* part,
                      cudaStream_t st);
 
+// Where a product goes: element (d, r) at p[d * sd + r * sr], r < R; sd = 0: the
+// padded rows [D][ldp] of a group that is contracted further.
+template <class T>
+struct Out {
+  T* p;
+  long long sd, sr;
+};
+
 // The sum over the ks partials part[.][D][ldp], compensated in FP32: 32 outputs
 // a CTA, the partials dealt to SG groups of threads whose sums are added in a
-// fixed order.  COL: out[r * D + d]; else out[d * ldp + r].
+// fixed order.
 constexpr int SG = 16;
 
-template <class T, bool COL>
+template <class T>
+__device__ __forceinline__ void put(const Out<T>& out, long long e, int ldp, int R, T v) {
+  if (out.sd == 0) {
+    out.p[e] = v;
+    return;
+  }
+  const long long d = e / ldp;
+  const int r = (int)(e - d * ldp);
+  if (r < R) out.p[d * out.sd + r * out.sr] = v;
+}
+
+template <class T>
 __global__ void __launch_bounds__(32 * SG) k_sum(const T* __restrict__ part, long long D, int R, int ldp, int ks,
-                                                 T* __restrict__ out) {
+                                                 Out<T> out) {
   __shared__ T hi[SG][32], lo[SG][32];
   const long long n = D * ldp;
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
@@ -145,26 +164,20 @@ __global__ void __launch_bounds__(32 * SG) k_sum(const T* __restrict__ part, lon
       t.add(hi[j][x]);
       if (sizeof(T) == 4) t.add(lo[j][x]);
     }
-    const long long d = e / ldp;
-    const int r = (int)(e - d * ldp);
-    if (!COL) out[e] = (T)t.value();
-    else if (r < R) out[(size_t)r * D + d] = (T)t.value();
+    put(out, e, ldp, R, (T)t.value());
   }
 }
 
 // The same for few partials: one output a thread.
-template <class T, bool COL>
+template <class T>
 __global__ void __launch_bounds__(256) k_sum_few(const T* __restrict__ part, long long D, int R, int ldp, int ks,
-                                                 T* __restrict__ out) {
+                                                 Out<T> out) {
   const long long n = D * ldp, e = (long long)blockIdx.x * 256 + threadIdx.x;
   if (e >= n) return;
   Acc<T> s;
 #pragma unroll 4
   for (int k = 0; k < ks; ++k) s.add(__ldcs(part + (size_t)k * n + e));
-  const long long d = e / ldp;
-  const int r = (int)(e - d * ldp);
-  if (!COL) out[e] = (T)s.value();
-  else if (r < R) out[(size_t)r * D + d] = (T)s.value();
+  put(out, e, ldp, R, (T)s.value());
 }
 
 // KR_F as [column block][nF rows padded to chunks][BN] (zeros in the padding)
@@ -207,10 +220,10 @@ inline cudaError_t gemm(const Plan& p, const double* T, const double* krF, const
   return gemm_f64(p, T, krF, krO, part, st);
 }
 
-// One product: out is column-major D x R (col) or [D][ldp].  scratch: 256-byte
-// aligned, p.total() bytes.  *launches counts the kernels.
+// One product.  scratch: 16-byte aligned, p.total() bytes.  *launches counts the
+// kernels.
 template <class T>
-inline cudaError_t run(Plan p, const T* X, const T* W, const CpDims& sh, T* out, bool col, void* scratch,
+inline cudaError_t run(Plan p, const T* X, const T* W, const CpDims& sh, Out<T> out, void* scratch,
                        cudaStream_t st, int* launches) {
   constexpr int PV = 16 / sizeof(T);  // values a 16-byte copy
   const long long ext = p.last ? p.w.D : p.w.dF;
@@ -229,8 +242,8 @@ inline cudaError_t run(Plan p, const T* X, const T* W, const CpDims& sh, T* out,
                                                     p.w.ldp, krF, krO);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  const bool direct = !col && p.ks == 1;
-  if ((e = gemm(p, X, krF, krO, direct ? out : part, st)) != cudaSuccess) return e;
+  const bool direct = out.sd == 0 && p.ks == 1;
+  if ((e = gemm(p, X, krF, krO, direct ? out.p : part, st)) != cudaSuccess) return e;
   *launches += direct ? 2 : 3;
   if (direct) return cudaSuccess;
   const long long n = p.w.D * p.w.ldp;
@@ -238,15 +251,25 @@ inline cudaError_t run(Plan p, const T* X, const T* W, const CpDims& sh, T* out,
   // (147456 outputs of 2 partials: 12 us dealt to groups, 3 us this way)
   if (p.ks <= 8 || n >= (1 << 20)) {
     const unsigned sb = (unsigned)((n + 255) / 256);
-    if (col) k_sum_few<T, true><<<sb, 256, 0, st>>>(part, p.w.D, sh.R, p.w.ldp, p.ks, out);
-    else k_sum_few<T, false><<<sb, 256, 0, st>>>(part, p.w.D, sh.R, p.w.ldp, p.ks, out);
+    k_sum_few<T><<<sb, 256, 0, st>>>(part, p.w.D, sh.R, p.w.ldp, p.ks, out);
     return cudaGetLastError();
   }
   const unsigned sb = (unsigned)((n + 31) / 32);
-  if (col) k_sum<T, true><<<sb, 32 * SG, 0, st>>>(part, p.w.D, sh.R, p.w.ldp, p.ks, out);
-  else k_sum<T, false><<<sb, 32 * SG, 0, st>>>(part, p.w.D, sh.R, p.w.ldp, p.ks, out);
+  k_sum<T><<<sb, 32 * SG, 0, st>>>(part, p.w.D, sh.R, p.w.ldp, p.ks, out);
   return cudaGetLastError();
 }
+
+// Where the MTTKRPs of every mode go: p[m] (null: not wanted) d_m x R,
+// column-major or (rows) row-major.
+struct Outs {
+  void* p[TFX_MAX_ORDER];
+  int rows;
+};
+
+// The MTTKRPs of every mode in out.p (mttkrp.cu); scratch as
+// tfx_mttkrp_all_scratch_bytes().
+int all_modes(int dtype, const void* T, const CpDims& sh, const void* W, const Outs& out, void* scratch,
+              size_t scratch_bytes, cudaStream_t st);
 
 }  // namespace mg
 }  // namespace tfx

@@ -5,17 +5,31 @@ import torch
 from . import _lib
 
 
+_FOUND = False
+
+
 def require_cuda():
+    global _FOUND
+    if _FOUND:        # asking again costs more than a launch
+        return
     if not torch.cuda.is_available():
         raise RuntimeError("tensorfox_gb300 needs a CUDA device (GB300, sm_103a); none is visible")
     _lib.load()
+    _FOUND = True
 
 
 def device():
     return torch.device("cuda", torch.cuda.current_device())
 
 
+_RAW_STREAM = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream():
+    """The current stream's handle (without a Stream object where torch has the
+    call for that)."""
+    if _RAW_STREAM is not None:
+        return int(_RAW_STREAM(torch.cuda.current_device()))
     return ctypes_stream(torch.cuda.current_stream())
 
 

@@ -50,13 +50,17 @@ ALL_SHAPES = [((200, 31, 33), 20), ((31, 33, 200), 20), ((70, 75, 80), 50), ((40
 @pytest.mark.parametrize("dims,R", ALL_SHAPES)
 def test_mttkrp_all_modes(dims, R, dtype):
     import tensorfox_gb300 as tfx
-    from tensorfox_gb300.autograd import mttkrp_all, _columns
+    from tensorfox_gb300.autograd import mttkrp_all, _flat
     g = torch.Generator(device="cuda").manual_seed(sum(dims) + R)
     L = len(dims)
     T = torch.randn(dims, device="cuda", generator=g, dtype=dtype)
     W = [torch.randn((d, R), device="cuda", generator=g, dtype=dtype) for d in dims]
+    # the flat layout from factors of any strides
     flat = torch.cat([w.t().reshape(-1) for w in W])
-    every = _columns(mttkrp_all(T, flat, list(dims), R), list(dims), R)
+    assert torch.equal(_flat(W), flat)
+    assert torch.equal(_flat([w.t().contiguous().t() for w in W]), flat)
+    assert torch.equal(_flat([torch.stack([w, w], 2)[:, :, 1] for w in W]), flat)
+    every = mttkrp_all(T, flat, list(dims), R)
     s = "abcdef"[:L]
     for l in range(L):
         rest = [m for m in range(L) if m != l]
