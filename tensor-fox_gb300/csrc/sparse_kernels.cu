@@ -373,75 +373,104 @@ __global__ void __launch_bounds__(256) k_factors_bf16(CooShape sh, const float* 
 }
 
 // FP32 residual with R % 4 == 0: 16-byte gathers of the factor rows (when
-// aligned), the model summed in a fixed order.
-__global__ void __launch_bounds__(256) k_sparse_residual_f4(const int* __restrict__ idx32, const float* __restrict__ vals,
+// aligned), the model summed in a fixed order.  Bound by the gathers from L2:
+// LPE lanes share an entry (4 from R = 12 on, 2 at 8, 1 at 4), so that a request
+// takes whole rows (8 rows of 64 bytes at R = 16 instead of a 16-byte piece of
+// 32 rows), two entries of a lane in flight on 32 warps a SM.  20000^3, 1e7
+// entries, R = 16: 211 us = 9.1 TB/s of factor rows (one lane an entry 401 us;
+// four entries in flight on 16 warps 337).
+template <int LPE>
+__global__ void __launch_bounds__(256, 4) k_sparse_residual_f4(const int* __restrict__ idx32, const float* __restrict__ vals,
                                                             long long nnz, CooShape sh,
                                                             const float* const* __restrict__ Wrow,
                                                             double* __restrict__ partial) {
+  constexpr int U3 = 2, UG = 2, EPW = 32 / LPE;  // entries in flight a lane (third order, others); entries a warp
   __shared__ double red[8];
   Acc<float> acc;
   const int R = sh.R, L = sh.L;
+  const int lane = threadIdx.x & 31, q = lane % LPE, slot = lane / LPE;
   bool al = true;
   for (int l = 0; l < L; ++l) al = al && ((unsigned long long)Wrow[l] & 15ull) == 0;
-  const long long S = (long long)gridDim.x * blockDim.x;
+  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
+  // the lanes of an entry add their parts (the same in all of them), one squares
+  auto close = [&](float m, float v, bool on) {
+#pragma unroll
+    for (int o = 1; o < LPE; o <<= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+    const float d = v - m;
+    if (on && q == 0) acc.fma_(d, d);
+  };
   if (L == 3) {
-    // third order: two entries a pass, their coordinates and then all six
-    // factor rows in flight together (the general loop indexes its row
-    // pointers at run time and waits on each mode in turn); products, sums
-    // and the order of the squared differences are those of the general loop
-    const float* W0 = Wrow[0];
-    const float* W1 = Wrow[1];
-    const float* W2 = Wrow[2];
-    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += 2 * S) {
-      const long long k2 = k + S;
-      const bool two = k2 < nnz;
-      const int a0 = idx32[k], b0 = idx32[nnz + k], c0 = idx32[2 * nnz + k];
-      const int a1 = two ? idx32[k2] : 0, b1 = two ? idx32[nnz + k2] : 0, c1 = two ? idx32[2 * nnz + k2] : 0;
-      const float v0 = vals[k], v1 = two ? vals[k2] : 0.f;
-      const float* x0 = W0 + (size_t)a0 * R;
-      const float* y0 = W1 + (size_t)b0 * R;
-      const float* z0 = W2 + (size_t)c0 * R;
-      const float* x1 = W0 + (size_t)a1 * R;
-      const float* y1 = W1 + (size_t)b1 * R;
-      const float* z1 = W2 + (size_t)c1 * R;
-      float m0 = 0.f, m1 = 0.f;
-#pragma unroll 4
-      for (int r = 0; r < R; r += 4) {
-        float4 p = ld4(x0 + r, al), q = ld4(x1 + r, al);
-        const float4 u0 = ld4(y0 + r, al), u1 = ld4(y1 + r, al);
-        const float4 t0 = ld4(z0 + r, al), t1 = ld4(z1 + r, al);
-        p.x *= u0.x; p.y *= u0.y; p.z *= u0.z; p.w *= u0.w;
-        p.x *= t0.x; p.y *= t0.y; p.z *= t0.z; p.w *= t0.w;
-        q.x *= u1.x; q.y *= u1.y; q.z *= u1.z; q.w *= u1.w;
-        q.x *= t1.x; q.y *= t1.y; q.z *= t1.z; q.w *= t1.w;
-        m0 += (p.x + p.y) + (p.z + p.w);
-        m1 += (q.x + q.y) + (q.z + q.w);
+    const float* W0 = Wrow[0] + 4 * q;
+    const float* W1 = Wrow[1] + 4 * q;
+    const float* W2 = Wrow[2] + 4 * q;
+    for (long long b = warp * (EPW * U3); b < nnz; b += warps * (EPW * U3)) {
+      int i0[U3], i1[U3], i2[U3];
+      float v[U3], m[U3];
+#pragma unroll
+      for (int u = 0; u < U3; ++u) {
+        const long long k = b + slot + EPW * u;
+        const bool in = k < nnz;
+        i0[u] = in ? idx32[k] : 0;
+        i1[u] = in ? idx32[nnz + k] : 0;
+        i2[u] = in ? idx32[2 * nnz + k] : 0;
+        v[u] = in ? vals[k] : 0.f;
+        m[u] = 0.f;
       }
-      const float d0 = v0 - m0;
-      acc.fma_(d0, d0);
-      if (two) {
-        const float d1 = v1 - m1;
-        acc.fma_(d1, d1);
+      for (int r = 0; r < R; r += 4 * LPE) {
+        if (r + 4 * q < R) {
+          float4 x[U3], y[U3], z[U3];
+#pragma unroll
+          for (int u = 0; u < U3; ++u) {
+            x[u] = ld4(W0 + (size_t)i0[u] * R + r, al);
+            y[u] = ld4(W1 + (size_t)i1[u] * R + r, al);
+            z[u] = ld4(W2 + (size_t)i2[u] * R + r, al);
+          }
+#pragma unroll
+          for (int u = 0; u < U3; ++u)
+            m[u] += (x[u].x * y[u].x * z[u].x + x[u].y * y[u].y * z[u].y) +
+                    (x[u].z * y[u].z * z[u].z + x[u].w * y[u].w * z[u].w);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U3; ++u) close(m[u], v[u], b + slot + EPW * u < nnz);
+    }
+  } else {
+    for (long long b = warp * (EPW * UG); b < nnz; b += warps * (EPW * UG)) {
+      float m[UG] = {0.f, 0.f};
+      for (int r = 0; r < R; r += 4 * LPE) {
+        if (r + 4 * q < R) {
+          float4 p[UG];
+          for (int l = 0; l < L; ++l) {
+            const float* w = Wrow[l] + 4 * q + r;
+            int ix[UG];
+#pragma unroll
+            for (int u = 0; u < UG; ++u) {
+              const long long k = b + slot + EPW * u;
+              ix[u] = k < nnz ? idx32[(size_t)l * nnz + k] : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < UG; ++u) {
+              const float4 x = ld4(w + (size_t)ix[u] * R, al);
+              if (l == 0) p[u] = x;
+              else {
+                p[u].x *= x.x;
+                p[u].y *= x.y;
+                p[u].z *= x.z;
+                p[u].w *= x.w;
+              }
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < UG; ++u) m[u] += (p[u].x + p[u].y) + (p[u].z + p[u].w);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < UG; ++u) {
+        const long long k = b + slot + EPW * u;
+        close(m[u], k < nnz ? vals[k] : 0.f, k < nnz);
       }
     }
-  } else
-  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += S) {
-    const float* w[TFX_MAX_ORDER];
-    for (int l = 0; l < L; ++l) w[l] = Wrow[l] + (size_t)idx32[(size_t)l * nnz + k] * R;
-    float model = 0.f;
-    for (int r = 0; r < R; r += 4) {
-      float4 p = ld4(w[0] + r, al);
-      for (int l = 1; l < L; ++l) {
-        const float4 x = ld4(w[l] + r, al);
-        p.x *= x.x;
-        p.y *= x.y;
-        p.z *= x.z;
-        p.w *= x.w;
-      }
-      model += (p.x + p.y) + (p.z + p.w);
-    }
-    const float df = vals[k] - model;
-    acc.fma_(df, df);
   }
   acc.warp_reduce();
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc.value();
@@ -783,9 +812,15 @@ extern "C" int tfx_sparse_residual(int dtype, const int* idx32, const void* vals
   cudaStream_t st = (cudaStream_t)stream;
   const int blocks = (int)std::max<long long>(1, std::min<long long>((nnz + 255) / 256, 8LL * sms()));
   double* partial = (double*)scratch;
-  if (dtype == TFX_F32 && R % 4 == 0)
-    k_sparse_residual_f4<<<blocks, 256, 0, st>>>(idx32, (const float*)vals, nnz, sh, (const float* const*)Wrow_dev,
-                                                 partial);
+  if (dtype == TFX_F32 && R % 4 == 0 && R >= 12)
+    k_sparse_residual_f4<4><<<blocks, 256, 0, st>>>(idx32, (const float*)vals, nnz, sh,
+                                                    (const float* const*)Wrow_dev, partial);
+  else if (dtype == TFX_F32 && R == 8)
+    k_sparse_residual_f4<2><<<blocks, 256, 0, st>>>(idx32, (const float*)vals, nnz, sh,
+                                                    (const float* const*)Wrow_dev, partial);
+  else if (dtype == TFX_F32 && R == 4)
+    k_sparse_residual_f4<1><<<blocks, 256, 0, st>>>(idx32, (const float*)vals, nnz, sh,
+                                                    (const float* const*)Wrow_dev, partial);
   else if (dtype == TFX_F32)
     k_sparse_residual<float><<<blocks, 256, 0, st>>>(idx32, (const float*)vals, nnz, sh, (const float* const*)Wrow_dev,
                                                      partial);
