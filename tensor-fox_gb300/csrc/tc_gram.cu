@@ -397,8 +397,15 @@ __global__ void __launch_bounds__(128, 1)
         if (row < D) {
           const int col0 = bj * TCG_BM + cc;
           float* o = out + (size_t)row * D + col0;
-          for (int j = 0; j < 32; ++j)
-            if (col0 + j < D) o[j] = __uint_as_float(v[j]);
+          if ((D & 3) == 0 && col0 + 32 <= D && ((uintptr_t)o & 15) == 0) {  // whole sectors a lane
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+              *reinterpret_cast<uint4*>(o + j) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (col0 + j < D) o[j] = __uint_as_float(v[j]);
+          }
         }
       }
     } else if (ok_all && nit == 0) {
@@ -415,20 +422,41 @@ __global__ void __launch_bounds__(128, 1)
   }
 }
 
-// G from the split-K partials of the upper blocks.  ks_d partials for blocks of
-// the diagonal 256 x 256 super-blocks, ks_o for the others (super2 == 0: one
-// count, ks_d, for every block).
-__global__ void k_gram_tc_reduce(const float* __restrict__ part, int D, int ks_d, int ks_o, int super2,
-                                 float* __restrict__ G) {
+// G from the split-K partials of the upper blocks, and its mirror.  ks_d
+// partials for blocks of the diagonal 256 x 256 super-blocks, ks_o for the others
+// (super2 == 0: one count, ks_d, for every block).  A CTA takes 8 rows x 32
+// columns on or above the diagonal, four groups of threads a quarter of the
+// partials each (compensated FP32, added in order).  512 x 512, 38 and 50
+// partials: 45 -> 13 us (one thread an element also for the mirrored half, whose
+// reads went down columns).
+__global__ void __launch_bounds__(1024) k_gram_tc_reduce(const float* __restrict__ part, int D, int ks_d, int ks_o,
+                                                         int super2, float* __restrict__ G) {
+  __shared__ float2 red[3][8][32];
+  const int nb = (D + 31) / 32;
+  int t = blockIdx.x >> 2, bi = 0;
+  while (t >= nb - bi) {
+    t -= nb - bi;
+    ++bi;
+  }
+  const int x = threadIdx.x & 31, y = (threadIdx.x >> 5) & 7, z = threadIdx.x >> 8;
+  const int i = bi * 32 + 8 * (blockIdx.x & 3) + y, j = (bi + t) * 32 + x;
   const long long n = (long long)D * D;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(e / D), j = (int)(e - (long long)i * D);
-    const long long src = (i / TCG_BM <= j / TCG_BM) ? e : (long long)j * D + i;
-    const int ksplit = (!super2 || (i / (2 * TCG_BM)) == (j / (2 * TCG_BM))) ? ks_d : ks_o;
-    // compensated FP32 sum of the partials, in split order (FP64 adds are slow on GB300)
-    Acc<float> s;
-    for (int k = 0; k < ksplit; ++k) s.add(__ldcs(part + (size_t)k * n + src));
-    G[e] = s.hi + s.lo;
+  const bool on = i < D && j < D && i <= j;
+  const int ks = (!super2 || (i / (2 * TCG_BM)) == (j / (2 * TCG_BM))) ? ks_d : ks_o;
+  Acc<float> s;
+  if (on) {
+    const float* p = part + (size_t)i * D + j;
+#pragma unroll 8
+    for (int k = ks * z / 4; k < ks * (z + 1) / 4; ++k) s.add(__ldcs(p + (size_t)k * n));
+  }
+  if (z > 0) red[z - 1][y][x] = make_float2(s.hi, s.lo);
+  __syncthreads();
+  if (z == 0 && on) {
+#pragma unroll
+    for (int u = 0; u < 3; ++u) s.add2(red[u][y][x].x, red[u][y][x].y);
+    const float v = s.hi + s.lo;
+    G[(size_t)i * D + j] = v;
+    if (j > i) G[(size_t)j * D + i] = v;
   }
 }
 
@@ -560,9 +588,8 @@ extern "C" int tfx_mode_gram_tc(const float* S, long long P, int D, long long Q,
   e = cudaGetLastError();
   if (e != cudaSuccess) return tfx_set_cuda_error(e, "mode_gram_tc launch");
   tfx_count_launch(1);
-  const long long n = (long long)D * D;
-  const int rb = (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 4LL * sm_count()));
-  k_gram_tc_reduce<<<rb, 256, 0, st>>>((const float*)scratch, D, kk.ks_d, kk.ks_o, tc_use2(D) ? 1 : 0, G);
+  const int n32 = (D + 31) / 32;
+  k_gram_tc_reduce<<<(unsigned)(2 * n32 * (n32 + 1)), 1024, 0, st>>>((const float*)scratch, D, kk.ks_d, kk.ks_o, tc_use2(D) ? 1 : 0, G);
   e = cudaGetLastError();
   if (e != cudaSuccess) return tfx_set_cuda_error(e, "mode_gram_tc reduce");
   tfx_count_launch(1);
