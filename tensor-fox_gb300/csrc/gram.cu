@@ -130,9 +130,9 @@ struct Loader {
 // For K-contiguous rows (not the last mode) fma.rn.f32x2 takes two k at once:
 // both operands are register pairs as they lie in shared memory, no moves, 16
 // one-wavefront reads for 128 FMA instructions.  For the last mode, whose rows
-// lie together, it takes two columns.  512 x 262144: 1.81 ms = 38 TFLOP/s on the
-// upper triangle, FMA pipe 60% busy (6.3 ms with 4 x 4 thread tiles on scalar
-// reads; 2.11 ms with each chunk's source addresses formed afresh).
+// lie together, it takes two columns.  512 x 262144: 1.66 ms = 41 TFLOP/s on the
+// upper triangle (1.79 with two steps unrolled; 6.3 with 4 x 4 thread tiles on scalar
+// reads; 2.11 with each chunk's source addresses formed afresh).
 // ---------------------------------------------------------------------------
 constexpr int FST = BK + 4, FSTAGES = 3;
 template <bool LAST>
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(NT, 2) k_gram_f32(const float* __restrict__ S,
     } else {
       const float* ap = A + (wm * 32 + lm) * FST + wk * 16;
       const float* bp = B + ln * FST + wk * 16;
-#pragma unroll 2
+#pragma unroll 1
       for (int k4 = 0; k4 < 16; k4 += 4) {
         ulonglong2 a[8];
 #pragma unroll

@@ -12,9 +12,9 @@
 // bytes where the contiguous extent is a multiple of 4 and the base aligned, 4
 // bytes otherwise, three stages deep.
 //
-// 512^3 at R = 50, a mode: 317 us (271 for the last one, whose rows lie
-// together) = 42 (50) TFLOP/s, FMA pipe 61% (69%) busy and the shared-memory
-// pipe 65% (75%); 2253 us with 4 x 4 thread tiles and Khatri-Rao rows formed in
+// 512^3 at R = 50, a mode: 296 us (256 for the last one, whose rows lie
+// together) = 45 (52) TFLOP/s (two steps of four k unrolled 310 and 270, one 323
+// and 288, eight as here); 2253 us with 4 x 4 thread tiles and Khatri-Rao rows formed in
 // the loop.  Also measured: the same tiles with the rows formed in the loop 508
 // us (a quarter of the stalls on the factor loads), with the next chunk's
 // loaded ahead 545 us (60% more instructions).
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(NT, Cfg<TN, WM, LAST, FOLD>::CTAS)
     asm volatile("cp.async.commit_group;\n" ::: "memory");
     const float* A = sm + stage * C::STG;
     const float* B = A + C::ASZ + wk * C::KW * C::BN;
-#pragma unroll 2
+#pragma unroll 8
     for (int k4 = 0; k4 < C::KW; k4 += 4) {
       float a[4][4];  // [row][k]
 #pragma unroll
