@@ -90,13 +90,15 @@ __global__ void __launch_bounds__(TFX_THREADS) k_gemm(const T* __restrict__ A, c
 // ---------------------------------------------------------------------------
 // Mode product for FP32 with a short left factor: out[p] (n x Q) = Ut (n x D)
 // times S[p] (D x Q), all row-major.  One warp owns 8 rows of the output tile
-// and each lane 8 x TN outputs; per 4 k steps a lane reads 8 broadcast float4
-// of Ut and TN float4 of S for 32*TN FMAs.  The (BK x BN) slab of S and the
-// (BM x BK) slab of Ut are double-buffered in shared memory and filled with
-// cp.async (16-byte copies, zero-filled past the edges), so the next slab
-// streams in while the current one is multiplied.  The block has
-// 32 * ceil(rows/8) threads (at most 8 warps): a 50-row factor wastes 6 rows
-// instead of 14.  Needs D % 4 == 0, Q % 4 == 0 and 16-byte aligned pointers.
+// and each lane 8 x TN outputs as column pairs (fma.rn.f32x2); per 4 k steps a
+// lane reads 8 broadcast float4 of Ut and TN float4 of S for 16*TN pair FMAs.
+// The (BK x BN) slab of S and the (BM x BK) slab of Ut are double-buffered in
+// shared memory and filled with cp.async (zero-filled past the edges), 16 bytes
+// a copy where D and Q are multiples of 4 and the pointers aligned (VEC), else
+// 4, so the next slab streams in while the current one is multiplied.  The
+// block has 32 * ceil(rows/8) threads (at most 8 warps): a 50-row factor wastes
+// 6 rows instead of 14.  Bound by the FP32 FMA rate: 50 x 512 x 262144 366
+// us (384 with one FMA an instruction).
 // ---------------------------------------------------------------------------
 constexpr int TTM_BK = 16;
 
@@ -104,11 +106,56 @@ __device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc, int src
   const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(gsrc), "r"(src_bytes) : "memory");
 }
+__device__ __forceinline__ void cp_async4(void* sdst, const void* gsrc, int src_bytes) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(sdst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sa), "l"(gsrc), "r"(src_bytes) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
+typedef unsigned long long fpair;  // two floats in a register pair
+__device__ __forceinline__ fpair pair_of(float a) {
+  fpair d;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(a));
+  return d;
+}
+__device__ __forceinline__ void pair_fma(fpair& c, fpair a, fpair b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float2 pair_get(fpair v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+
+// acc[8][TN / 2] += the 8 rows' four k values (a: broadcast reads, row stride
+// as) times four rows of TN columns a lane (b: row stride bs, columns 128 j4 + 4
+// lane ...)
 template <int TN>
+__device__ __forceinline__ void rows8_fma4(fpair (&acc)[8][TN / 2], const float* a0, int as, const float* b0, int bs) {
+  float4 a[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) a[i] = *(const float4*)(a0 + i * as);
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    fpair bv[TN / 2];
+#pragma unroll
+    for (int j4 = 0; j4 < TN / 4; ++j4) {
+      const ulonglong2 v = *(const ulonglong2*)(b0 + u * bs + j4 * 128);
+      bv[2 * j4] = v.x;
+      bv[2 * j4 + 1] = v.y;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const fpair ai = pair_of(u == 0 ? a[i].x : u == 1 ? a[i].y : u == 2 ? a[i].z : a[i].w);
+#pragma unroll
+      for (int j = 0; j < TN / 2; ++j) pair_fma(acc[i][j], ai, bv[j]);
+    }
+  }
+}
+
+template <int TN, bool VEC>
 __global__ void __launch_bounds__(256, 2) k_ttm_f32(const float* __restrict__ Ut, const float* __restrict__ S,
                                                     float* __restrict__ out, int n, int D, long long Q, long long P) {
   constexpr int BN = 32 * TN;
@@ -125,25 +172,40 @@ __global__ void __launch_bounds__(256, 2) k_ttm_f32(const float* __restrict__ Ut
     const float* Sp = S + p * (long long)D * Q;
     auto issue = [&](int t, int b) {
       const int k0 = t * TTM_BK;
-      for (int e = tid; e < BM * (TTM_BK / 4); e += nt) {
-        const int m = e >> 2, k4 = (e & 3) * 4;
-        const bool ok = m0 + m < n && k0 + k4 < D;
-        cp_async16(&sA[b][m][k4], ok ? (const void*)(Ut + (long long)(m0 + m) * D + k0 + k4) : (const void*)Ut,
-                   ok ? 16 : 0);
-      }
-      for (int e = tid; e < TTM_BK * (BN / 4); e += nt) {
-        const int kk = e / (BN / 4), c4 = (e - kk * (BN / 4)) * 4;
-        const bool ok = k0 + kk < D && q0 + c4 < Q;
-        cp_async16(&sB[b][kk][c4], ok ? (const void*)(Sp + (long long)(k0 + kk) * Q + q0 + c4) : (const void*)Sp,
-                   ok ? 16 : 0);
+      if (VEC) {
+        for (int e = tid; e < BM * (TTM_BK / 4); e += nt) {
+          const int m = e >> 2, k4 = (e & 3) * 4;
+          const bool ok = m0 + m < n && k0 + k4 < D;
+          cp_async16(&sA[b][m][k4], ok ? (const void*)(Ut + (long long)(m0 + m) * D + k0 + k4) : (const void*)Ut,
+                     ok ? 16 : 0);
+        }
+        for (int e = tid; e < TTM_BK * (BN / 4); e += nt) {
+          const int kk = e / (BN / 4), c4 = (e - kk * (BN / 4)) * 4;
+          const bool ok = k0 + kk < D && q0 + c4 < Q;
+          cp_async16(&sB[b][kk][c4], ok ? (const void*)(Sp + (long long)(k0 + kk) * Q + q0 + c4) : (const void*)Sp,
+                     ok ? 16 : 0);
+        }
+      } else {
+        for (int e = tid; e < BM * TTM_BK; e += nt) {
+          const int m = e / TTM_BK, k = e % TTM_BK;
+          const bool ok = m0 + m < n && k0 + k < D;
+          cp_async4(&sA[b][m][k], ok ? (const void*)(Ut + (long long)(m0 + m) * D + k0 + k) : (const void*)Ut,
+                    ok ? 4 : 0);
+        }
+        for (int e = tid; e < TTM_BK * BN; e += nt) {
+          const int kk = e / BN, c = e - kk * BN;
+          const bool ok = k0 + kk < D && q0 + c < Q;
+          cp_async4(&sB[b][kk][c], ok ? (const void*)(Sp + (long long)(k0 + kk) * Q + q0 + c) : (const void*)Sp,
+                    ok ? 4 : 0);
+        }
       }
       cp_async_commit();
     };
-    float acc[8][TN];
+    fpair acc[8][TN / 2];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-      for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+      for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0ull;
     __syncthreads();  // the previous p's readers are done with both buffers
     issue(0, 0);
     for (int t = 0; t < nk; ++t) {
@@ -156,29 +218,8 @@ __global__ void __launch_bounds__(256, 2) k_ttm_f32(const float* __restrict__ Ut
       }
       __syncthreads();
 #pragma unroll
-      for (int k4 = 0; k4 < TTM_BK; k4 += 4) {
-        float4 a[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) a[i] = *(const float4*)&sA[b][wid * 8 + i][k4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          float bv[TN];
-#pragma unroll
-          for (int j4 = 0; j4 < TN / 4; ++j4) {
-            const float4 v = *(const float4*)&sB[b][k4 + u][j4 * 128 + lane * 4];
-            bv[4 * j4 + 0] = v.x;
-            bv[4 * j4 + 1] = v.y;
-            bv[4 * j4 + 2] = v.z;
-            bv[4 * j4 + 3] = v.w;
-          }
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float ai = u == 0 ? a[i].x : u == 1 ? a[i].y : u == 2 ? a[i].z : a[i].w;
-#pragma unroll
-            for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(ai, bv[j], acc[i][j]);
-          }
-        }
-      }
+      for (int k4 = 0; k4 < TTM_BK; k4 += 4)
+        rows8_fma4<TN>(acc, &sA[b][wid * 8][k4], AKS, &sB[b][k4][lane * 4], BN);
       __syncthreads();  // slab b is free for the copy issued next iteration
     }
     float* op = out + p * (long long)n * Q;
@@ -189,9 +230,16 @@ __global__ void __launch_bounds__(256, 2) k_ttm_f32(const float* __restrict__ Ut
 #pragma unroll
       for (int j4 = 0; j4 < TN / 4; ++j4) {
         const long long q = q0 + j4 * 128 + lane * 4;
-        if (q < Q)
-          *(float4*)(op + (long long)m * Q + q) =
-              make_float4(acc[i][4 * j4], acc[i][4 * j4 + 1], acc[i][4 * j4 + 2], acc[i][4 * j4 + 3]);
+        const float2 x = pair_get(acc[i][2 * j4]), y = pair_get(acc[i][2 * j4 + 1]);
+        float* o = op + (long long)m * Q + q;
+        if (VEC) {
+          if (q < Q) *(float4*)o = make_float4(x.x, x.y, y.x, y.y);
+        } else {
+          if (q < Q) o[0] = x.x;
+          if (q + 1 < Q) o[1] = x.y;
+          if (q + 2 < Q) o[2] = y.x;
+          if (q + 3 < Q) o[3] = y.y;
+        }
       }
     }
   }
@@ -1137,9 +1185,9 @@ extern "C" int tfx_ttm(int dtype, const void* S, long long P, int D, long long Q
                        void* stream) {
   if (!S || !Ut || !out || P < 1 || D < 1 || Q < 1 || n < 1) return tfx_set_error(TFX_STATUS_ERR_ARG, "ttm args");
   cudaStream_t st = (cudaStream_t)stream;
-  const bool vec = dtype == TFX_F32 && D % 4 == 0 && Q % 4 == 0 && ((uintptr_t)S & 15) == 0 &&
-                   ((uintptr_t)Ut & 15) == 0 && ((uintptr_t)out & 15) == 0;
-  if (vec && Q >= 128) {
+  const bool vec = D % 4 == 0 && Q % 4 == 0 && ((uintptr_t)S & 15) == 0 && ((uintptr_t)Ut & 15) == 0 &&
+                   ((uintptr_t)out & 15) == 0;
+  if (dtype == TFX_F32 && Q >= 128) {
     const int rows = n < 64 ? n : 64;
     const int nw = (rows + 7) / 8;
     const int mt = (n + 8 * nw - 1) / (8 * nw);
@@ -1148,10 +1196,14 @@ extern "C" int tfx_ttm(int dtype, const void* S, long long P, int D, long long Q
     const long long tq = wide ? (Q + 255) / 256 : (Q + 127) / 128;
     if (tq > 2147483647LL) return tfx_set_error(TFX_STATUS_ERR_UNSUPPORTED, "ttm too wide");
     dim3 grid((unsigned)tq, (unsigned)(P < 65535 ? P : 65535), (unsigned)mt);
-    if (wide)
-      k_ttm_f32<8><<<grid, 32 * nw, 0, st>>>((const float*)Ut, (const float*)S, (float*)out, n, D, Q, P);
-    else
-      k_ttm_f32<4><<<grid, 32 * nw, 0, st>>>((const float*)Ut, (const float*)S, (float*)out, n, D, Q, P);
+    const float *u = (const float*)Ut, *s = (const float*)S;
+    if (vec) {
+      if (wide) k_ttm_f32<8, true><<<grid, 32 * nw, 0, st>>>(u, s, (float*)out, n, D, Q, P);
+      else k_ttm_f32<4, true><<<grid, 32 * nw, 0, st>>>(u, s, (float*)out, n, D, Q, P);
+    } else {
+      if (wide) k_ttm_f32<8, false><<<grid, 32 * nw, 0, st>>>(u, s, (float*)out, n, D, Q, P);
+      else k_ttm_f32<4, false><<<grid, 32 * nw, 0, st>>>(u, s, (float*)out, n, D, Q, P);
+    }
     return check_launch("ttm");
   }
   if (dtype == TFX_F64 && (Q == 1 || Q >= 8) && (Q == 1 ? P : Q) <= 0x7fffffffLL) {
@@ -1271,131 +1323,185 @@ int tfx_cp_residual_tc_launch(const float* T, const int* dims, int R, const floa
                               int max_partials, int* err, int* nblocks, cudaStream_t st);
 
 // ---------------------------------------------------------------------------
-// FP32 ||T - [[W]]||^2 as a register-tiled GEMM with the Khatri-Rao operand
-// generated on the fly.  A block owns 256 columns q of the other modes: it
-// forms their Khatri-Rao rows once (R x 256, shared memory, R <= 64), then
-// walks every row tile of mode 0: the model tile (8 rows per warp, 8 x 8
-// outputs per lane as in k_ttm_f32) = W_0 (rows x R) KR^T (R x 256), and the
-// epilogue subtracts the streamed tensor tile and accumulates squares in
-// float-float.  Block partials are summed in FP64 by k_final_sum.
+// The FP32 model [[W]] as a register-tiled GEMM with the Khatri-Rao operand
+// generated on the fly: subtracted from the tensor and squared, or written
+// (FULL).  A block owns 32 TN columns q of the other modes: it forms their
+// Khatri-Rao rows (up to 64 ranks at a time, shared memory), then walks its row
+// tiles of mode 0 (blockIdx.y deals them): the model tile (8 rows per warp, 8 x
+// TN outputs per lane as column pairs, as in k_ttm_f32) = W_0 (rows x R) KR^T
+// (R x columns).  The residual accumulates squares in float-float; block
+// partials are summed in FP64 by k_final_sum.  A written tile goes out through
+// shared memory, whole lines a warp whatever the row's alignment.  Bound by the
+// FP32 FMA rate and, written, by HBM: 300 x 262 x 217 at R = 40 82 us (92 with 4 x
+// 4 outputs a thread on scalar reads); residual of 187 x 143 x 95 at R = 21 22 us
+// (40 with one block a column tile, 53 of them).
 // ---------------------------------------------------------------------------
-constexpr int RES_BN = 256, RES_RMAX = 64;
+constexpr int RES_RMAX = 64, RES_AKS = RES_RMAX + 4;
 
-__global__ void __launch_bounds__(256, 2) k_cp_residual_f32(const float* __restrict__ Tt, const float* __restrict__ W,
-                                                            CpShape sh, long long Q0, double* __restrict__ partial) {
-  constexpr int TN = 8, BN = RES_BN, AKS = RES_RMAX + 4;
+template <int TN>
+constexpr size_t model_smem(bool full) {
+  return (size_t)(RES_RMAX * 32 * TN + 64 * RES_AKS + (full ? 64 * (32 * TN + 4) : 0)) * sizeof(float);
+}
+
+template <int TN, bool FULL>
+__global__ void __launch_bounds__(256, 2) k_cp_model_f32(const float* __restrict__ Tt, const float* __restrict__ W,
+                                                         const __grid_constant__ CpShape sh, long long Q0,
+                                                         double* __restrict__ partial, float* __restrict__ full) {
+  constexpr int BN = 32 * TN, OST = BN + 4;
   extern __shared__ __align__(16) float res_sm[];
   float* sKR = res_sm;                      // [RES_RMAX][BN]
-  float* sA = sKR + RES_RMAX * BN;          // [64][AKS]
+  float* sA = sKR + RES_RMAX * BN;          // [64][RES_AKS]
+  float* sO = sA + 64 * RES_AKS;            // FULL: [64][OST]
   __shared__ int sIdx[BN][TFX_MAX_ORDER];
   __shared__ double red[8];
-  __shared__ int sD[TFX_MAX_ORDER], sOff[TFX_MAX_ORDER];  // shape, indexed at run time
   const int nw = blockDim.x >> 5, nt = blockDim.x;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-#pragma unroll
-  for (int l = 0; l < TFX_MAX_ORDER; ++l)
-    if (tid == l) {
-      sD[l] = sh.d[l];
-      sOff[l] = sh.off[l];
-    }
   const int L = sh.L, R = sh.R, d0 = sh.d[0];
-  const int Rp = (R + 3) & ~3;
-  const int BM = 8 * nw;
+  const int BM = 8 * nw, mt = (d0 + BM - 1) / BM;
+  const int mb = mt * blockIdx.y / gridDim.y, me = mt * (blockIdx.y + 1) / gridDim.y;
   const long long qt = (Q0 + BN - 1) / BN;
   Acc<float> acc2;
   for (long long t = blockIdx.x; t < qt; t += gridDim.x) {
     const long long q0 = t * BN;
-    __syncthreads();  // shape copied; the previous tile's readers are done
+    __syncthreads();  // the previous tile's readers are done
     for (int c = tid; c < BN; c += nt) {
       long long q = q0 + c;
       if (q >= Q0) q = Q0 - 1;  // padding columns repeat a valid one; their terms are skipped
       for (int l = L - 1; l >= 1; --l) {
-        sIdx[c][l] = (int)(q % sD[l]);
-        q /= sD[l];
+        const long long qq = Q0 <= 0x7fffffffLL ? (long long)((unsigned)q / (unsigned)sh.d[l]) : q / sh.d[l];
+        sIdx[c][l] = (int)(q - qq * sh.d[l]);
+        q = qq;
       }
     }
-    __syncthreads();
-    for (int e = tid; e < Rp * BN; e += nt) {
-      const int r = e / BN, c = e - r * BN;
-      float v = 0.f;
-      if (r < R) {
-        v = 1.f;
-        for (int l = 1; l < L; ++l) v *= __ldg(W + sOff[l] + (size_t)r * sD[l] + sIdx[c][l]);
-      }
-      sKR[r * BN + c] = v;
-    }
-    for (int m0 = 0; m0 < d0; m0 += BM) {
-      __syncthreads();  // KR rows ready / the previous row tile's W_0 slab consumed
-      for (int e = tid; e < BM * Rp; e += nt) {
-        const int m = e / Rp, r = e - m * Rp;
-        sA[m * AKS + r] = (m0 + m < d0 && r < R) ? __ldg(W + (size_t)r * d0 + m0 + m) : 0.f;
-      }
-      __syncthreads();
-      float acc[8][TN];
+    for (int m = mb; m < me; ++m) {
+      const int m0 = m * BM;
+      fpair acc[8][TN / 2];
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-      for (int k4 = 0; k4 < Rp; k4 += 4) {
-        float4 a[8];
+        for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0ull;
+      for (int rb = 0; rb < R; rb += RES_RMAX) {
+        const int rn = min(RES_RMAX, R - rb), rp = (rn + 3) & ~3;
+        __syncthreads();  // indices ready / the previous readers are done
+        if (m == mb || R > RES_RMAX)
+          for (int e = tid; e < rp * BN; e += nt) {
+            const int r = e / BN, c = e - r * BN;
+            float v = 0.f;
+            if (r < rn) {
+              v = 1.f;
+              for (int l = 1; l < L; ++l) v *= __ldg(W + sh.off[l] + (size_t)(rb + r) * sh.d[l] + sIdx[c][l]);
+            }
+            sKR[r * BN + c] = v;
+          }
+        for (int e = tid; e < BM * rp; e += nt) {  // rows along the lanes: W_0's columns lie together
+          const int r = e / BM, i = e - r * BM;
+          sA[i * RES_AKS + r] = (m0 + i < d0 && r < rn) ? __ldg(W + (size_t)(rb + r) * d0 + m0 + i) : 0.f;
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int k4 = 0; k4 < rp; k4 += 4)
+          rows8_fma4<TN>(acc, sA + wid * 8 * RES_AKS + k4, RES_AKS, sKR + k4 * BN + lane * 4, BN);
+      }
+      if (FULL) {
+        float* o = sO + wid * 8 * OST;  // the warp's own rows
 #pragma unroll
-        for (int i = 0; i < 8; ++i) a[i] = *(const float4*)&sA[(wid * 8 + i) * AKS + k4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          float bv[TN];
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
           for (int j4 = 0; j4 < TN / 4; ++j4) {
-            const float4 v = *(const float4*)&sKR[(k4 + u) * BN + j4 * 128 + lane * 4];
-            bv[4 * j4 + 0] = v.x;
-            bv[4 * j4 + 1] = v.y;
-            bv[4 * j4 + 2] = v.z;
-            bv[4 * j4 + 3] = v.w;
+            const float2 x = pair_get(acc[i][2 * j4]), y = pair_get(acc[i][2 * j4 + 1]);
+            *(float4*)(o + i * OST + j4 * 128 + lane * 4) = make_float4(x.x, x.y, y.x, y.y);
           }
+        __syncwarp();
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float ai = u == 0 ? a[i].x : u == 1 ? a[i].y : u == 2 ? a[i].z : a[i].w;
+        for (int i = 0; i < 8; ++i) {
+          const int row = m0 + wid * 8 + i;
+          if (row >= d0) break;
+          float* g = full + (long long)row * Q0 + q0;
 #pragma unroll
-            for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(ai, bv[j], acc[i][j]);
-          }
+          for (int j = 0; j < TN; ++j)
+            if (q0 + 32 * j + lane < Q0) __stcs(g + 32 * j + lane, o[i * OST + 32 * j + lane]);
         }
-      }
-      // epilogue: the tensor tile (4 consecutive q per read when aligned)
+        __syncwarp();
+      } else {
+        // the tensor tile (4 consecutive q per read when aligned)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int m = m0 + wid * 8 + i;
-        if (m >= d0) continue;
+        for (int i = 0; i < 8; ++i) {
+          const int row = m0 + wid * 8 + i;
+          if (row >= d0) continue;
 #pragma unroll
-        for (int j4 = 0; j4 < TN / 4; ++j4) {
-          const long long q = q0 + j4 * 128 + lane * 4;
-          const float* tp = Tt + (long long)m * Q0 + q;
-          if (q + 3 < Q0 && ((((unsigned long long)tp) & 15) == 0)) {
-            const float4 tv = __ldcs(reinterpret_cast<const float4*>(tp));
-            const float e0 = tv.x - acc[i][4 * j4], e1 = tv.y - acc[i][4 * j4 + 1];
-            const float e2 = tv.z - acc[i][4 * j4 + 2], e3 = tv.w - acc[i][4 * j4 + 3];
-            acc2.fma_(e0, e0);
-            acc2.fma_(e1, e1);
-            acc2.fma_(e2, e2);
-            acc2.fma_(e3, e3);
-          } else {
+          for (int j4 = 0; j4 < TN / 4; ++j4) {
+            const long long q = q0 + j4 * 128 + lane * 4;
+            const float* tp = Tt + (long long)row * Q0 + q;
+            const float2 x = pair_get(acc[i][2 * j4]), y = pair_get(acc[i][2 * j4 + 1]);
+            const float md[4] = {x.x, x.y, y.x, y.y};
+            if (q + 3 < Q0 && ((((unsigned long long)tp) & 15) == 0)) {
+              const float4 tv = __ldcs(reinterpret_cast<const float4*>(tp));
+              const float e0 = tv.x - md[0], e1 = tv.y - md[1], e2 = tv.z - md[2], e3 = tv.w - md[3];
+              acc2.fma_(e0, e0);
+              acc2.fma_(e1, e1);
+              acc2.fma_(e2, e2);
+              acc2.fma_(e3, e3);
+            } else {
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-              if (q + u < Q0) {
-                const float df = __ldcs(tp + u) - acc[i][4 * j4 + u];
-                acc2.fma_(df, df);
-              }
+              for (int u = 0; u < 4; ++u)
+                if (q + u < Q0) {
+                  const float df = __ldcs(tp + u) - md[u];
+                  acc2.fma_(df, df);
+                }
+            }
           }
         }
       }
     }
   }
+  if (FULL) return;
   acc2.warp_reduce();
   if (lane == 0) red[wid] = acc2.value();
   __syncthreads();
   if (tid == 0) {
     double sum = 0.0;
     for (int w = 0; w < nw; ++w) sum += red[w];
-    partial[blockIdx.x] = sum;
+    partial[blockIdx.y * gridDim.x + blockIdx.x] = sum;
   }
+}
+
+// Blocks: 256 columns each where those fill two CTAs a SM, else 128; the row
+// tiles dealt over as many CTAs more as that leaves free.  Returns the number of
+// partials, or a negative status.
+template <bool FULL>
+static int launch_model_f32(const float* T, const float* W, const CpShape& sh, long long Q0, double* partial,
+                            float* full, cudaStream_t st) {
+  const int d0 = sh.d[0], rows = d0 < 64 ? d0 : 64, nw = (rows + 7) / 8;
+  const long long slots = 2LL * num_sms(), mt = (d0 + 8 * nw - 1) / (8 * nw);
+  const bool wide = (Q0 + 255) / 256 >= slots && !FULL;
+  const long long qt = wide ? (Q0 + 255) / 256 : (Q0 + 127) / 128;
+  const unsigned bx = (unsigned)std::min<long long>(qt, slots);
+  const unsigned by = (unsigned)std::max<long long>(1, std::min<long long>(mt, slots / bx));
+  const size_t smb = wide ? model_smem<8>(FULL) : model_smem<4>(FULL);
+  cudaError_t e = wide ? cudaFuncSetAttribute(k_cp_model_f32<8, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb)
+                       : cudaFuncSetAttribute(k_cp_model_f32<4, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
+  if (e != cudaSuccess) return -tfx_set_cuda_error(e, "cp_model attr");
+  if (wide) k_cp_model_f32<8, FULL><<<dim3(bx, by), 32 * nw, smb, st>>>(T, W, sh, Q0, partial, full);
+  else k_cp_model_f32<4, FULL><<<dim3(bx, by), 32 * nw, smb, st>>>(T, W, sh, Q0, partial, full);
+  if (int r = check_launch("cp_model")) return -r;
+  return (int)(bx * by);
+}
+
+// cp_full for FP32 (called from autograd_kernels.cu)
+int tfx_cp_full_f32(int L, const int* dims, int R, const float* W, float* out, cudaStream_t st) {
+  CpShape sh;
+  sh.L = L;
+  sh.R = R;
+  int s = 0;
+  long long Q0 = 1;
+  for (int l = 0; l < L; ++l) {
+    sh.d[l] = dims[l];
+    sh.off[l] = R * s;
+    s += dims[l];
+    if (l) Q0 *= dims[l];
+  }
+  const int r = launch_model_f32<true>(nullptr, W, sh, Q0, nullptr, out, st);
+  return r < 0 ? -r : TFX_STATUS_OK;
 }
 
 // ||T - [[W]]||^2 into out (double) and out_t (the working type), either may be null
@@ -1431,26 +1537,15 @@ static int cp_residual(int dtype, const void* Tp, int L, const int* dims, int R,
     }
     if (r != TFX_STATUS_ERR_UNSUPPORTED) return r;
   }
-  if (dtype == TFX_F32 && Q0 >= RES_BN && R <= RES_RMAX) {
-    const int rows = dims[0] < 64 ? dims[0] : 64;
-    const int nw = (rows + 7) / 8;
-    const long long tiles = (Q0 + RES_BN - 1) / RES_BN;
-    const int blocks = (int)std::max<long long>(1, std::min<long long>(tiles, 2LL * num_sms()));
-    const size_t smb = ((size_t)RES_RMAX * RES_BN + 64 * (RES_RMAX + 4)) * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(k_cp_residual_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
-    if (e != cudaSuccess) return tfx_set_cuda_error(e, "cp_residual attr");
-    k_cp_residual_f32<<<blocks, 32 * nw, smb, st>>>((const float*)Tp, (const float*)W, sh, Q0, partial);
-    int r = check_launch("cp_residual");
-    if (r) return r;
-    k_final_sum<T><<<1, 256, 0, st>>>(partial, blocks, 1, nullptr, out, out_t);
+  if (dtype == TFX_F32) {
+    const int nb = launch_model_f32<false>((const float*)Tp, (const float*)W, sh, Q0, partial, nullptr, st);
+    if (nb < 0) return -nb;
+    k_final_sum<T><<<1, 256, 0, st>>>(partial, nb, 1, nullptr, out, out_t);
     return check_launch("final_sum");
   }
   const long long tiles = ((dims[0] + 63) / 64) * ((Q0 + 63) / 64);
   const int blocks = (int)std::max<long long>(1, std::min<long long>(tiles, 8LL * num_sms()));
-  if (dtype == TFX_F32)
-    k_cp_residual<float, 4><<<blocks, TFX_THREADS, 0, st>>>((const float*)Tp, (const float*)W, sh, partial);
-  else
-    k_cp_residual<double, 4><<<blocks, TFX_THREADS, 0, st>>>((const double*)Tp, (const double*)W, sh, partial);
+  k_cp_residual<double, 4><<<blocks, TFX_THREADS, 0, st>>>((const double*)Tp, (const double*)W, sh, partial);
   int r = check_launch("cp_residual");
   if (r) return r;
   k_final_sum<T><<<1, 256, 0, st>>>(partial, blocks, 1, nullptr, out, out_t);
