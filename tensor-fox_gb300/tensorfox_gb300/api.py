@@ -171,9 +171,8 @@ def _engine_launch(Td, x0, R, options, prec, aliased=False, fix_mode=-1):
 def _engine_collect(b, options):
     """Reads a launched engine solve: (best, step_sizes, errors, improv,
     gradients, stop), the global RNG advanced past the 'cg' caps' draws."""
-    res = b.result[0].cpu().numpy()
+    res, stats = (v[0] for v in b.report())
     _lib.check_solve_status(res)
-    stats = b.stats[0].cpu().numpy()
     n = int(res[1])
     advance_rng(options, n)
     m = options.maxiter

@@ -93,26 +93,37 @@ class _Batch:
             dims_c = (ctypes.c_int * L)(*t.shape)
             nb = lib.tfx_dgn_workspace_bytes(_dev.lib_dtype(precision), L, dims_c, int(R))
             self.ws.append(torch.empty(int(nb), dtype=torch.uint8, device=t.device))
-        # host -> device copies through pinned staging: they queue behind the
-        # device work instead of waiting for it
+        # One pinned block holds the descriptors (the library copies them to the
+        # device itself), the CG caps and the damping schedule; the latter two go
+        # over in one asynchronous copy, queued behind the device work.  One
+        # zeroed device block takes what the engine reports.  This object keeps
+        # both alive until the results are read.
+        dev = tensors[0].device
         if budgets is None:
-            self.budgets = [_dev.h2d(cg_budgets(options, t.dim()), None, t.device) for t in tensors]
-        else:   # per-problem caps drawn by the caller (maxiter ints each)
-            self.budgets = [_dev.h2d(np.asarray(b, dtype=np.int32), None, t.device)
-                            for b, t in zip(budgets, tensors)]
+            budgets = [cg_budgets(options, t.dim()) for t in tensors]
+        caps = np.concatenate([np.asarray(b, dtype=np.int32) for b in budgets])
         sched = options.init_damp if isinstance(options.init_damp, list) else None
-        self.sched = None
-        if sched is not None:
-            self.sched = _dev.h2d(np.asarray(sched, dtype=np.float64), torch.float64, tensors[0].device)
-        self.stats = torch.zeros((self.n, 4 * self.maxiter), dtype=torch.float64, device=tensors[0].device)
-        self.result = torch.zeros((self.n, 4), dtype=torch.int32, device=tensors[0].device)
-        self.info = torch.zeros((self.n, 8), dtype=torch.float64, device=tensors[0].device)
-        self.prof = torch.zeros((self.n, 24), dtype=torch.int64, device=tensors[0].device)
-        # the descriptors live in pinned memory, so the library's copy of them
-        # to the device is asynchronous (this object keeps the buffer alive
-        # until the results are read)
-        self._desc_host = torch.zeros(ctypes.sizeof(_lib.DgnProblem) * self.n, dtype=torch.uint8).pin_memory()
-        self.desc = (_lib.DgnProblem * self.n).from_address(self._desc_host.data_ptr())
+        sc = np.asarray(sched if sched is not None else [], dtype=np.float64)
+        nd = ctypes.sizeof(_lib.DgnProblem) * self.n
+        o_sc = (nd + 15) // 16 * 16
+        o_cap = o_sc + 8 * sc.size
+        self._host = torch.empty(o_cap + 4 * caps.size, dtype=torch.uint8, pin_memory=True)
+        view = self._host.numpy()
+        view[:nd] = 0
+        view[o_sc:o_cap].view(np.float64)[:] = sc
+        view[o_cap:].view(np.int32)[:] = caps
+        self.d_desc = torch.empty(self._host.numel(), dtype=torch.uint8, device=dev)
+        self.d_desc[o_sc:].copy_(self._host[o_sc:], non_blocking=True)
+        base = self.d_desc.data_ptr()
+        caps_at = base + o_cap + 4 * np.concatenate([[0], np.cumsum([len(b) for b in budgets])])
+        self.sched = sched
+        n, m = self.n, self.maxiter
+        self._out = torch.zeros(n * (2 + 4 * m + 8 + 24), dtype=torch.float64, device=dev)
+        self.result = self._out[:2 * n].view(torch.int32).view(n, 4)
+        self.stats = self._out[2 * n:n * (2 + 4 * m)].view(n, 4 * m)
+        self.info = self._out[n * (2 + 4 * m):n * (10 + 4 * m)].view(n, 8)
+        self.prof = self._out[n * (10 + 4 * m):].view(torch.int64).view(n, 24)
+        self.desc = (_lib.DgnProblem * self.n).from_address(self._host.data_ptr())
         for p in range(self.n):
             d = self.desc[p]
             d.L = len(self.dims[p])
@@ -123,14 +134,12 @@ class _Batch:
             d.x = _dev.ptr(xs[p])
             d.best = _dev.ptr(self.best[p])
             d.work = _dev.ptr(self.ws[p])
-            d.budgets = _dev.ptr(self.budgets[p])
-            d.damp_sched = _dev.ptr(self.sched) if self.sched is not None else None
+            d.budgets = int(caps_at[p])
+            d.damp_sched = base + o_sc if sched is not None else None
             d.stats = _dev.ptr(self.stats[p])
             d.result = _dev.ptr(self.result[p])
             d.info = _dev.ptr(self.info[p])
             d.prof = _dev.ptr(self.prof[p])
-        self.d_desc = torch.empty(ctypes.sizeof(_lib.DgnProblem) * self.n, dtype=torch.uint8,
-                                  device=tensors[0].device)
         o = _lib.DgnOptions()
         o.maxiter = self.maxiter
         o.tol, o.tol_step, o.tol_improv = float(options.tol), float(options.tol_step), float(options.tol_improv)
@@ -143,6 +152,12 @@ class _Batch:
         o.aliased = 1 if aliased else 0
         o.fixed = int(fix_mode) + 1
         self.opts = o
+
+    def report(self):
+        """(result (n, 4), stats (n, 4 maxiter)) on the host, one transfer."""
+        n = self.n
+        h = self._out[:n * (2 + 4 * self.maxiter)].cpu().numpy()
+        return h[:2 * n].view(np.int32).reshape(n, 4), h[2 * n:].reshape(n, -1)
 
     def launch(self, cluster, stream=None):
         lib = _lib.load()
@@ -286,7 +301,7 @@ def dGN(T, factors, R, options=None, precision=None):
     for l in range(L):        # [W] marks a fixed factor (bicpd), GaussNewton.py:92-99
         if isinstance(factors[l], list):
             fix, factors[l] = l, factors[l][0]
-    x0 = torch.from_numpy(_dev.flat_factors(factors)).to(device=Td.device, dtype=dt)
+    x0 = _dev.h2d(_dev.flat_factors(factors), dt, Td.device)
     from .stepped import uses_stepped, dgn_stepped
     if uses_stepped(options):
         best, ss, er, im, gr, st = dgn_stepped(Td, x0, R, options, prec, fix_mode=fix, aliased=aliased)
@@ -294,12 +309,11 @@ def dGN(T, factors, R, options=None, precision=None):
     if aliased and len(set(dims)) != 1:
         raise ValueError("one factor array for every mode needs equal dimensions")
     b = dGN_device(Td, x0, R, options, prec, aliased=aliased, fix_mode=fix)
-    res = b.result[0].cpu().numpy()
+    res, stats = (v[0] for v in b.report())
     _lib.check_solve_status(res)
-    stats = b.stats[0].cpu().numpy()
     n = int(res[1])
     advance_rng(options, n)
-    best = _dev.unflat(b.best[0].double().cpu().numpy(), dims, R)
+    best = _dev.unflat(b.best[0].cpu().numpy(), dims, R)
     m = options.maxiter
     return (best, stats[m:m + n].copy(), stats[:n].copy(), stats[2 * m:2 * m + n].copy(),
             stats[3 * m:3 * m + n].copy(), int(res[0]))
