@@ -83,7 +83,7 @@ __host__ __device__ inline size_t g3_p0x(int d0, int d1, int d2) {
 }
 
 struct SmemPlan {
-  size_t sA, sB, sPart, sAk, sY, sM, sDG, sGam, sNorm, sBase, sIdx, rs4, rs12, misc, hist, rs1, rs1b, sScale, wsl, sG3, sE3;
+  size_t sA, sB, sPart, sAk, sY, sM, sDG, sGam, sNorm, sBase, sIdx, rs4, rs12, misc, hist, sScale, wsl, sG3, sE3;
   size_t sQf, sWf, sP1o, sP2o, sVec;  // staged operands of the CG (valid when stage != 0)
   int stage;
   size_t total;
@@ -110,12 +110,10 @@ __host__ __device__ inline SmemPlan smem_plan(int TS, size_t es, int maxL, int m
   p.sIdx = o; o += al16((size_t)NB * maxL * sizeof(int));
   p.rs4 = o; o += al16(sizeof(RedScratch<4>));
   p.rs12 = o; o += al16(sizeof(RedScratch<TFX_MAX_ORDER>));
-  p.misc = o; o += 64 + 16 * TFX_MAX_ORDER * 8;
+  p.misc = o; o += 64 + 16 * TFX_MAX_ORDER * 8 - 128;  // 8 scalars, the dimensions and offsets (544 bytes used)
   p.hist = o; o += al16((size_t)2 * maxiter * sizeof(double));
-  p.rs1 = o; o += al16(sizeof(RedScratch<1>));
-  p.rs1b = o; o += al16(sizeof(RedScratch<1>));
   p.sScale = o; o += al16((size_t)maxL * maxncol * es);
-  p.wsl = o; o += al16(sizeof(PushSlots<3>));
+  p.wsl = o; o += al16(sizeof(PushSlots));
   // third-order gradient scratch (every mode up to 64): three slab stages,
   // transposed own factor columns, M0 | M1 | M2, partial sums, stage barriers
   p.sG3 = 0;
@@ -160,7 +158,7 @@ __device__ __forceinline__ char* dyn_smem() {
 // shared memory; otherwise they are read from global memory (L2).
 // ---------------------------------------------------------------------------
 struct CgOffsets {
-  size_t d, sQf, sWf, sP1o, sP2o, sAk, sY, sM, sDG, rs4, rs1, sVec, wsl;
+  size_t d, sQf, sWf, sP1o, sP2o, sAk, sY, sM, sDG, rs4, sVec, wsl;
 };
 
 // Copy n elements written by other CTAs of the team from global memory into
@@ -299,7 +297,24 @@ __device__ __forceinline__ void cg_matvec(const int L, const int R, const int nx
   // more multiply-adds (the pass is bound by shared-memory wavefronts); each
   // dot keeps its two interleaved chains (even and odd i), as one output per
   // thread would.
-  {
+  // FP64: one output a thread (the pass is bound by the FP64 pipe, which a
+  // warp's instruction holds for 64 cycles however few of its lanes work).
+  if constexpr (sizeof(T) == 8) {
+    for (int e = tid; e < L * RN; e += TFX_THREADS) {
+      const int k = e / RN, rem = e - k * RN, c = rem / R, a = rem - c * R, dk = d[k];
+      const T* dv = Din + off[k] + a * dk;
+      const T* wv = Wr + off[k] + (c0 + c) * dk;
+      T ev = T(0), od = T(0);
+      int i = 0;
+#pragma unroll 4
+      for (; i + 1 < dk; i += 2) {
+        ev = fma(dv[i], wv[i], ev);
+        od = fma(dv[i + 1], wv[i + 1], od);
+      }
+      if (i < dk) ev = fma(dv[i], wv[i], ev);
+      sAk[(size_t)k * RN + a * ncol + c] = ev + od;
+    }
+  } else {
     const int RP = (R + 1) >> 1, ncg4 = (ncol + 3) >> 2;
     for (int e = tid; e < L * ncg4 * RP; e += TFX_THREADS) {
       const int k = e / (ncg4 * RP), rem = e - k * ncg4 * RP, cg = rem / RP, ap = rem - cg * RP;
@@ -347,8 +362,10 @@ __device__ __forceinline__ void cg_matvec(const int L, const int R, const int nx
   ctick(3);
   // z_l = W_l Y_l + D_l P1_l over all owned outputs of all modes at once;
   // a thread takes one row i of one mode and four owned columns
+  // (FP64: one, as above)
+  constexpr int ZC = sizeof(T) == 8 ? 1 : 4;
   const int sumd = nx / R;
-  const int ncg = (ncol + 3) >> 2;
+  const int ncg = (ncol + ZC - 1) / ZC;
   for (int e = tid; e < ncg * sumd; e += TFX_THREADS) {
     const int cgi = e / sumd;
     int l = 0, i = e - cgi * sumd;
@@ -356,7 +373,7 @@ __device__ __forceinline__ void cg_matvec(const int L, const int R, const int nx
       i -= d[l];
       ++l;
     }
-    const int cb = cgi * 4, cn = min(4, ncol - cb);
+    const int cb = cgi * ZC, cn = min(ZC, ncol - cb);
     const int dl = d[l], ol = off[l];
     const T* wrow = Wr + ol + i;
     const T* drow = Din + ol + i;
@@ -381,6 +398,8 @@ __device__ __forceinline__ void cg_matvec(const int L, const int R, const int nx
         a2[2] = fma(dd, (T)p4.z, a2[2]);
         a2[3] = fma(dd, (T)p4.w, a2[3]);
       }
+    } else if (ZC == 1) {
+      z_cols<T, 1>(R, dl, wrow, drow, yc, ncp, p1c, p1s, a1, a2);
     } else {
       switch (cn) {
         case 1: z_cols<T, 1>(R, dl, wrow, drow, yc, ncp, p1c, p1s, a1, a2); break;
@@ -390,7 +409,7 @@ __device__ __forceinline__ void cg_matvec(const int L, const int R, const int nx
       }
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < ZC; ++u)
       if (u < cn) {
         if (zloc)
           zloc[ncol * (ol / R) + (cb + u) * dl + i] = a1[u] + a2[u];
@@ -422,8 +441,7 @@ __device__ __forceinline__ int cg_team(const Team tm, const int L, const int R, 
   const int* off = d + TFX_MAX_ORDER;
   const T* sM = (const T*)(sm + so.sM);
   const T* sDG = (const T*)(sm + so.sDG);
-  PushSlots<1>* ps1 = (PushSlots<1>*)(sm + so.wsl);
-  PushSlots<3>* ps3 = (PushSlots<3>*)(sm + so.wsl);
+  PushSlots* ps = (PushSlots*)(sm + so.wsl);
   T* sQf = (T*)(sm + so.sQf);
   const int tid = threadIdx.x;
   // own slice: element (l, c, i) lives at local index ncol*(off[l]/R) + c*d[l] + i
@@ -461,7 +479,7 @@ __device__ __forceinline__ int cg_team(const Team tm, const int L, const int R, 
       v[0].fma_(rr, rr);
     }
   }
-  team_sum_push<1>(tm, v, tot, ps1, flipw);
+  team_sum_push<1>(tm, v, tot, ps, flipw);
   Acc<T> rnA = tot[0];
   T rn = acc_val(rnA);
   if (rn == T(0)) {
@@ -476,6 +494,10 @@ __device__ __forceinline__ int cg_team(const Team tm, const int L, const int R, 
   } else {
     tol = T(0);
   }
+  // FP64: the step lengths and the stop test are formed by one thread (an FP64
+  // division on every warp queues eight times 15 instructions of 64 cycles for
+  // four pipes) and read from these slots; two barriers separate their uses
+  T* sDiv = (T*)(sm + so.d - 32);  // the last four of the scalar slots
   int itn = 0;
   bool broke = false;
   for (itn = 0; itn < maxit; ++itn) {
@@ -533,16 +555,27 @@ __device__ __forceinline__ int cg_team(const Team tm, const int L, const int R, 
     }
     Acc<T> t3[3];
     if (MERGED) {
-      team_sum_push<3>(tm, w, t3, ps3, flipw);
+      team_sum_push<3>(tm, w, t3, ps, flipw);
     } else {
       Acc<T> w1[1] = {w[0]};
-      team_sum_push<1>(tm, w1, tot, ps1, flipw);
+      team_sum_push<1>(tm, w1, tot, ps, flipw);
       t3[0] = tot[0];
     }
     ctick(5);
-    T den = acc_val(t3[0]);
-    if (den == T(0)) den = T(1e-6);
-    const T ta = rn / den;
+    T ta;
+    if constexpr (sizeof(T) == 8) {
+      if (tid == 0) {
+        T den = acc_val(t3[0]);
+        if (den == T(0)) den = T(1e-6);
+        sDiv[0] = rn / den;
+      }
+      __syncthreads();
+      ta = sDiv[0];
+    } else {
+      T den = acc_val(t3[0]);
+      if (den == T(0)) den = T(1e-6);
+      ta = rn / den;
+    }
     Acc<T> u[1];
     if (STAGED) {
       for (int e = tid; e < own; e += TFX_THREADS) {
@@ -580,12 +613,25 @@ __device__ __forceinline__ int cg_team(const Team tm, const int L, const int R, 
       if (!(acc_val(rnN) > T(1e-4) * rn)) exact = true;
     }
     if (exact) {
-      team_sum_push<1>(tm, u, tot, ps1, flipw);
+      team_sum_push<1>(tm, u, tot, ps, flipw);
       rnN = tot[0];
     }
     ctick(6);
     const T rn_new = acc_val(rnN);
-    const T tb = rn_new / rn;
+    T tb;
+    bool small;
+    if constexpr (sizeof(T) == 8) {
+      if (tid == 0) {
+        sDiv[1] = rn_new / rn;
+        sDiv[2] = rn_new <= tol ? T(1) : T(0);
+      }
+      __syncthreads();
+      tb = sDiv[1];
+      small = __double_as_longlong((double)sDiv[2]) != 0;
+    } else {
+      tb = rn_new / rn;
+      small = rn_new <= tol;
+    }
     rn = rn_new;
     rnA = rnN;
     if (STAGED) {
@@ -600,7 +646,7 @@ __device__ __forceinline__ int cg_team(const Team tm, const int L, const int R, 
       }
     }
     ctick(7);
-    if (rn <= tol) {
+    if (small) {
       broke = true;
       break;
     }
@@ -637,6 +683,17 @@ __device__ __forceinline__ void lds4(const double* p, double (&v)[4]) {
   v[3] = b.y;
 }
 
+__device__ __forceinline__ void lds2(const float* p, float (&v)[2]) {
+  const float2 a = *reinterpret_cast<const float2*>(p);
+  v[0] = a.x;
+  v[1] = a.y;
+}
+__device__ __forceinline__ void lds2(const double* p, double (&v)[2]) {
+  const double2 a = *reinterpret_cast<const double2*>(p);
+  v[0] = a.x;
+  v[1] = a.y;
+}
+
 template <class T, int TS>
 struct Engine {
   using TL = Tile<TS, TS>;
@@ -657,8 +714,7 @@ struct Engine {
   int* sIdx;
   RedScratch<4>* rs4;
   RedScratch<TFX_MAX_ORDER>* rs12;
-  int flip4, flip12, flip1, flip1b, flipw;
-  RedScratch<1>* rs1b;
+  int flip4, flip12, flip1, flipw;
   T* sScale;
   double damp, Tsize;
   tfx_dgn_options op;
@@ -758,42 +814,88 @@ struct Engine {
   // FP64 every 16 terms when T is float); P1/P2 rounded to T for the matvec.
   __device__ void gramians_and_precond() {
     const int RR = R * R;
-    for (int u = tm.rank * TFX_THREADS + tid; u < L * RR; u += tm.size * TFX_THREADS) {
-      const int l = u / RR, q = u - l * RR, a = q / R, b = q - a * R;
-      if (a > b) continue;
+    // the pairs a <= b without idle threads: row pr of R - pr pairs together
+    // with row R - 1 - pr of pr + 1 pairs make R + 1 (an odd R's middle row
+    // stands alone)
+    const int RT = ((R + 1) / 2) * (R + 1);
+    auto pair_of = [&](int u, int& a, int& b) -> bool {
+      const int pr = u / (R + 1), q = u - pr * (R + 1);
+      a = pr;
+      b = pr + q;
+      if (q < R - pr) return true;
+      a = R - 1 - pr;
+      b = a + (q - (R - pr));
+      return a != pr;
+    };
+    for (int u = tm.rank * TFX_THREADS + tid; u < L * RT; u += tm.size * TFX_THREADS) {
+      const int l = u / RT;
+      int a, b;
+      if (!pair_of(u - l * RT, a, b)) continue;
       const T* pa = Wr + off[l] + a * d[l];
       const T* pb = Wr + off[l] + b * d[l];
       double acc = 0.0;
       for (int i0 = 0; i0 < d[l]; i0 += 16) {
         T p = T(0);
-        const int ie = min(d[l], i0 + 16);
-        for (int i = i0; i < ie; ++i) p = fma(pa[i], pb[i], p);
+        if (i0 + 16 <= d[l]) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) p = fma(pa[i0 + i], pb[i0 + i], p);
+        } else {
+          for (int i = i0; i < d[l]; ++i) p = fma(pa[i], pb[i], p);
+        }
         acc += (double)p;
       }
       G[(size_t)l * RR + a * R + b] = acc;
       G[(size_t)l * RR + b * R + a] = acc;
     }
     tm.sync();
-    // P2[l][k] = prod_{m not in {l,k}} G_m (ascending m), own columns only
-    for (int e = tid; e < L * L * R * ncol; e += TFX_THREADS) {
-      const int lk = e / (R * ncol), q = e - lk * (R * ncol), a = q / ncol, c = q - a * ncol;
-      const int l = lk / L, k = lk - l * L;
-      if (l == k) continue;
-      const int b = c0 + c;
-      double p = 1.0;
-      for (int m = 0; m < L; ++m)
-        if (m != l && m != k) p *= G[(size_t)m * RR + a * R + b];
-      P2at(l, k, a, c) = (T)p;
-    }
-    // P1 with the reference's product order
-    for (int e = tid; e < L * R * ncol; e += TFX_THREADS) {
-      const int l = e / (R * ncol), q = e - l * (R * ncol), a = q / ncol, c = q - a * ncol;
-      const int b = c0 + c;
-      P1at(l, a, c) = (T)p1_value(l, a, b);
+    if (L == 3) {
+      // each Gramian entry of the own columns is read once: P2[l][k] is the
+      // third mode's, P1 the reference's two-factor products (the whole phase at
+      // 50^3, R 50: 17.7 -> 9.3 us)
+      for (int e = tid; e < R * ncol; e += TFX_THREADS) {
+        const int a = e / ncol, c = e - a * ncol, q = a * R + c0 + c;
+        const double g0 = G[q], g1 = G[RR + q], g2 = G[2 * RR + q];
+        const T t0 = (T)g0, t1 = (T)g1, t2 = (T)g2;
+        P2at(0, 1, a, c) = t2;
+        P2at(1, 0, a, c) = t2;
+        P2at(0, 2, a, c) = t1;
+        P2at(2, 0, a, c) = t1;
+        P2at(1, 2, a, c) = t0;
+        P2at(2, 1, a, c) = t0;
+        P1at(0, a, c) = (T)(g2 * g1);
+        P1at(1, a, c) = (T)(g2 * g0);
+        P1at(2, a, c) = (T)(g1 * g0);
+      }
+    } else {
+      // P2[l][k] = prod_{m not in {l,k}} G_m (ascending m), own columns only
+      for (int e = tid; e < L * L * R * ncol; e += TFX_THREADS) {
+        const int lk = e / (R * ncol), q = e - lk * (R * ncol), a = q / ncol, c = q - a * ncol;
+        const int l = lk / L, k = lk - l * L;
+        if (l == k) continue;
+        const int b = c0 + c;
+        double p = 1.0;
+        for (int m = 0; m < L; ++m)
+          if (m != l && m != k) p *= G[(size_t)m * RR + a * R + b];
+        P2at(l, k, a, c) = (T)p;
+      }
+      // P1 with the reference's product order
+      for (int e = tid; e < L * R * ncol; e += TFX_THREADS) {
+        const int l = e / (R * ncol), q = e - l * (R * ncol), a = q / ncol, c = q - a * ncol;
+        const int b = c0 + c;
+        P1at(l, a, c) = (T)p1_value(l, a, b);
+      }
     }
     // tmp = max |P1[L-1]| over the whole matrix (every CTA computes it)
     double mx = 0.0;
-    for (int q = tid; q < RR; q += TFX_THREADS) mx = fmax(mx, fabs(p1_value(L - 1, q / R, q % R)));
+    if (L == 3) {
+#pragma unroll 4
+      for (int u = tid; u < RT; u += TFX_THREADS) {
+        int a, b;
+        if (pair_of(u, a, b)) mx = fmax(mx, fabs(G[RR + a * R + b] * G[a * R + b]));
+      }
+    } else {
+      for (int q = tid; q < RR; q += TFX_THREADS) mx = fmax(mx, fabs(p1_value(L - 1, q / R, q % R)));
+    }
     mx = warp_max(mx);
     if ((tid & 31) == 0) rs4->warp[tid >> 5][0] = mx;
     __syncthreads();
@@ -808,7 +910,7 @@ struct Engine {
       const int l = e / ncol, c = e - l * ncol, b = c0 + c;
       const double g = tmp * sqrt(fabs(p1_value(l, b, b)));
       sGam[e] = g;
-      const double m = 1.0 / sqrt(g * g + damp * damp * (g * g));
+      const double m = rsqrt(g * g + damp * damp * (g * g));
       sM[e] = (T)m;
       sDG[e] = (T)(damp * g);
     }
@@ -907,6 +1009,140 @@ struct Engine {
             : "memory");
       if (!ok) g3err = 1;
     };
+    const int nwr = min(NW, (d1 + 3) / 4);  // warps with rows
+    // One group's slabs.  Warps without rows, the second half of the rows (above
+    // 32) and of the k-groups are branched around: an FP64 instruction holds its
+    // pipe for 64 cycles a warp whether its lanes have work or not.
+    auto slabs = [&]() {
+      constexpr int CN = 4;
+      // own k-groups q8 and q8 + 8 and their rows of W2
+      T creg[2][4][CN], acc2[2][4][CN];
+#pragma unroll
+      for (int s2 = 0; s2 < 2; ++s2) {
+        const int kg = q8 + 8 * s2;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          T cc[4] = {T(0), T(0), T(0), T(0)};
+          if (kg < nkg) lds4(sC4 + (4 * kg + u) * 4, cc);
+#pragma unroll
+          for (int c = 0; c < CN; ++c) {
+            creg[s2][u][c] = cc[c];
+            acc2[s2][u][c] = T(0);
+          }
+        }
+      }
+      T bj[2][CN], m1[2][CN];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int c = 0; c < CN; ++c) {
+          bj[h][c] = T(0);
+          m1[h][c] = T(0);
+        }
+        if (rs + 32 * h < d1) {
+          T b4[4];
+          lds4(sB4 + (rs + 32 * h) * 4, b4);
+#pragma unroll
+          for (int c = 0; c < CN; ++c) bj[h][c] = b4[c];
+        }
+      }
+      gtick(0);
+      for (int i = 0; i < d0; ++i) {
+        wait_slab(i);
+        __syncthreads();  // every warp is past slab i-1: its stage may be refilled
+        gtick(1);
+        if (i + 2 < d0) issue(i + 2);
+        if (wid == NW - 1 && lane < 4 && i > 0) {  // M0 of slab i-1 from its warp partials
+          T sacc = T(0);
+          for (int w = 0; w < nwr; ++w) sacc += sP0[((i - 1) & 1) * NW * 4 + w * 4 + lane];
+          sM0[(i - 1) * 4 + lane] = sacc;
+        }
+        gtick(2);
+        if (wid < nwr) {
+          T ai[4];
+          lds4(sA4 + i * 4, ai);
+          T p0[CN];
+#pragma unroll
+          for (int c = 0; c < CN; ++c) p0[c] = T(0);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (4 * wid + 32 * h >= d1) break;  // no rows in this warp
+            const int row = rs + 32 * h;
+            T y[CN];
+#pragma unroll
+            for (int c = 0; c < CN; ++c) y[c] = T(0);
+            if (row < d1) {
+              const T* tr = sT + ((g3base + i) % 3) * SL + row * d2;
+              T kr[CN];
+#pragma unroll
+              for (int c = 0; c < CN; ++c) kr[c] = ai[c] * bj[h][c];
+#pragma unroll
+              for (int s2 = 0; s2 < 2; ++s2) {
+                const int kg = q8 + 8 * s2;
+                if (8 * s2 < nkg && kg < nkg) {
+                  T tv[4];
+#pragma unroll
+                  for (int u = 0; u < 4; ++u) tv[u] = (4 * kg + u < d2) ? tr[4 * kg + u] : T(0);
+#pragma unroll
+                  for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int c = 0; c < CN; ++c) {
+                      y[c] = fma(tv[u], creg[s2][u][c], y[c]);
+                      acc2[s2][u][c] = fma(tv[u], kr[c], acc2[s2][u][c]);
+                    }
+                }
+              }
+            }
+#pragma unroll
+            for (int c = 0; c < CN; ++c) {
+              y[c] += __shfl_xor_sync(0xffffffffu, y[c], 1);
+              y[c] += __shfl_xor_sync(0xffffffffu, y[c], 2);
+              y[c] += __shfl_xor_sync(0xffffffffu, y[c], 4);
+              m1[h][c] = fma(y[c], ai[c], m1[h][c]);
+              p0[c] = fma(y[c], bj[h][c], p0[c]);  // used in the lanes of q8 == 0
+            }
+          }
+#pragma unroll
+          for (int c = 0; c < CN; ++c) {
+            p0[c] += __shfl_xor_sync(0xffffffffu, p0[c], 8);
+            p0[c] += __shfl_xor_sync(0xffffffffu, p0[c], 16);
+          }
+          if (lane == 0)
+#pragma unroll
+            for (int c = 0; c < CN; ++c) sP0[(i & 1) * NW * 4 + wid * 4 + c] = p0[c];
+        }
+        gtick(3);
+      }
+      __syncthreads();
+      if (wid == NW - 1 && lane < 4) {
+        T sacc = T(0);
+        for (int w = 0; w < nwr; ++w) sacc += sP0[((d0 - 1) & 1) * NW * 4 + w * 4 + lane];
+        sM0[(d0 - 1) * 4 + lane] = sacc;
+      }
+      if (q8 == 0)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (rs + 32 * h < d1)
+#pragma unroll
+            for (int c = 0; c < CN; ++c) sM1[(rs + 32 * h) * 4 + c] = m1[h][c];
+      // M2: the rows of a warp (lanes with the same q8), then the warps
+      if (wid < nwr) {
+#pragma unroll
+        for (int s2 = 0; s2 < 2; ++s2) {
+          if (8 * s2 >= nkg) break;
+          const int kg = q8 + 8 * s2;
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int c = 0; c < CN; ++c) {
+              T v = acc2[s2][u][c];
+              v += __shfl_xor_sync(0xffffffffu, v, 8);
+              v += __shfl_xor_sync(0xffffffffu, v, 16);
+              if (lane < 8 && kg < nkg) sR2[(wid * d2p + 4 * kg + u) * 4 + c] = v;
+            }
+        }
+      }
+    };
     for (int cb = 0; cb < ncol; cb += 4) {
       const int cn = min(4, ncol - cb);
       for (int e = tid; e < (d0 + d1 + d2p) * 4; e += TFX_THREADS) {
@@ -926,121 +1162,12 @@ struct Engine {
       __syncthreads();  // sF ready; the previous group is done with every stage
       issue(0);
       if (d0 > 1) issue(1);
-      // own k-groups q8 and q8 + 8 and their rows of W2
-      T creg[2][4][4], acc2[2][4][4];
-#pragma unroll
-      for (int s2 = 0; s2 < 2; ++s2) {
-        const int kg = q8 + 8 * s2;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          T cc[4] = {T(0), T(0), T(0), T(0)};
-          if (kg < nkg) lds4(sC4 + (4 * kg + u) * 4, cc);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            creg[s2][u][c] = cc[c];
-            acc2[s2][u][c] = T(0);
-          }
-        }
-      }
-      T bj[2][4], m1[2][4];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          bj[h][c] = T(0);
-          m1[h][c] = T(0);
-        }
-        if (rs + 32 * h < d1) lds4(sB4 + (rs + 32 * h) * 4, bj[h]);
-      }
-      gtick(0);
-      for (int i = 0; i < d0; ++i) {
-        wait_slab(i);
-        __syncthreads();  // every warp is past slab i-1: its stage may be refilled
-        gtick(1);
-        if (i + 2 < d0) issue(i + 2);
-        if (wid == NW - 1 && lane < 4 && i > 0) {  // M0 of slab i-1 from its warp partials
-          T sacc = T(0);
-          for (int w = 0; w < NW; ++w) sacc += sP0[((i - 1) & 1) * NW * 4 + w * 4 + lane];
-          sM0[(i - 1) * 4 + lane] = sacc;
-        }
-        gtick(2);
-        T ai[4];
-        lds4(sA4 + i * 4, ai);
-        T p0[4] = {T(0), T(0), T(0), T(0)};
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int row = rs + 32 * h;
-          T y[4] = {T(0), T(0), T(0), T(0)};
-          if (row < d1) {
-            const T* tr = sT + ((g3base + i) % 3) * SL + row * d2;
-            T kr[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) kr[c] = ai[c] * bj[h][c];
-#pragma unroll
-            for (int s2 = 0; s2 < 2; ++s2) {
-              const int kg = q8 + 8 * s2;
-              if (kg < nkg) {
-                T tv[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) tv[u] = (4 * kg + u < d2) ? tr[4 * kg + u] : T(0);
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-#pragma unroll
-                  for (int c = 0; c < 4; ++c) {
-                    y[c] = fma(tv[u], creg[s2][u][c], y[c]);
-                    acc2[s2][u][c] = fma(tv[u], kr[c], acc2[s2][u][c]);
-                  }
-              }
-            }
-          }
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            y[c] += __shfl_xor_sync(0xffffffffu, y[c], 1);
-            y[c] += __shfl_xor_sync(0xffffffffu, y[c], 2);
-            y[c] += __shfl_xor_sync(0xffffffffu, y[c], 4);
-            m1[h][c] = fma(y[c], ai[c], m1[h][c]);
-            if (q8 == 0) p0[c] = fma(y[c], bj[h][c], p0[c]);
-          }
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          p0[c] += __shfl_xor_sync(0xffffffffu, p0[c], 8);
-          p0[c] += __shfl_xor_sync(0xffffffffu, p0[c], 16);
-        }
-        if (lane == 0)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) sP0[(i & 1) * NW * 4 + wid * 4 + c] = p0[c];
-        gtick(3);
-      }
-      __syncthreads();
-      if (wid == NW - 1 && lane < 4) {
-        T sacc = T(0);
-        for (int w = 0; w < NW; ++w) sacc += sP0[((d0 - 1) & 1) * NW * 4 + w * 4 + lane];
-        sM0[(d0 - 1) * 4 + lane] = sacc;
-      }
-      if (q8 == 0)
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          if (rs + 32 * h < d1)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) sM1[(rs + 32 * h) * 4 + c] = m1[h][c];
-      // M2: the rows of a warp (lanes with the same q8), then the warps
-#pragma unroll
-      for (int s2 = 0; s2 < 2; ++s2)
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            T v = acc2[s2][u][c];
-            v += __shfl_xor_sync(0xffffffffu, v, 8);
-            v += __shfl_xor_sync(0xffffffffu, v, 16);
-            const int kg = q8 + 8 * s2;
-            if (lane < 8 && kg < nkg) sR2[(wid * d2p + 4 * kg + u) * 4 + c] = v;
-          }
+      slabs();
       __syncthreads();
       for (int e = tid; e < nkg * 16; e += TFX_THREADS) {
+        if ((e & 3) >= cn) continue;
         T v = T(0);
-        for (int w = 0; w < NW; ++w) v += sR2[w * d2p * 4 + e];
+        for (int w = 0; w < nwr; ++w) v += sR2[w * d2p * 4 + e];
         sM2[e] = v;
       }
       __syncthreads();
@@ -1076,25 +1203,25 @@ struct Engine {
   }
 
   // -------------------------------------------------------------------------
-  // Third-order gradient with the SLABS split across the team (every mode <=
-  // 64, R <= 64, and the partials below fit in the three slab stages).  CTA q
-  // streams its own slabs T[i, :, :], i in [d0 q / n, d0 (q + 1) / n), and forms
-  // for every column at once (64 x 64 register tiles, 4 x 4 outputs a thread):
+  // Third-order gradient with the SLABS split across the team (every mode and R
+  // <= 64, and the partials below fit in the idle scratch).  CTA q streams its
+  // own slabs T[i, :, :], i in [d0 q / n, d0 (q + 1) / n), and forms for every
+  // column at once
   //   Y = T[i] W2                      M0[i, :] = sum_j Y[j, :] o W1[j, :]
   //   M1 += Y o (1 W0[i, :])           M2 += (T[i]^T W1) o (1 W0[i, :])
-  // (the MTTKRP dimension tree, two small products per slab).  M0's rows go to
-  // a global scratch vector, the M1 and M2 partials to the CTA's (then idle)
-  // slab stages; after a team barrier the CTA owning column c sums the peers'
-  // partials of that column through distributed shared memory in rank order
-  // and writes grad_l = M_l - W_l P1_l (the negative of GaussNewton.py:401-427).
-  // Deterministic: every sum has a fixed order.
-  // -------------------------------------------------------------------------
-  __device__ bool l3_slab_split_ok() const {
-    const int SL = (int)g3_stage(d[1], d[2]);
-    return R <= 64 && (d[1] + d[2]) * 64 <= 3 * SL;
-  }
-
-  template <bool STAGED>
+  // (the MTTKRP dimension tree, two small products per slab): warps 0-3 the
+  // first product, warps 4-7 the second, 16 x 8 threads each with UR x UC
+  // outputs a thread.  M0's rows go to a global scratch vector, the M1 and M2
+  // partials to the CTA's (then idle) slab stages; after a team barrier the CTA
+  // owning column c sums the peers' partials of that column through distributed
+  // shared memory in rank order and writes grad_l = M_l - W_l P1_l (the negative
+  // of GaussNewton.py:401-427).  Deterministic: every sum has a fixed order.
+  // Bound by instruction issue; the tile follows the sizes because rows and
+  // columns past the end are computed all the same.  A gradient of 10^3, R 10, FP64
+  // on 8 CTAs: 10 us, where columns shared out took 63; 30^3, R 20, FP32 on 16:
+  // 8.4 and 27; 50^3, R 50 (in 64 x 64 tiles of both products on all 256 threads
+  // in turn, partials read row by row from the peers): 27 and 44.  // -------------------------------------------------------------------------
+  template <bool STAGED, int UR, int UC>
   __device__ __noinline__ void gradient_l3s() {
     long long gt = gprof ? clock64() : 0;
     auto gtick = [&](int ph) {
@@ -1104,7 +1231,6 @@ struct Engine {
         gt = now;
       }
     };
-    constexpr int NW = TFX_THREADS / 32;
     const int d0 = d[0], d1 = d[1], d2 = d[2];
     char* smb = dyn_smem();
     const T* Wl = STAGED ? (const T*)(smb + cgo.sWf) : W;
@@ -1112,17 +1238,18 @@ struct Engine {
     const int p1s = STAGED ? ((ncol + 3) & ~3) : R;  // P1 column stride
     const int p1c = STAGED ? 0 : c0;    // P1 column offset
     const int SL = (int)g3_stage(d1, d2);
-    T* sT = (T*)(smb + g3off);  // 3 stages, then the M1 | M2 partials (64 columns a row)
+    T* sT = (T*)(smb + g3off);  // 3 stages, then the M1 | M2 partials (column-major)
     T* sM1p = sT;
-    T* sM2p = sT + d1 * 64;
-    T* sP0x = sT + g3_p0x(d0, d1, d2);  // [2][NW][64] M0 warp partials
+    T* sM2p = sT + d1 * R;
+    T* sP0x = sT + g3_p0x(d0, d1, d2);  // [2][4][64] M0 warp partials
     unsigned long long* mbar = (unsigned long long*)(smb + g3off + g3_floats(d0, d1, d2) * sizeof(T));
     const T* W0 = Wl + off[0];
     const T* W1 = Wl + off[1];
     const T* W2 = Wl + off[2];
     T* M0g = z + off[0];  // M0 rows, column-major like the factors (z is free outside the CG)
-    const int lane = tid & 31, wid = tid >> 5;
-    const int tx = tid & 15, ty = tid >> 4;
+    const int lane = tid & 31, w4 = (tid >> 5) & 3;
+    const bool first = tid < TFX_THREADS / 2;  // Y (rows j, sum over k), else M2 (rows k, sum over j)
+    const int tx = tid & 7, ty = (tid >> 3) & 15;
     const int i0 = (int)((long long)d0 * tm.rank / tm.size);
     const int ns = (int)((long long)d0 * (tm.rank + 1) / tm.size) - i0;
     const unsigned bytes = (unsigned)((size_t)d1 * d2 * sizeof(T));
@@ -1146,27 +1273,36 @@ struct Engine {
       const unsigned par = (n / 3) & 1;
       if (!mbar_wait_bounded(mb, par, 1u << 24)) g3err = 1;
     };
-    // M0 row of slab t from the warp partials of buffer (t & 1), by 64 threads
+    // M0 row of slab t from the warp partials of buffer (t & 1), by threads of
+    // the second half (which has less to do)
     auto m0_row = [&](int t) {
-      if (tid < 64 && tid < R) {
-        const T* pp = sP0x + (t & 1) * NW * 64 + tid;
-        T sacc = pp[0];
-#pragma unroll
-        for (int w = 1; w < NW; ++w) sacc += pp[w * 64];
-        M0g[tid * d0 + i0 + t] = sacc;
+      const int r = tid - TFX_THREADS / 2;
+      if (r >= 0 && r < R) {
+        const T* pp = sP0x + (t & 1) * 4 * 64 + r;
+        M0g[r * d0 + i0 + t] = ((pp[0] + pp[64]) + pp[128]) + pp[192];
       }
     };
+    // the thread's rows and columns: those past the end read the last one and
+    // are not stored
+    const int dr = first ? d1 : d2, dk = first ? d2 : d1;
+    const int as = first ? d2 : 1, ak = first ? 1 : d2;  // T[i]'s strides along rows and along the sum
+    const T* Wb = first ? W2 : W1;
+    int ra[UR], rb[UC];
+#pragma unroll
+    for (int u = 0; u < UR; ++u) ra[u] = min(ty + 16 * u, dr - 1) * as;
+#pragma unroll
+    for (int v = 0; v < UC; ++v) rb[v] = min(tx + 8 * v, R - 1);
+    // two steps of the sum in one load where every row starts on a pair
+    const bool even = ((d1 | d2 | (R * d0)) & 1) == 0;
+    const bool work = 4 * w4 < dr;  // some row of the warp exists (UR == 1)
     __syncthreads();  // every stage is free (the previous phase ended with barriers)
     if (ns > 0) issue(0);
     if (ns > 1) issue(1);
-    T m1a[4][4], m2a[4][4];
+    T ma[UR][UC];
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+    for (int u = 0; u < UR; ++u)
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        m1a[u][v] = T(0);
-        m2a[u][v] = T(0);
-      }
+      for (int v = 0; v < UC; ++v) ma[u][v] = T(0);
     gtick(0);
     for (int t = 0; t < ns; ++t) {
       wait_slab(t);
@@ -1177,130 +1313,207 @@ struct Engine {
       gtick(2);
       const T* tr = sT + ((g3base + t) % 3) * SL;
       const int i = i0 + t;
-      T w0[4];
+      if (work) {
+        T w0[UC], y[UR][UC];
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const int r = tx + 16 * v;
-        w0[v] = r < R ? W0[r * d0 + i] : T(0);
-      }
-      // Y = T[i] W2 (rows j = ty + 16u, columns r = tx + 16v)
-      T y[4][4];
+        for (int v = 0; v < UC; ++v) w0[v] = W0[rb[v] * d0 + i];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < UR; ++u)
 #pragma unroll
-        for (int v = 0; v < 4; ++v) y[u][v] = T(0);
+          for (int v = 0; v < UC; ++v) y[u][v] = T(0);
+        if (even && first) {
 #pragma unroll 2
-      for (int k = 0; k < d2; ++k) {
-        T a[4], b[4];
+          for (int k = 0; k < dk; k += 2) {
+            T a[UR][2], b[UC][2];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) a[u] = (ty + 16 * u < d1) ? tr[(ty + 16 * u) * d2 + k] : T(0);
+            for (int u = 0; u < UR; ++u) lds2(tr + ra[u] + k, a[u]);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) b[v] = (tx + 16 * v < R) ? W2[(tx + 16 * v) * d2 + k] : T(0);
+            for (int v = 0; v < UC; ++v) lds2(W2 + rb[v] * d2 + k, b[v]);
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+            for (int w = 0; w < 2; ++w)
 #pragma unroll
-          for (int v = 0; v < 4; ++v) y[u][v] = fma(a[u], b[v], y[u][v]);
-      }
-      // M1 partial and this slab's M0 partial (over the thread's rows)
-      T p[4] = {T(0), T(0), T(0), T(0)};
+              for (int u = 0; u < UR; ++u)
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int j = ty + 16 * u;
+                for (int v = 0; v < UC; ++v) y[u][v] = fma(a[u][w], b[v][w], y[u][v]);
+          }
+        } else if (even) {
+#pragma unroll 2
+          for (int j = 0; j < dk; j += 2) {
+            T a[2][UR], b[UC][2];
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const int r = tx + 16 * v;
-          m1a[u][v] = fma(y[u][v], w0[v], m1a[u][v]);
-          if (j < d1 && r < R) p[v] = fma(y[u][v], W1[r * d1 + j], p[v]);
+            for (int u = 0; u < UR; ++u) {
+              a[0][u] = tr[j * d2 + ra[u]];
+              a[1][u] = tr[(j + 1) * d2 + ra[u]];
+            }
+#pragma unroll
+            for (int v = 0; v < UC; ++v) lds2(W1 + rb[v] * d1 + j, b[v]);
+#pragma unroll
+            for (int w = 0; w < 2; ++w)
+#pragma unroll
+              for (int u = 0; u < UR; ++u)
+#pragma unroll
+                for (int v = 0; v < UC; ++v) y[u][v] = fma(a[w][u], b[v][w], y[u][v]);
+          }
+        } else {
+#pragma unroll 2
+          for (int k = 0; k < dk; ++k) {
+            T a[UR], b[UC];
+#pragma unroll
+            for (int u = 0; u < UR; ++u) a[u] = tr[ra[u] + k * ak];
+#pragma unroll
+            for (int v = 0; v < UC; ++v) b[v] = Wb[rb[v] * dk + k];
+#pragma unroll
+            for (int u = 0; u < UR; ++u)
+#pragma unroll
+              for (int v = 0; v < UC; ++v) y[u][v] = fma(a[u], b[v], y[u][v]);
+          }
         }
+#pragma unroll
+        for (int u = 0; u < UR; ++u)
+#pragma unroll
+          for (int v = 0; v < UC; ++v) ma[u][v] = fma(y[u][v], w0[v], ma[u][v]);
+        if (first) {
+          // this slab's M0 partial: the thread's rows, then the warp's
+          T p[UC];
+#pragma unroll
+          for (int v = 0; v < UC; ++v) p[v] = T(0);
+#pragma unroll
+          for (int u = 0; u < UR; ++u) {
+            const int j = ty + 16 * u;
+            if (j < d1)
+#pragma unroll
+              for (int v = 0; v < UC; ++v) p[v] = fma(y[u][v], W1[rb[v] * d1 + j], p[v]);
+          }
+#pragma unroll
+          for (int v = 0; v < UC; ++v) {
+            p[v] += __shfl_xor_sync(0xffffffffu, p[v], 8);
+            p[v] += __shfl_xor_sync(0xffffffffu, p[v], 16);
+          }
+          if (lane < 8)
+#pragma unroll
+            for (int v = 0; v < UC; ++v) sP0x[(t & 1) * 4 * 64 + w4 * 64 + tx + 8 * v] = p[v];
+        }
+      } else if (first) {
+        if (lane < 8)
+#pragma unroll
+          for (int v = 0; v < UC; ++v) sP0x[(t & 1) * 4 * 64 + w4 * 64 + tx + 8 * v] = T(0);
       }
-#pragma unroll
-      for (int v = 0; v < 4; ++v) p[v] += __shfl_xor_sync(0xffffffffu, p[v], 16);
-      if (lane < 16)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) sP0x[(t & 1) * NW * 64 + wid * 64 + tx + 16 * v] = p[v];
-      // M2 partial: (T[i]^T W1)[k, r] W0[i, r] (rows k = ty + 16u)
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) y[u][v] = T(0);
-#pragma unroll 2
-      for (int j = 0; j < d1; ++j) {
-        T a[4], b[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) a[u] = (ty + 16 * u < d2) ? tr[j * d2 + ty + 16 * u] : T(0);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) b[v] = (tx + 16 * v < R) ? W1[(tx + 16 * v) * d1 + j] : T(0);
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int v = 0; v < 4; ++v) y[u][v] = fma(a[u], b[v], y[u][v]);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) m2a[u][v] = fma(y[u][v], w0[v], m2a[u][v]);
       gtick(3);
     }
     __syncthreads();  // every slab consumed; the stages are idle (every copy was waited for)
     if (ns > 0) m0_row(ns - 1);
+    {
+      T* mp = first ? sM1p : sM2p;
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < UR; ++u)
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const int r = tx + 16 * v, row = ty + 16 * u;
-        if (r < R) {
-          if (row < d1) sM1p[row * 64 + r] = m1a[u][v];
-          if (row < d2) sM2p[row * 64 + r] = m2a[u][v];
+        for (int v = 0; v < UC; ++v) {
+          const int r = tx + 8 * v, row = ty + 16 * u;
+          if (r < R && row < dr) mp[r * dr + row] = ma[u][v];
         }
-      }
+    }
     g3base += ns;
     tm.sync();  // partials and M0 rows visible to the team
     gtick(4);
     const int sd = d0 + d1 + d2;
-    for (int e = tid; e < sd * ncol; e += TFX_THREADS) {
-      const int c = e / sd;
-      int l = 0, i = e - c * sd;
-      if (i >= d0) {
-        i -= d0;
-        l = 1;
-        if (i >= d1) {
-          i -= d1;
-          l = 2;
+    // one row of one mode and NC of the own columns a thread: four share the
+    // factor's and a vector read of P1's row
+    auto rows_out = [&](auto ncc) {
+      constexpr int NC = decltype(ncc)::value;
+      const int ng = (ncol + NC - 1) / NC;
+      for (int e = tid; e < sd * ng; e += TFX_THREADS) {
+        const int cb = (e / sd) * NC, cn = min(NC, ncol - cb);
+        int l = 0, i = e % sd;
+        if (i >= d0) {
+          i -= d0;
+          l = 1;
+          if (i >= d1) {
+            i -= d1;
+            l = 2;
+          }
         }
-      }
-      const int col = c0 + c;
-      T m;
-      if (l == 0) {
-        m = __ldcg(M0g + col * d0 + i);
-      } else {
-        const T* part = (l == 1 ? sM1p : sM2p) + i * 64 + col;
-        T pv[TFX_MAX_TEAM];
+        const int dl = d[l], col = c0 + cb;
+        T m[NC], wp[NC];
+        if (l == 0) {
 #pragma unroll
-        for (int q = 0; q < TFX_MAX_TEAM; ++q) pv[q] = q < tm.size ? *tm.peer(part, q) : T(0);
-        m = pv[0];
+          for (int c = 0; c < NC; ++c) m[c] = __ldcg(M0g + min(col + c, R - 1) * d0 + i);
+        } else {
+          const T* part = (l == 1 ? sM1p : sM2p) + col * dl + i;
 #pragma unroll
-        for (int q = 1; q < TFX_MAX_TEAM; ++q)
-          if (q < tm.size) m += pv[q];
+          for (int c = 0; c < NC; ++c)
+            if (c < cn) {
+              T pv[TFX_MAX_TEAM];
+#pragma unroll
+              for (int q = 0; q < TFX_MAX_TEAM; ++q) pv[q] = q < tm.size ? *tm.peer(part + c * dl, q) : T(0);
+              m[c] = pv[0];
+#pragma unroll
+              for (int q = 1; q < TFX_MAX_TEAM; ++q)
+                if (q < tm.size) m[c] += pv[q];
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < NC; ++c) wp[c] = T(0);
+        const T* p1 = P1l + (size_t)l * R * p1s + p1c + cb;
+        const T* wl = Wl + off[l] + i;
+#pragma unroll 4
+        for (int s2 = 0; s2 < R; ++s2) {
+          const T w = wl[s2 * dl];
+          if (STAGED && NC == 4) {
+            T q[4];
+            lds4(p1 + s2 * p1s, q);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) wp[c] = fma(w, q[c], wp[c]);
+          } else {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) wp[c] = fma(w, p1[s2 * p1s + min(c, cn - 1)], wp[c]);
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+          if (c < cn) grad[off[l] + (col + c) * dl + i] = m[c] - wp[c];
       }
-      const int dl = d[l];
-      T wp = T(0);
-      const T* p1 = P1l + (size_t)l * R * p1s + p1c + c;
-      for (int s2 = 0; s2 < R; ++s2) wp = fma(Wl[off[l] + s2 * dl + i], p1[s2 * p1s], wp);
-      grad[off[l] + col * dl + i] = m - wp;
-    }
+    };
+    if (sd * ncol > TFX_THREADS)
+      rows_out(std::integral_constant<int, 4>());
+    else
+      rows_out(std::integral_constant<int, 1>());
     gtick(5);
     // the peers are done reading this CTA's partials; the CG reads every column
     tm.sync();
     gtick(7);
   }
 
+  template <bool STAGED>
+  __device__ void gradient_slabs() {
+    const int dm = max(d[1], d[2]);
+    if (dm <= 16 && R <= 16)
+      gradient_l3s<STAGED, 1, 2>();
+    else if (dm <= 32 && R <= 32)
+      gradient_l3s<STAGED, 2, 4>();
+    else
+      gradient_l3s<STAGED, 4, 8>();
+  }
+  // Slabs shared out or columns shared out: the first computes every column of
+  // its slabs in tiles, the second streams every slab for its own columns, four
+  // at a time.  Instructions a slab and warp scheduler of either, times the
+  // slabs, decide; few columns of large modes leave the tiles empty.
+  __device__ bool slab_split() const {
+    const int dm = max(d[1], d[2]);
+    if (R > 64 || (size_t)(d[1] + d[2]) * R > g3_p0x(d[0], d[1], d[2])) return false;
+    const int tile = (dm <= 16 && R <= 16) ? 2 : (dm <= 32 && R <= 32) ? 8 : 32;
+    const int slabs = (d[0] + tm.size - 1) / tm.size;
+    const int groups = ((R + tm.size - 1) / tm.size + 3) / 4;
+    const int halves = (d[1] > 32 ? 2 : 1) * (d[2] > 32 ? 2 : 1);
+    return 2 * tile * dm * slabs < groups * d[0] * (32 * halves + 48) * (d[1] > 16 ? 2 : 1);
+  }
+
   // the gradient by the fastest form that applies
   __device__ void gradient_any() {
-    if (sG3 && l3_slab_split_ok()) {
+    if (sG3 && slab_split()) {
       if (stage)
-        gradient_l3s<true>();
+        gradient_slabs<true>();
       else
-        gradient_l3s<false>();
+        gradient_slabs<false>();
     } else if (sG3) {
       if (stage)
         gradient_l3<true>();
@@ -1476,19 +1689,22 @@ struct Engine {
         Acc<T> s;
         for (int i = lane; i < d[l]; i += 32) s.fma_(col[i], col[i]);
         s.warp_reduce();
-        if (lane == 0) sNorm[p] = sqrt(s.value());
+        if (lane == 0) sNorm[p] = s.value();
       }
       __syncthreads();
+      // (one thread a norm: a square root by each warp's first lane would hold
+      // the FP64 pipes once a column)
+      for (int p = tid; p < L * ncol; p += TFX_THREADS) sNorm[p] = sqrt(sNorm[p]);
+      __syncthreads();
       // one balancing factor per (mode, column): (prod_m n_m)^(1/L) / n_l
-      for (int c = tid; c < ncol; c += TFX_THREADS) {
+      // (cbrt for three modes: a fraction of pow's FP64 instructions)
+      for (int p = tid; p < L * ncol; p += TFX_THREADS) {
+        const int c = p % ncol;
         double prod = 1.0;
         for (int m = 0; m < L; ++m) prod *= sNorm[m * ncol + c];
-        if (prod != 0.0) {
-          const double num = pow(prod, 1.0 / (double)L);
-          for (int m = 0; m < L; ++m) sScale[m * ncol + c] = (T)(num / sNorm[m * ncol + c]);
-        } else {
-          for (int m = 0; m < L; ++m) sScale[m * ncol + c] = T(1);
-        }
+        double sc = 1.0;
+        if (prod != 0.0) sc = (L == 3 ? cbrt(prod) : pow(prod, 1.0 / (double)L)) / sNorm[p];
+        sScale[p] = (T)sc;
       }
       __syncthreads();
       for_own([&](int e, int l, int c) { dst[e] = sScale[l * ncol + c] * src[e]; });
@@ -1576,10 +1792,27 @@ struct Engine {
     __syncthreads();  // staged W1, W2; every stage is free (the gradient ended with barriers)
     if (nmy > 0) issue(0);
     if (nmy > 1) issue(1);
+    // W0[i, :] of the next slab: lane r of every warp holds columns r and
+    // r + 32 (one L2 latency a slab, where a load in the loop over r cost one
+    // every other column)
+    const int lane = tid & 31;
+    T an[2] = {T(0), T(0)};
+    auto load_a = [&](int t) {
+      const T* a = Wf + off[0] + first + t * step;
+      if (lane < R) an[0] = a[lane * d0];
+      if (lane + 32 < R) an[1] = a[(lane + 32) * d0];
+    };
+    if (nmy > 0) load_a(0);
     const int nk4 = d2p >> 2, nj4 = d1p >> 2;
     const int j4 = tid / nk4, k4 = tid - j4 * nk4;
     const bool active = tid < nj4 * nk4;  // <= 16 x 16
-    Acc<T> acc;
+    const bool wactive = (tid & ~31) < nj4 * nk4;
+    // FP64: a warp takes 20 instructions a column for a 4 x 4 block and 2 for
+    // one entry, and four pipes share the warps, so up to about 1000 entries
+    // single entries on more warps are the shorter way (10^3, R 10: 20.7 -> 6 us
+    // with the prefetch above; the FP32 block at 50^3 is unmoved at 20)
+    const bool single = sizeof(T) == 8 && d1 * d2 <= 1024;
+    Acc<T> acc, acc4[3];  // the 4 x 4 block's rows add separately: a short chain
     for (int t = 0; t < nmy; ++t) {
       const unsigned n = g3base + t;
       {
@@ -1596,20 +1829,38 @@ struct Engine {
       }
       __syncthreads();  // every warp is past slab t-1: its stage may be refilled
       if (t + 2 < nmy) issue(t + 2);
-      if (active) {
-        const int i = first + t * step;
+      const T ac[2] = {an[0], an[1]};
+      if (t + 1 < nmy) load_a(t + 1);
+      const T* slab = sT + (n % 3) * SL;
+      if (single) {
+        const int np = d1 * d2;
+        for (int e0 = tid & ~31; e0 < np; e0 += TFX_THREADS) {
+          const int e = min(e0 + lane, np - 1), j = e / d2, k = e - j * d2;
+          T x = T(0);
+#pragma unroll 4
+          for (int r = 0; r < R; ++r) {
+            const T ai = __shfl_sync(0xffffffffu, r < 32 ? ac[0] : ac[1], r & 31);
+            x = fma(ai * sBt[r * d1p + j], sCt[r * d2p + k], x);
+          }
+          if (e0 + lane < np) {
+            const T df = slab[e] - x;
+            acc.fma_(df, df);
+          }
+        }
+      } else if (wactive) {
         T x[4][4];
 #pragma unroll
         for (int u = 0; u < 4; ++u)
 #pragma unroll
           for (int v = 0; v < 4; ++v) x[u][v] = T(0);
-        const T* a = Wf + off[0] + i;
-#pragma unroll 2
+        const T* pb = sBt + (active ? 4 * j4 : 0);
+        const T* pc = sCt + (active ? 4 * k4 : 0);
+#pragma unroll 4
         for (int r = 0; r < R; ++r) {
-          const T ai = a[r * d0];
+          const T ai = __shfl_sync(0xffffffffu, r < 32 ? ac[0] : ac[1], r & 31);
           T b[4], c[4];
-          lds4(sBt + r * d1p + 4 * j4, b);
-          lds4(sCt + r * d2p + 4 * k4, c);
+          lds4(pb + r * d1p, b);
+          lds4(pc + r * d2p, c);
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             const T bu = ai * b[u];
@@ -1617,24 +1868,30 @@ struct Engine {
             for (int v = 0; v < 4; ++v) x[u][v] = fma(bu, c[v], x[u][v]);
           }
         }
-        const T* slab = sT + (n % 3) * SL;
+        if (active) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int j = 4 * j4 + u;
+          for (int u = 0; u < 4; ++u) {
+            const int j = 4 * j4 + u;
 #pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            const int k = 4 * k4 + v;
-            if (j < d1 && k < d2) {
-              const T df = slab[j * d2 + k] - x[u][v];
-              acc.fma_(df, df);
+            for (int v = 0; v < 4; ++v) {
+              const int k = 4 * k4 + v;
+              if (j < d1 && k < d2) {
+                const T df = slab[j * d2 + k] - x[u][v];
+                if (u == 0)
+                  acc.fma_(df, df);
+                else
+                  acc4[u - 1].fma_(df, df);
+              }
             }
           }
         }
       }
     }
     g3base += nmy;
+#pragma unroll
+    for (int u = 0; u < 3; ++u) acc.add2_(acc4[u]);
     Acc<T> v1[1] = {acc}, tot[1];
-    team_sum_push<1>(tm, v1, tot, (PushSlots<1>*)(smb + cgo.wsl), flipw);
+    team_sum_push<1>(tm, v1, tot, (PushSlots*)(smb + cgo.wsl), flipw);
     // one thread forms the double result (FP64 is slow on GB300), the CTA reads it
     double* res = (double*)(smb + e3off);
     __syncthreads();  // the staged factors are no longer read
@@ -1912,10 +2169,8 @@ __device__ __forceinline__ void engine_setup(Engine<T, TS>& E, const tfx_dgn_pro
   E.cgo.sM = sp.sM;
   E.cgo.sDG = sp.sDG;
   E.cgo.rs4 = sp.rs4;
-  E.cgo.rs1 = sp.rs1;
   E.cgo.sVec = sp.sVec;
   E.cgo.wsl = sp.wsl;
-  E.rs1b = (RedScratch<1>*)(smem + sp.rs1b);
   E.sScale = (T*)(smem + sp.sScale);
   E.aliased = op.aliased != 0;
   // third-order gradient path: every mode <= 64 (the plan), 16-byte slabs
@@ -1936,10 +2191,35 @@ __device__ __forceinline__ void engine_setup(Engine<T, TS>& E, const tfx_dgn_pro
   }
   __syncthreads();
   E.flip1 = 0;
-  E.flip1b = 0;
   E.flip4 = 0;
   E.flip12 = 0;
   E.flipw = 0;
+}
+
+// The stop tests after iteration `it` (GaussNewton.py:229-283): the reference's
+// stop code, or -1 to go on.  hErr and hImp hold the iterations so far.
+static __device__ __noinline__ int stop_code(int it, int cnst, double error, double ssz, double imp, double gmax,
+                                             double tol, double tol_step, double tol_improv,
+                                             double tol_grad, double limit, const double* hErr,
+                                             const double* hImp) {
+  if (it <= 1) return -1;
+  if (error < tol) return 0;
+  if (ssz < tol_step) return 1;
+  if (imp < tol_improv) return 2;
+  if (gmax < tol_grad) return 3;
+  if (it > 2 * cnst && it % cnst == 0) {
+    double m1 = 0.0, m2 = 0.0, m3 = 0.0;
+    for (int j = it - 2 * cnst; j < it - cnst; ++j) m1 += hErr[j];
+    for (int j = it - cnst; j < it; ++j) m2 += hErr[j];
+    for (int j = it - cnst; j < it; ++j) m3 += hImp[j];
+    m1 /= cnst;
+    m2 /= cnst;
+    m3 /= cnst;
+    if (m1 - m2 <= tol_improv) return 4;
+    if (m3 < 1e-3 * m2) return 7;
+  }
+  if (error > limit) return 6;
+  return -1;
 }
 
 template <class T, int TS>
@@ -1976,6 +2256,7 @@ __device__ void solve_problem(const tfx_dgn_problem& pb, const tfx_dgn_options& 
     tol = tol_step = tol_improv = tol_grad = 0.0;
   }
   const int cnst = 1 + maxiter / 10;
+  const double limit = fmax(1.0, Tsize * Tsize) / (1e-16 + tol);
   double error = 1.0, best_error = INFINITY;
   int stop = 5, it = 0, n_dogleg = 0;
   long long matvecs = 0;
@@ -2033,53 +2314,60 @@ __device__ void solve_problem(const tfx_dgn_problem& pb, const tfx_dgn_options& 
     }
     tick(5);
     // gain ratio, step size, gradient norm (x_new - x_old with the final x)
-    Acc<T> va[4];
-    MaxAcc<T> ga[1];
-    double v[4], gm[1];
+    Acc<T> va[3], vt[3];
+    T ga = T(0), gt;
     const T dmp = (T)E.damp;
     E.for_own([&](int e, int l, int c) {
       const T dx = E.xn[e] - E.xc[e];
       va[0].fma_(dx, E.grad[e] + dmp * dx);
       va[1].fma_(dx, dx);
       va[2].fma_(E.xc[e], E.xc[e]);
-      ga[0].v = fmax(ga[0].v, fabs(E.grad[e]));
+      ga = fmax(ga, fabs(E.grad[e]));
     });
-    team_sum_acc<4, T>(E.tm, va, v, E.rs4, E.flip4);
-    team_reduce_acc<1, true>(E.tm, ga, gm, E.rs1b, E.flip1b);
-    const double num = (Tsize * Tsize) * (old_error * old_error - error * error);
-    double gain;
-    if (v[0] != 0.0) {
-      gain = num / v[0];
-    } else if (num != 0.0) {
-      gain = (num > 0.0 ? 1.0 : -1.0) * INFINITY;
-    } else {
-      gain = -INFINITY;
-    }
-    if (op.use_damp_sched) {
-      E.damp = pb.damp_sched[it];
-    } else if (gain < 0.25) {
-      E.damp = 3.0 * E.damp;
-    } else if (gain > 0.75) {
-      E.damp = E.damp / 3.0;
-    }
-    if (error < best_error) {
-      best_error = error;
-      E.for_own([&](int e, int l, int c) { best[e] = E.W[e]; });
-    }
-    const double ssz = sqrt(v[1]) / sqrt(v[2]);
-    const double imp = (it == 0) ? error : fabs(error - old_error);
-    __syncthreads();
+    team_push_sum3_max<T>(E.tm, va, ga, vt, gt, (PushSlots*)(smem + sp.wsl), E.flipw, 2);
+    // The scalar control runs on one thread of two warps, the damping on the
+    // first and the stop tests on the second, and reaches the others through
+    // shared memory: an FP64 division or square root is tens of instructions
+    // of 64 cycles, and eight warps of a CTA running them queue for four pipes
+    // (with the one exchange above, 14.8 -> 9 us an iteration).
     if (threadIdx.x == 0) {
+      const double num = (Tsize * Tsize) * (old_error * old_error - error * error);
+      const double v0 = vt[0].value();
+      double gain;
+      if (v0 != 0.0) {
+        gain = num / v0;
+      } else if (num != 0.0) {
+        gain = (num > 0.0 ? 1.0 : -1.0) * INFINITY;
+      } else {
+        gain = -INFINITY;
+      }
+      double dn = E.damp;
+      if (op.use_damp_sched) {
+        dn = pb.damp_sched[it];
+      } else if (gain < 0.25) {
+        dn = 3.0 * dn;
+      } else if (gain > 0.75) {
+        dn = dn / 3.0;
+      }
+      E.sMisc[1] = dn;
+    } else if (threadIdx.x == 32) {
+      const double ssz = sqrt(vt[1].value()) / sqrt(vt[2].value()), gmax = (double)gt;
+      const double imp = (it == 0) ? error : fabs(error - old_error);
       hErr[it] = error;
       hImp[it] = imp;
       if (E.tm.rank == 0) {
         errors[it] = error;
         step_sizes[it] = ssz;
         improv[it] = imp;
-        gradients[it] = gm[0];
+        gradients[it] = gmax;
       }
+      E.sMisc[2] = (double)stop_code(it, cnst, error, ssz, imp, gmax, tol, tol_step, tol_improv, tol_grad,
+                                     limit, hErr, hImp);
     }
-    __syncthreads();
+    if (error < best_error) {
+      best_error = error;
+      E.for_own([&](int e, int l, int c) { best[e] = E.W[e]; });
+    }
     // swap x buffers: xc <- xn
     {
       T* t = E.xc;
@@ -2087,23 +2375,11 @@ __device__ void solve_problem(const tfx_dgn_problem& pb, const tfx_dgn_options& 
       E.xn = t;
     }
     E.tm.sync();
-    if (it > 1) {
-      if (error < tol) { stop = 0; break; }
-      if (ssz < tol_step) { stop = 1; break; }
-      if (imp < tol_improv) { stop = 2; break; }
-      if (gm[0] < tol_grad) { stop = 3; break; }
-      if (it > 2 * cnst && it % cnst == 0) {
-        double m1 = 0.0, m2 = 0.0, m3 = 0.0;
-        for (int j = it - 2 * cnst; j < it - cnst; ++j) m1 += hErr[j];
-        for (int j = it - cnst; j < it; ++j) m2 += hErr[j];
-        for (int j = it - cnst; j < it; ++j) m3 += hImp[j];
-        m1 /= cnst;
-        m2 /= cnst;
-        m3 /= cnst;
-        if (m1 - m2 <= tol_improv) { stop = 4; break; }
-        if (m3 < 1e-3 * m2) { stop = 7; break; }
-      }
-      if (error > fmax(1.0, Tsize * Tsize) / (1e-16 + tol)) { stop = 6; break; }
+    E.damp = E.sMisc[1];
+    const int code = (int)E.sMisc[2];
+    if (code >= 0) {
+      stop = code;
+      break;
     }
   }
   const int iters = (it < maxiter) ? it + 1 : maxiter;

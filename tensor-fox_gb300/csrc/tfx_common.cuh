@@ -14,6 +14,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace cgx = cooperative_groups;
 
 #define TFX_MAX_ORDER 12
@@ -80,6 +82,7 @@ struct Acc<float> {
     lo = err - (hi - s);
   }
   __device__ __forceinline__ void add(float x) { add2(x, 0.f); }
+  __device__ __forceinline__ void add2_(const Acc<float>& b) { add2(b.hi, b.lo); }
   __device__ __forceinline__ void fma_(float x, float y) {
     const float p = x * y;
     add2(p, fmaf(x, y, -p));
@@ -102,6 +105,7 @@ struct Acc<double> {
   double v;
   __device__ __forceinline__ Acc() : v(0.0) {}
   __device__ __forceinline__ void add(double x) { v += x; }
+  __device__ __forceinline__ void add2_(const Acc<double>& b) { v += b.v; }
   __device__ __forceinline__ void fma_(double x, double y) { v = fma(x, y, v); }
   __device__ __forceinline__ double value() const { return v; }
   __device__ __forceinline__ double hi_or_v() const { return v; }
@@ -169,17 +173,6 @@ struct DMax {
   __device__ __forceinline__ void warp_reduce() { v = warp_max(v); }
   __device__ __forceinline__ double value() const { return v; }
 };
-template <class T>
-struct MaxAcc {  // running maximum in the working precision
-  T v;
-  __device__ __forceinline__ MaxAcc() : v(T(0)) {}
-  __device__ __forceinline__ void warp_reduce() {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  }
-  __device__ __forceinline__ double value() const { return (double)v; }
-};
-
 template <int NV, bool MAX>
 __device__ __forceinline__ void team_reduce(const Team& tm, double (&v)[NV], RedScratch<NV>* rs, int& flip) {
   if (MAX) {
@@ -195,114 +188,23 @@ __device__ __forceinline__ void team_reduce(const Team& tm, double (&v)[NV], Red
   }
 }
 
-template <int NV, class T>
-__device__ __forceinline__ void team_sum_acc(const Team& tm, Acc<T> (&v)[NV], double (&out)[NV], RedScratch<NV>* rs,
-                                             int& flip) {
-  team_reduce_acc<NV, false>(tm, v, out, rs, flip);
-}
-
-// One-barrier team sum for the CG loop.  Every warp publishes its reduced
-// partial (a float-float pair, or a double on the FP64 path) in its own
-// double-buffered shared-memory slot; after one team barrier every warp of
-// every CTA reads all team_size x 8 partials, local and remote, and combines
-// them with shuffles.  No CTA-level barrier and no FP64 arithmetic on the FP32
-// path; every thread returns the totals as accumulators.  Two calls in a row
-// may reuse a slot buffer only after the barrier of the call in between,
-// which the alternating `flip` guarantees.
-template <int NV>
-struct WarpSlots {
-  double raw[2][TFX_THREADS / 32][NV];
-};
-
-template <int NV>
-__device__ __forceinline__ void team_sum_fast(const Team& tm, Acc<float> (&v)[NV], Acc<float> (&out)[NV],
-                                              WarpSlots<NV>* ws, int& flip) {
-  constexpr int NW = TFX_THREADS / 32;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int j = 0; j < NV; ++j) v[j].warp_reduce();
-  float2* mine = reinterpret_cast<float2*>(&ws->raw[flip][0][0]);
-  if (lane == 0)
-#pragma unroll
-    for (int j = 0; j < NV; ++j) mine[wid * NV + j] = make_float2(v[j].hi, v[j].lo);
-  tm.sync();
-  const int np = tm.size * NW;
-  float2 p[(TFX_MAX_TEAM * NW + 31) / 32][NV];
-#pragma unroll
-  for (int u = 0; u < (TFX_MAX_TEAM * NW + 31) / 32; ++u) {
-    const int q = lane + 32 * u;
-    if (q < np) {
-      const float2* src = tm.peer(mine, q / NW) + (q % NW) * NV;
-#pragma unroll
-      for (int j = 0; j < NV; ++j) p[u][j] = src[j];
-    } else {
-#pragma unroll
-      for (int j = 0; j < NV; ++j) p[u][j] = make_float2(0.f, 0.f);
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < NV; ++j) {
-    Acc<float> a;
-#pragma unroll
-    for (int u = 0; u < (TFX_MAX_TEAM * NW + 31) / 32; ++u) a.add2(p[u][j].x, p[u][j].y);
-    a.warp_reduce();
-    out[j] = a;
-  }
-  flip ^= 1;
-}
-
-template <int NV>
-__device__ __forceinline__ void team_sum_fast(const Team& tm, Acc<double> (&v)[NV], Acc<double> (&out)[NV],
-                                              WarpSlots<NV>* ws, int& flip) {
-  constexpr int NW = TFX_THREADS / 32;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int j = 0; j < NV; ++j) v[j].warp_reduce();
-  double* mine = &ws->raw[flip][0][0];
-  if (lane == 0)
-#pragma unroll
-    for (int j = 0; j < NV; ++j) mine[wid * NV + j] = v[j].v;
-  tm.sync();
-  const int np = tm.size * NW;
-  double p[(TFX_MAX_TEAM * NW + 31) / 32][NV];
-#pragma unroll
-  for (int u = 0; u < (TFX_MAX_TEAM * NW + 31) / 32; ++u) {
-    const int q = lane + 32 * u;
-    if (q < np) {
-      const double* src = tm.peer(mine, q / NW) + (q % NW) * NV;
-#pragma unroll
-      for (int j = 0; j < NV; ++j) p[u][j] = src[j];
-    } else {
-#pragma unroll
-      for (int j = 0; j < NV; ++j) p[u][j] = 0.0;
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < NV; ++j) {
-    Acc<double> a;
-#pragma unroll
-    for (int u = 0; u < (TFX_MAX_TEAM * NW + 31) / 32; ++u) a.add(p[u][j]);
-    a.warp_reduce();
-    out[j] = a;
-  }
-  flip ^= 1;
-}
-
 // Push-based team sum: the CTA reduces its warps' partials first (one CTA
 // barrier), then one lane per team member stores the CTA's partial into that
 // member's shared memory; after one team barrier every warp combines the
 // team_size partials sitting in its own shared memory with shuffles.  Remote
 // traffic is team_size stores per CTA and nothing remote is on the path after
-// the barrier.  Slots alternate with `flip` (see team_sum_fast).
-template <int NV>
+// the barrier.  Slots alternate with `flip`: a buffer is rewritten only after
+// the barrier of the call in between.  Calls of one to four values share the
+// slots, so the two buffers lie apart whatever the count.
+#define TFX_PUSH_MAX 4
 struct PushSlots {
-  double team[2][TFX_MAX_TEAM][NV];
-  double warp[TFX_THREADS / 32][NV];
+  double team[2][TFX_MAX_TEAM][TFX_PUSH_MAX];
+  double warp[TFX_THREADS / 32][TFX_PUSH_MAX];
 };
 
 template <int NV>
 __device__ __forceinline__ void team_sum_push(const Team& tm, Acc<float> (&v)[NV], Acc<float> (&out)[NV],
-                                              PushSlots<NV>* ps, int& flip) {
+                                              PushSlots* ps, int& flip) {
   constexpr int NW = TFX_THREADS / 32;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   float2* wslot = reinterpret_cast<float2*>(&ps->warp[0][0]);
@@ -311,14 +213,14 @@ __device__ __forceinline__ void team_sum_push(const Team& tm, Acc<float> (&v)[NV
   for (int j = 0; j < NV; ++j) v[j].warp_reduce();
   if (lane == 0)
 #pragma unroll
-    for (int j = 0; j < NV; ++j) wslot[wid * NV + j] = make_float2(v[j].hi, v[j].lo);
+    for (int j = 0; j < NV; ++j) wslot[wid * TFX_PUSH_MAX + j] = make_float2(v[j].hi, v[j].lo);
   __syncthreads();
   if (wid == 0) {
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
       Acc<float> a;
       if (lane < NW) {
-        const float2 q = wslot[lane * NV + j];
+        const float2 q = wslot[lane * TFX_PUSH_MAX + j];
         a.hi = q.x;
         a.lo = q.y;
       }
@@ -331,7 +233,7 @@ __device__ __forceinline__ void team_sum_push(const Team& tm, Acc<float> (&v)[NV
       // lanes 0..NW-1 hold the CTA total; every storing lane takes lane 0's
       a.hi = __shfl_sync(0xffffffffu, a.hi, 0);
       a.lo = __shfl_sync(0xffffffffu, a.lo, 0);
-      if (lane < tm.size) tm.peer(tslot, lane)[tm.rank * NV + j] = make_float2(a.hi, a.lo);
+      if (lane < tm.size) tm.peer(tslot, lane)[tm.rank * TFX_PUSH_MAX + j] = make_float2(a.hi, a.lo);
     }
   }
   tm.sync();
@@ -339,7 +241,7 @@ __device__ __forceinline__ void team_sum_push(const Team& tm, Acc<float> (&v)[NV
   for (int j = 0; j < NV; ++j) {
     Acc<float> a;
     if (lane < tm.size) {
-      const float2 q = tslot[lane * NV + j];
+      const float2 q = tslot[lane * TFX_PUSH_MAX + j];
       a.hi = q.x;
       a.lo = q.y;
     }
@@ -358,34 +260,120 @@ __device__ __forceinline__ void team_sum_push(const Team& tm, Acc<float> (&v)[NV
 
 template <int NV>
 __device__ __forceinline__ void team_sum_push(const Team& tm, Acc<double> (&v)[NV], Acc<double> (&out)[NV],
-                                              PushSlots<NV>* ps, int& flip) {
+                                              PushSlots* ps, int& flip) {
   constexpr int NW = TFX_THREADS / 32;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   double* wslot = &ps->warp[0][0];
   double* tslot = &ps->team[flip][0][0];
 #pragma unroll
-  for (int j = 0; j < NV; ++j) v[j].warp_reduce();
+  for (int j = 0; j < NV; ++j)
+    // a warp without terms (few owned elements) leaves the FP64 pipe alone
+    if (__any_sync(0xffffffffu, __double_as_longlong(v[j].v) != 0)) v[j].warp_reduce();
   if (lane == 0)
 #pragma unroll
-    for (int j = 0; j < NV; ++j) wslot[wid * NV + j] = v[j].v;
+    for (int j = 0; j < NV; ++j) wslot[wid * TFX_PUSH_MAX + j] = v[j].v;
   __syncthreads();
   if (wid == 0) {
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
-      double a = lane < NW ? wslot[lane * NV + j] : 0.0;
+      double a = lane < NW ? wslot[lane * TFX_PUSH_MAX + j] : 0.0;
 #pragma unroll
       for (int o = 1; o < NW; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
       a = __shfl_sync(0xffffffffu, a, 0);
-      if (lane < tm.size) tm.peer(tslot, lane)[tm.rank * NV + j] = a;
+      if (lane < tm.size) tm.peer(tslot, lane)[tm.rank * TFX_PUSH_MAX + j] = a;
     }
   }
   tm.sync();
 #pragma unroll
   for (int j = 0; j < NV; ++j) {
-    double a = lane < tm.size ? tslot[lane * NV + j] : 0.0;
+    double a = lane < tm.size ? tslot[lane * TFX_PUSH_MAX + j] : 0.0;
 #pragma unroll
-    for (int o = 1; o < TFX_MAX_TEAM; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    for (int o = 1; o < TFX_MAX_TEAM; o <<= 1)
+      if (o < tm.size) a += __shfl_xor_sync(0xffffffffu, a, o);
     out[j].v = __shfl_sync(0xffffffffu, a, 0);
+  }
+  flip ^= 1;
+}
+
+// Three sums and one maximum in one push exchange; the result is formed by
+// every warp with wid < nwo only (the others return zeros).
+template <class T>
+__device__ __forceinline__ void team_push_sum3_max(const Team& tm, Acc<T> (&v)[3], T m, Acc<T> (&out)[3], T& mout,
+                                                   PushSlots* ps, int& flip, int nwo) {
+  using S = typename std::conditional<sizeof(T) == 4, float2, double>::type;
+  constexpr int NW = TFX_THREADS / 32, P = TFX_PUSH_MAX;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  S* wslot = reinterpret_cast<S*>(&ps->warp[0][0]);
+  S* tslot = reinterpret_cast<S*>(&ps->team[flip][0][0]);
+  // lanes l < n hold partials; sums and maximum over them in every lane
+  auto fold = [&](Acc<T>(&a)[3], T& mm, int n) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      if (o >= n) break;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        if constexpr (sizeof(T) == 4) {
+          const float oh = __shfl_xor_sync(0xffffffffu, a[j].hi, o);
+          const float ol = __shfl_xor_sync(0xffffffffu, a[j].lo, o);
+          a[j].add2(oh, ol);
+        } else {
+          a[j].v += __shfl_xor_sync(0xffffffffu, a[j].v, o);
+        }
+      }
+      mm = fmax(mm, __shfl_xor_sync(0xffffffffu, mm, o));
+    }
+  };
+  auto put = [&](S* dst, const Acc<T>(&a)[3], T mm) {
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) dst[j] = make_float2(a[j].hi, a[j].lo);
+      dst[3] = make_float2(mm, 0.f);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) dst[j] = a[j].v;
+      dst[3] = mm;
+    }
+  };
+  auto get = [&](const S* src, Acc<T>(&a)[3], T& mm) {
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        a[j].hi = src[j].x;
+        a[j].lo = src[j].y;
+      }
+      mm = src[3].x;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) a[j].v = src[j];
+      mm = src[3];
+    }
+  };
+  fold(v, m, 32);
+  if (lane == 0) put(wslot + wid * P, v, m);
+  __syncthreads();
+  if (wid == 0) {
+    Acc<T> a[3];
+    T mm = T(0);
+    if (lane < NW) get(wslot + lane * P, a, mm);
+    fold(a, mm, NW);
+    // lanes 0..NW-1 hold the CTA's totals; every storing lane takes lane 0's
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      if constexpr (sizeof(T) == 4) {
+        a[j].hi = __shfl_sync(0xffffffffu, a[j].hi, 0);
+        a[j].lo = __shfl_sync(0xffffffffu, a[j].lo, 0);
+      } else {
+        a[j].v = __shfl_sync(0xffffffffu, a[j].v, 0);
+      }
+    }
+    mm = __shfl_sync(0xffffffffu, mm, 0);
+    if (lane < tm.size) put(tm.peer(tslot, lane) + tm.rank * P, a, mm);
+  }
+  tm.sync();
+  mout = T(0);
+  if (wid < nwo) {
+    if (lane < tm.size) get(tslot + lane * P, out, mout);
+    fold(out, mout, tm.size);
   }
   flip ^= 1;
 }
