@@ -272,6 +272,10 @@ int tfx_coo_sort_mode(int dtype, const int* idx32, const void* vals, long long n
  * (GaussNewton.py:401-427 on sparse2dense, Conversion.py:144-164). */
 int tfx_coo_mttkrp(int dtype, const int* sidx, const void* svals, long long nnz, const long long* rowptr, int L,
                    const int* dims, int R, int mode, const void* const* Wrow_dev, void* out, void* stream);
+/* The same from a host array of the L device pointers (read before the call
+ * returns), which go into the kernels' parameters. */
+int tfx_coo_mttkrp_rows(int dtype, const int* sidx, const void* svals, long long nnz, const long long* rowptr, int L,
+                        const int* dims, int R, int mode, const void* const* Wrow, void* out, void* stream);
 /* The same COO MTTKRP from BF16 factor rows with per-column scaling (FP32
  * values and sums): tfx_factors_bf16 writes row-major BF16 copies of the flat
  * FP32 factors, column r of mode m divided by scale[m*R + r], a power of two
@@ -288,6 +292,9 @@ int tfx_coo_mttkrp_bf16(const int* sidx, const float* svals, long long nnz, cons
 size_t tfx_sparse_residual_scratch_bytes(void);
 int tfx_sparse_residual(int dtype, const int* idx32, const void* vals, long long nnz, int L, const int* dims, int R,
                         const void* const* Wrow_dev, double* out, void* scratch, void* stream);
+/* The same from a host array of the L device pointers (read before the call returns). */
+int tfx_sparse_residual_rows(int dtype, const int* idx32, const void* vals, long long nnz, int L, const int* dims,
+                             int R, const void* const* Wrow, double* out, void* scratch, void* stream);
 /* Compression.py:211-215 with 240-258 (dot_product_mkl(Tl, Tl.T)): dense
  * T_(l) T_(l)^T from COO; entries of one fibre are matched by comparing their
  * coordinates, so any dimensions are exact; nnz < 2^31 (TFX_STATUS_ERR_ARG

@@ -33,6 +33,16 @@ struct CooShape {
   int dims[TFX_MAX_ORDER];
 };
 
+// The row-major factors' addresses, in the kernel's parameters or in a device
+// array (an array formed per call is a blocking copy per call: one sweep and the
+// residual of 1e7 entries, R 16, order 3: 799 -> 740 us without the four).
+template <class T>
+struct RowPtrs {
+  const T* p[TFX_MAX_ORDER];
+  const T* const* dev;
+  __device__ __forceinline__ const T* operator[](int m) const { return dev ? dev[m] : p[m]; }
+};
+
 // ---------------------------------------------------------------------------
 __global__ void k_coo_encode(const long long* __restrict__ idx64, long long nnz, int L, CooShape sh,
                              int* __restrict__ idx32, int* __restrict__ err) {
@@ -114,7 +124,7 @@ __global__ void k_scatter_rows(const int* __restrict__ idx32, const T* __restric
 template <class T, int RB>
 __global__ void __launch_bounds__(256) k_coo_mttkrp(const int* __restrict__ sidx, const T* __restrict__ svals,
                                                     long long nnz, const long long* __restrict__ rowptr, CooShape sh,
-                                                    int mode, const T* const* __restrict__ Wrow, T* __restrict__ out,
+                                                    int mode, const RowPtrs<T> Wrow, T* __restrict__ out,
                                                     int r0) {
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -160,7 +170,7 @@ __device__ __forceinline__ float4 ld4(const float* p, bool aligned) {
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256, 4) k_coo_mttkrp_f4(const int* __restrict__ sidx, const float* __restrict__ svals,
                                                        long long nnz, const long long* __restrict__ rowptr, CooShape sh,
-                                                       int mode, const float* const* __restrict__ Wrow,
+                                                       int mode, const RowPtrs<float> Wrow,
                                                        float* __restrict__ out, int r0) {
   const int lane = threadIdx.x & 31, q = lane & 3, slot = lane >> 2;
   const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -382,7 +392,7 @@ __global__ void __launch_bounds__(256) k_factors_bf16(CooShape sh, const float* 
 template <int LPE>
 __global__ void __launch_bounds__(256, 4) k_sparse_residual_f4(const int* __restrict__ idx32, const float* __restrict__ vals,
                                                             long long nnz, CooShape sh,
-                                                            const float* const* __restrict__ Wrow,
+                                                            const RowPtrs<float> Wrow,
                                                             double* __restrict__ partial) {
   constexpr int U3 = 2, UG = 2, EPW = 32 / LPE;  // entries in flight a lane (third order, others); entries a warp
   __shared__ double red[8];
@@ -487,7 +497,7 @@ __global__ void __launch_bounds__(256, 4) k_sparse_residual_f4(const int* __rest
 // ---------------------------------------------------------------------------
 template <class T>
 __global__ void __launch_bounds__(256) k_sparse_residual(const int* __restrict__ idx32, const T* __restrict__ vals,
-                                                         long long nnz, CooShape sh, const T* const* __restrict__ Wrow,
+                                                         long long nnz, CooShape sh, const RowPtrs<T> Wrow,
                                                          double* __restrict__ partial) {
   __shared__ double red[8];
   Acc<T> acc;
@@ -778,28 +788,83 @@ extern "C" int tfx_coo_sort_mode(int dtype, const int* idx32, const void* vals, 
   return TFX_STATUS_OK;
 }
 
+namespace tfx {
+
+template <class T>
+static RowPtrs<T> row_ptrs(const void* const* W_host, const void* const* W_dev, int L) {
+  RowPtrs<T> w;
+  for (int m = 0; m < TFX_MAX_ORDER; ++m) w.p[m] = W_host && m < L ? (const T*)W_host[m] : nullptr;
+  w.dev = W_host ? nullptr : (const T* const*)W_dev;
+  return w;
+}
+static bool null_row(const void* const* W_host, int L) {
+  for (int m = 0; m < L; ++m)
+    if (!W_host[m]) return true;
+  return false;
+}
+
+static int coo_mttkrp(int dtype, const int* sidx, const void* svals, long long nnz, const long long* rowptr,
+                      const CooShape& sh, int mode, const void* const* W_host, const void* const* W_dev, void* out,
+                      cudaStream_t st) {
+  const int d = sh.dims[mode], R = sh.R;
+  const int blocks = (int)std::max<long long>(1, std::min<long long>(((long long)d * 32 + 255) / 256, 16LL * sms()));
+  for (int r0 = 0; r0 < R; r0 += 16) {
+    if (dtype == TFX_F32 && R % 4 == 0 && ((unsigned long long)out & 15) == 0)
+      k_coo_mttkrp_f4<<<blocks, 256, 0, st>>>(sidx, (const float*)svals, nnz, rowptr, sh, mode,
+                                              row_ptrs<float>(W_host, W_dev, sh.L), (float*)out, r0);
+    else if (dtype == TFX_F32)
+      k_coo_mttkrp<float, 16><<<blocks, 256, 0, st>>>(sidx, (const float*)svals, nnz, rowptr, sh, mode,
+                                                      row_ptrs<float>(W_host, W_dev, sh.L), (float*)out, r0);
+    else
+      k_coo_mttkrp<double, 16><<<blocks, 256, 0, st>>>(sidx, (const double*)svals, nnz, rowptr, sh, mode,
+                                                       row_ptrs<double>(W_host, W_dev, sh.L), (double*)out, r0);
+    if (int s = launched("coo_mttkrp")) return s;
+  }
+  return TFX_STATUS_OK;
+}
+
+static int sparse_residual(int dtype, const int* idx32, const void* vals, long long nnz, const CooShape& sh,
+                           const void* const* W_host, const void* const* W_dev, double* out, void* scratch,
+                           cudaStream_t st) {
+  const int R = sh.R;
+  const int blocks = (int)std::max<long long>(1, std::min<long long>((nnz + 255) / 256, 8LL * sms()));
+  double* partial = (double*)scratch;
+  const RowPtrs<float> wf = row_ptrs<float>(W_host, W_dev, sh.L);
+  if (dtype == TFX_F32 && R % 4 == 0 && R >= 12)
+    k_sparse_residual_f4<4><<<blocks, 256, 0, st>>>(idx32, (const float*)vals, nnz, sh, wf, partial);
+  else if (dtype == TFX_F32 && R == 8)
+    k_sparse_residual_f4<2><<<blocks, 256, 0, st>>>(idx32, (const float*)vals, nnz, sh, wf, partial);
+  else if (dtype == TFX_F32 && R == 4)
+    k_sparse_residual_f4<1><<<blocks, 256, 0, st>>>(idx32, (const float*)vals, nnz, sh, wf, partial);
+  else if (dtype == TFX_F32)
+    k_sparse_residual<float><<<blocks, 256, 0, st>>>(idx32, (const float*)vals, nnz, sh, wf, partial);
+  else
+    k_sparse_residual<double><<<blocks, 256, 0, st>>>(idx32, (const double*)vals, nnz, sh,
+                                                      row_ptrs<double>(W_host, W_dev, sh.L), partial);
+  if (int s = launched("sparse_residual")) return s;
+  k_final_sum<double><<<1, 256, 0, st>>>(partial, blocks, 1, nullptr, out, nullptr);
+  return launched("final_sum");
+}
+
+}  // namespace tfx
+
 extern "C" int tfx_coo_mttkrp(int dtype, const int* sidx, const void* svals, long long nnz, const long long* rowptr,
                               int L, const int* dims, int R, int mode, const void* const* Wrow_dev, void* out,
                               void* stream) {
   CooShape sh;
   if (fill_shape(sh, L, dims, R) || mode < 0 || mode >= L || !sidx || !svals || !rowptr || !Wrow_dev || !out)
     return tfx_set_error(TFX_STATUS_ERR_ARG, "coo_mttkrp args");
-  cudaStream_t st = (cudaStream_t)stream;
-  const int d = dims[mode];
-  const int blocks = (int)std::max<long long>(1, std::min<long long>(((long long)d * 32 + 255) / 256, 16LL * sms()));
-  for (int r0 = 0; r0 < R; r0 += 16) {
-    if (dtype == TFX_F32 && R % 4 == 0 && ((unsigned long long)out & 15) == 0)
-      k_coo_mttkrp_f4<<<blocks, 256, 0, st>>>(sidx, (const float*)svals, nnz, rowptr, sh, mode,
-                                              (const float* const*)Wrow_dev, (float*)out, r0);
-    else if (dtype == TFX_F32)
-      k_coo_mttkrp<float, 16><<<blocks, 256, 0, st>>>(sidx, (const float*)svals, nnz, rowptr, sh, mode,
-                                                      (const float* const*)Wrow_dev, (float*)out, r0);
-    else
-      k_coo_mttkrp<double, 16><<<blocks, 256, 0, st>>>(sidx, (const double*)svals, nnz, rowptr, sh, mode,
-                                                       (const double* const*)Wrow_dev, (double*)out, r0);
-    if (int s = launched("coo_mttkrp")) return s;
-  }
-  return TFX_STATUS_OK;
+  return coo_mttkrp(dtype, sidx, svals, nnz, rowptr, sh, mode, nullptr, Wrow_dev, out, (cudaStream_t)stream);
+}
+
+extern "C" int tfx_coo_mttkrp_rows(int dtype, const int* sidx, const void* svals, long long nnz,
+                                   const long long* rowptr, int L, const int* dims, int R, int mode,
+                                   const void* const* Wrow, void* out, void* stream) {
+  CooShape sh;
+  if (fill_shape(sh, L, dims, R) || mode < 0 || mode >= L || !sidx || !svals || !rowptr || !Wrow ||
+      null_row(Wrow, L) || !out)
+    return tfx_set_error(TFX_STATUS_ERR_ARG, "coo_mttkrp_rows args");
+  return coo_mttkrp(dtype, sidx, svals, nnz, rowptr, sh, mode, Wrow, nullptr, out, (cudaStream_t)stream);
 }
 
 extern "C" size_t tfx_sparse_residual_scratch_bytes(void) { return (size_t)8 * (16 * 1024 + 8); }
@@ -809,27 +874,16 @@ extern "C" int tfx_sparse_residual(int dtype, const int* idx32, const void* vals
   CooShape sh;
   if (fill_shape(sh, L, dims, R) || !idx32 || !vals || !Wrow_dev || !out || !scratch)
     return tfx_set_error(TFX_STATUS_ERR_ARG, "sparse_residual args");
-  cudaStream_t st = (cudaStream_t)stream;
-  const int blocks = (int)std::max<long long>(1, std::min<long long>((nnz + 255) / 256, 8LL * sms()));
-  double* partial = (double*)scratch;
-  if (dtype == TFX_F32 && R % 4 == 0 && R >= 12)
-    k_sparse_residual_f4<4><<<blocks, 256, 0, st>>>(idx32, (const float*)vals, nnz, sh,
-                                                    (const float* const*)Wrow_dev, partial);
-  else if (dtype == TFX_F32 && R == 8)
-    k_sparse_residual_f4<2><<<blocks, 256, 0, st>>>(idx32, (const float*)vals, nnz, sh,
-                                                    (const float* const*)Wrow_dev, partial);
-  else if (dtype == TFX_F32 && R == 4)
-    k_sparse_residual_f4<1><<<blocks, 256, 0, st>>>(idx32, (const float*)vals, nnz, sh,
-                                                    (const float* const*)Wrow_dev, partial);
-  else if (dtype == TFX_F32)
-    k_sparse_residual<float><<<blocks, 256, 0, st>>>(idx32, (const float*)vals, nnz, sh, (const float* const*)Wrow_dev,
-                                                     partial);
-  else
-    k_sparse_residual<double><<<blocks, 256, 0, st>>>(idx32, (const double*)vals, nnz, sh,
-                                                      (const double* const*)Wrow_dev, partial);
-  if (int s = launched("sparse_residual")) return s;
-  k_final_sum<double><<<1, 256, 0, st>>>(partial, blocks, 1, nullptr, out, nullptr);
-  return launched("final_sum");
+  return sparse_residual(dtype, idx32, vals, nnz, sh, nullptr, Wrow_dev, out, scratch, (cudaStream_t)stream);
+}
+
+extern "C" int tfx_sparse_residual_rows(int dtype, const int* idx32, const void* vals, long long nnz, int L,
+                                        const int* dims, int R, const void* const* Wrow, double* out, void* scratch,
+                                        void* stream) {
+  CooShape sh;
+  if (fill_shape(sh, L, dims, R) || !idx32 || !vals || !Wrow || null_row(Wrow, L) || !out || !scratch)
+    return tfx_set_error(TFX_STATUS_ERR_ARG, "sparse_residual_rows args");
+  return sparse_residual(dtype, idx32, vals, nnz, sh, Wrow, nullptr, out, scratch, (cudaStream_t)stream);
 }
 
 extern "C" size_t tfx_coo_gram_scratch_bytes(long long nnz, int d) {

@@ -127,6 +127,8 @@ _EXTRA_SIGNATURES = {
     "tfx_mode_gram_tc": [_P, _LL, _I, _LL, _P, _P, _SZ, _P, _P],
     "tfx_coo_sort_mode": [_I, _P, _P, _LL, _I, POINTER(c_int), _I, _P, _P, _P, _P, _P],
     "tfx_coo_mttkrp": [_I, _P, _P, _LL, _P, _I, POINTER(c_int), _I, _I, _P, _P, _P],
+    "tfx_coo_mttkrp_rows": [_I, _P, _P, _LL, _P, _I, POINTER(c_int), _I, _I, POINTER(c_void_p), _P, _P],
+    "tfx_sparse_residual_rows": [_I, _P, _P, _LL, _I, POINTER(c_int), _I, POINTER(c_void_p), _P, _P, _P],
     "tfx_sparse_residual": [_I, _P, _P, _LL, _I, POINTER(c_int), _I, _P, _P, _P, _P],
     "tfx_coo_gram": [_I, _P, _P, _LL, _P, _P, _I, POINTER(c_int), _I, _P, _P, _SZ, _P, _P],
     "tfx_sparse_ttmc": [_I, _P, _P, _LL, _I, POINTER(c_int), POINTER(c_int), _P, _P, _P, _SZ, _P],

@@ -104,6 +104,10 @@ def _row_major_ptrs(factors_rm):
     return arr
 
 
+def _host_ptrs(X, factors_rm):
+    return (ctypes.c_void_p * X.L)(*[_dev.ptr(w) for w in factors_rm[:X.L]])
+
+
 def coo_mttkrp(X, factors_rm, mode):
     """Sparse MTTKRP ``T_(l) (KR of the other factors)`` as a (d_l, R) row-major tensor.
 
@@ -111,9 +115,9 @@ def coo_mttkrp(X, factors_rm, mode):
     rowptr, sidx, svals = X.sort_mode(mode)
     R = int(factors_rm[0].shape[1])
     out = torch.empty((X.dims[mode], R), dtype=X.vals.dtype, device=X.vals.device)
-    ptrs = _row_major_ptrs(factors_rm)
-    _lib.call("tfx_coo_mttkrp", X.dt(), _vp(sidx), _vp(svals), X.nnz, _vp(rowptr), X.L, _cint(X.dims), R, int(mode),
-              _vp(ptrs), _vp(out), _st())
+    ptrs = _host_ptrs(X, factors_rm)
+    _lib.call("tfx_coo_mttkrp_rows", X.dt(), _vp(sidx), _vp(svals), X.nnz, _vp(rowptr), X.L, _cint(X.dims), R, int(mode),
+              ptrs, _vp(out), _st())
     return out
 
 
@@ -123,8 +127,8 @@ def sparse_residual_sq(X, factors_rm):
     lib = _lib.load()
     scratch = torch.empty(int(lib.tfx_sparse_residual_scratch_bytes()), dtype=torch.uint8, device=X.vals.device)
     out = torch.empty(1, dtype=torch.float64, device=X.vals.device)
-    ptrs = _row_major_ptrs(factors_rm)
-    _lib.call("tfx_sparse_residual", X.dt(), _vp(X.idx32), _vp(X.vals), X.nnz, X.L, _cint(X.dims), R, _vp(ptrs),
+    ptrs = _host_ptrs(X, factors_rm)
+    _lib.call("tfx_sparse_residual_rows", X.dt(), _vp(X.idx32), _vp(X.vals), X.nnz, X.L, _cint(X.dims), R, ptrs,
               _vp(out), _vp(scratch), _st())
     return out
 
