@@ -7,27 +7,32 @@
 // method forms U_l^T S_(l) as Sigma V^T, and :170-173 with
 // MultilinearAlgebra.py:72-105 multilin_mult for the classic one).  The
 // contraction index d is the strided one in memory (T[p, d, q] has q
-// contiguous), so the tensor is the A operand with M = q and K = d after a
-// transposition in shared memory; U^T (n x D, n <= 64) is the B operand.
+// contiguous), so the tensor is the A operand with M = q and K = d; U^T (n x D,
+// n <= 64) is the B operand.
 // Both are split x = x_hi + x_lo (x_hi: 13 low mantissa bits cleared, exact
 // in TF32) and the product is A_hi B_hi + A_hi B_lo + A_lo B_hi, so the core
 // keeps FP32 accuracy (a single TF32 pass moved the headline CPD's final
 // error by 1%).
 //
-// A persistent CTA takes 128-wide q tiles.  Per tile the D axis runs in chunks
-// of 32:
-//   * warp 0 (producer) brings each chunk's 32 x 128 tensor tile and the
+// A persistent CTA takes 256-wide q tiles, two halves of 128 rows.  Per tile
+// the D axis runs in chunks of 32:
+//   * warp 0 (producer) brings each chunk's 32 x 256 tensor tile and the
 //     chunk's 64 x 32 block of U^T (K-major SWIZZLE_128B) by TMA into a
 //     four-stage ring (a stage is refilled once the converters read it);
-//   * warps 2-9 (converters) each take 32 rows q and half the d range of the
-//     tile and write them, split hi / lo, into the A operands (128 x 32, K-major
-//     SWIZZLE_128B: four d values as one 16-byte store, conflict-free), and
-//     split the U^T block in place of layout, into a two-stage ring;
-//   * warp 1 issues tcgen05.mma kind::tf32 (M = 128, N = 64, K = 8), three
-//     per K step, into one TMEM accumulator and commits each operand stage
+//   * warps 2-9 (converters), four to a half, take one row q a thread: its 32
+//     values, split hi / lo, go to the thread's lane of tensor memory (one
+//     column a d: the transposition costs nothing), and together they split
+//     the U^T block in place of layout into a two-stage ring of shared memory;
+//   * warp 1 issues tcgen05.mma kind::tf32 (M = 128, N = 64, K = 8; A from
+//     tensor memory), three per K step and half, and commits each operand stage
 //     back to the converters;
-//   * after a tile's last chunk the converters read the accumulator
-//     (tcgen05.ld) and store out[p, j, q0 + row] for j < n.
+//   * warps 10-13 read a finished tile's accumulators (tcgen05.ld) and store
+//     out[p, j, q0 + row] for j < n while the next tile's products go to the
+//     other pair of accumulators.
+// Tensor memory: 4 accumulators and 2 x 2 operands (hi | lo) of 64 columns.
+// With A staged in shared memory as well the chunk of 128 rows moved 1340
+// wavefronts of 128 bytes (A written and read three times, B read three times)
+// and shared memory bound the kernel: MEASURED
 // Every wait is bounded; a wait that runs out sets *err, the CTA stops, waits
 // (bounded) for its copies and products in flight and frees TMEM.
 #include <cuda.h>
@@ -42,7 +47,10 @@
 namespace tfx {
 namespace ttc {
 
-constexpr int BQ = 128, BD = 32, NJ = 64, NCW = 8, NT = 64 + 32 * NCW, TST = 4, AST = 2, DMAX = 8192;
+constexpr int BM = 128, BQ = 2 * BM, BD = 32, NJ = 64, NCW = 8, NEW = 4, NT = 64 + 32 * (NCW + NEW);
+constexpr int TST = 4, AST = 2, DMAX = 8192, TMEM_COLS = 512;
+// tensor memory columns: accumulators [buffer][half], then operands [stage][half] of BD hi and BD lo
+constexpr uint32_t TM_ACC = 0, TM_A = 2 * 2 * NJ;
 constexpr uint32_t SPIN = 1u << 26;
 constexpr uint32_t TTILE = BD * BQ * 4;      // one tensor tile, bytes
 constexpr uint32_t BCHUNK = NJ * BD * 4;     // one chunk of U^T, bytes
@@ -96,14 +104,15 @@ __device__ __forceinline__ uint64_t desc(const void* tile) {
 
 // D = F32, A = B = TF32, both K-major, M = 128, N = 64
 __host__ __device__ constexpr uint32_t idesc() {
-  return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NJ >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
+  return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NJ >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 }
 
-__device__ __forceinline__ void mma(uint32_t tmem, uint64_t a, uint64_t b, uint32_t acc) {
+// A from tensor memory (128 lanes, a column a K step), B from shared memory
+__device__ __forceinline__ void mma(uint32_t tmem, uint32_t a, uint64_t b, uint32_t acc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-      "l"(a), "l"(b), "r"(idesc()), "r"(acc)
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem),
+      "r"(a), "l"(b), "r"(idesc()), "r"(acc)
       : "memory");
 }
 
@@ -112,21 +121,31 @@ __device__ __forceinline__ void commit(uint64_t* bar) {
                : "memory");
 }
 
+// 32 columns of the warp's lanes
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+      "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]),
+      "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]),
+      "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+      : "memory");
+}
+
 __device__ __forceinline__ float hi13(float x) { return __uint_as_float(__float_as_uint(x) & 0xFFFFE000u); }
 
 struct Smem {
-  alignas(1024) unsigned char t[TST][TTILE];           // tensor tiles [32 d][128 q]
+  alignas(1024) unsigned char t[TST][TTILE];           // tensor tiles [32 d][256 q]
   alignas(1024) unsigned char u[TST][BCHUNK];          // U^T blocks, 64 rows j x 32 d (swizzled)
-  alignas(1024) unsigned char ahi[AST][BQ * 128];      // transposed tiles: 128 rows q x 32 d
-  alignas(1024) unsigned char alo[AST][BQ * 128];
   alignas(1024) unsigned char bhi[AST][BCHUNK];
   alignas(1024) unsigned char blo[AST][BCHUNK];
   alignas(8) uint64_t tfull[TST];
   alignas(8) uint64_t tfree[TST];
   alignas(8) uint64_t afull[AST];
   alignas(8) uint64_t afree[AST];
-  alignas(8) uint64_t accfull;
-  alignas(8) uint64_t accfree;
+  alignas(8) uint64_t accfull[2];
+  alignas(8) uint64_t accfree[2];
   uint32_t tmem;
   int abort;
   int tissued;    // chunks whose tensor copies the producer issued
@@ -160,8 +179,10 @@ __global__ void __launch_bounds__(NT, 1)
       mbar_init(&S.afull[s], NCW);
       mbar_init(&S.afree[s], 1);
     }
-    mbar_init(&S.accfull, 1);
-    mbar_init(&S.accfree, NCW);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&S.accfull[s], 1);
+      mbar_init(&S.accfree[s], NEW);
+    }
     S.abort = 0;
     S.tissued = 0;
     S.tconsumed = 0;
@@ -169,7 +190,9 @@ __global__ void __launch_bounds__(NT, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 64;" ::"r"(su32(&S.tmem)) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(&S.tmem)),
+                 "n"(TMEM_COLS)
+                 : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -210,35 +233,42 @@ __global__ void __launch_bounds__(NT, 1)
           S.abort = 1;
           break;
         }
-        if (c == 0 && tl > 0 && !wait_bar(&S.accfree, (uint32_t)(tl - 1) & 1u)) {
+        const int ab = tl & 1;
+        if (c == 0 && tl > 1 && !wait_bar(&S.accfree[ab], (uint32_t)(tl / 2 - 1) & 1u)) {
           atomicExch(err, 7);
           S.abort = 1;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint64_t ah = desc(S.ahi[as]), al = desc(S.alo[as]);
         const uint64_t bh = desc(S.bhi[as]), bl = desc(S.blo[as]);
+        long long p, q0;
+        tile_of(tl, p, q0);
+        const int nh = q0 + BM < sh.Q ? 2 : 1;  // a half past the end has no rows
+        for (int hf = 0; hf < nh; ++hf) {
+          const uint32_t acc = tmem + TM_ACC + (uint32_t)(ab * 2 + hf) * NJ;
+          const uint32_t ah = tmem + TM_A + (uint32_t)(as * 2 + hf) * 2 * BD, al = ah + BD;
 #pragma unroll
-        for (int pass = 0; pass < 3; ++pass) {
-          // hi*hi, hi*lo, lo*hi
-          const uint64_t da = pass == 2 ? al : ah, db = pass == 1 ? bl : bh;
+          for (int pass = 0; pass < 3; ++pass) {
+            // hi*hi, hi*lo, lo*hi
+            const uint32_t da = pass == 2 ? al : ah;
+            const uint64_t db = pass == 1 ? bl : bh;
 #pragma unroll
-          for (int kk = 0; kk < BD / 8; ++kk)
-            mma(tmem, da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2), (c > 0 || pass > 0 || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < BD / 8; ++kk)
+              mma(acc, da + (uint32_t)(kk * 8), db + (uint64_t)(kk * 2), (c > 0 || pass > 0 || kk > 0) ? 1u : 0u);
+          }
         }
         commit(&S.afree[as]);
-        if (c == DC - 1) commit(&S.accfull);
+        if (c == DC - 1) commit(&S.accfull[ab]);
         S.missued = g + 1;
       }
     }
-  } else {
-    // converters (warps 2-9): transpose, then the epilogue of each finished tile
-    const int cw = warp - 2;
-    const int qr = (cw & 3) * 32 + lane;        // the row this thread transposes
-    const int dh = cw >> 2;                     // its half of the chunk's d range
-    const int erow = 32 * (warp & 3) + lane;    // the accumulator lane it reads
+  } else if (warp < 2 + NCW) {
+    // converters (warps 2-9)
+    const int cw = warp - 2, hf = cw >> 2;
+    const uint32_t lanes = (uint32_t)(32 * (warp & 3));  // the lanes of tensor memory this warp reaches
+    const int qr = hf * BM + (int)lanes + lane;          // the row it converts
     for (int g = 0; g < nchunk; ++g) {
-      const int s = g % TST, as = g % AST, c = g % DC, tl = g / DC;
+      const int s = g % TST, as = g % AST;
       if (!wait_bar(&S.tfull[s], (uint32_t)(g / TST) & 1u)) {
         if (lane == 0) {
           atomicExch(err, 1);
@@ -251,44 +281,45 @@ __global__ void __launch_bounds__(NT, 1)
           S.abort = 1;
         }
       }
-      if (*(volatile int*)&S.abort) break;
+      if (__any_sync(0xffffffffu, *(volatile int*)&S.abort)) break;  // the whole warp: what follows is warp-wide
       if (warp == 2 && lane == 0) S.tconsumed = g + 1;
+      long long p, q0;
+      tile_of(g / DC, p, q0);
+      // U^T block: element-wise, the layout stays (the MMA reads hi and lo
+      // with the same descriptor form)
       {
-        const float* tt = reinterpret_cast<const float*>(S.t[s]);
-        const uint32_t ro = (uint32_t)qr * 128;
-#pragma unroll
-        for (int d4 = dh * (BD / 8); d4 < (dh + 1) * (BD / 8); ++d4) {
-          float4 v, h, lo;
-          v.x = tt[(4 * d4 + 0) * BQ + qr];
-          v.y = tt[(4 * d4 + 1) * BQ + qr];
-          v.z = tt[(4 * d4 + 2) * BQ + qr];
-          v.w = tt[(4 * d4 + 3) * BQ + qr];
-          h.x = hi13(v.x); lo.x = v.x - h.x;
-          h.y = hi13(v.y); lo.y = v.y - h.y;
-          h.z = hi13(v.z); lo.z = v.z - h.z;
-          h.w = hi13(v.w); lo.w = v.w - h.w;
-          const uint32_t o = ro + ((((uint32_t)d4 ^ (uint32_t)(qr & 7)) & 7u) << 4);
-          *reinterpret_cast<float4*>(S.ahi[as] + o) = h;
-          *reinterpret_cast<float4*>(S.alo[as] + o) = lo;
-        }
-        // U^T block: element-wise, the layout stays (the MMA reads hi and lo
-        // with the same descriptor form)
         const float4* u4 = reinterpret_cast<const float4*>(S.u[s]);
         float4* bh4 = reinterpret_cast<float4*>(S.bhi[as]);
         float4* bl4 = reinterpret_cast<float4*>(S.blo[as]);
-        for (int e = cw * 32 + lane; e < (int)(BCHUNK / 16); e += 32 * NCW) {
-          const float4 v = u4[e];
+#pragma unroll
+        for (int e = 0; e < (int)(BCHUNK / 16) / (32 * NCW); ++e) {
+          const float4 v = u4[e * 32 * NCW + cw * 32 + lane];
           float4 h, lo;
           h.x = hi13(v.x); lo.x = v.x - h.x;
           h.y = hi13(v.y); lo.y = v.y - h.y;
           h.z = hi13(v.z); lo.z = v.z - h.z;
           h.w = hi13(v.w); lo.w = v.w - h.w;
-          bh4[e] = h;
-          bl4[e] = lo;
+          bh4[e * 32 * NCW + cw * 32 + lane] = h;
+          bl4[e * 32 * NCW + cw * 32 + lane] = lo;
         }
       }
-      // generic-proxy writes -> visible to the tensor core's async proxy; the
-      // tensor stage goes back to the producer, the operand to the MMA warp
+      if (q0 + hf * BM < sh.Q) {  // uniform: the half has rows
+        const float* tt = reinterpret_cast<const float*>(S.t[s]) + qr;
+        uint32_t h[32], lo[32];
+#pragma unroll
+        for (int d = 0; d < BD; ++d) {
+          const float v = tt[d * BQ], vh = hi13(v);
+          h[d] = __float_as_uint(vh);
+          lo[d] = __float_as_uint(v - vh);
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");  // the operand's products were waited for
+        const uint32_t ta = tmem + (lanes << 16) + TM_A + (uint32_t)(as * 2 + hf) * 2 * BD;
+        tmem_st32(ta, h);
+        tmem_st32(ta + BD, lo);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      }
+      // the operands are visible to the tensor core; the tensor stage goes
+      // back to the producer, the operand to the MMA warp
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -296,24 +327,31 @@ __global__ void __launch_bounds__(NT, 1)
         arrive(&S.tfree[s]);
         arrive(&S.afull[as]);
       }
-      if (c == DC - 1) {
-        // the tile's accumulator: rows q0 + erow, columns j
-        if (!wait_bar(&S.accfull, (uint32_t)tl & 1u)) {
-          if (lane == 0) {
-            atomicExch(err, 3);
-            S.abort = 1;
-          }
+    }
+  } else {
+    // epilogue (warps 10-13): a tile's accumulators, rows q0 + hf * 128 + erow, columns j
+    const uint32_t lanes = (uint32_t)(32 * (warp & 3));
+    const int erow = (int)lanes + lane;
+    for (int tl = 0; tl < mytiles; ++tl) {
+      const int ab = tl & 1;
+      if (!wait_bar(&S.accfull[ab], (uint32_t)(tl / 2) & 1u)) {
+        if (lane == 0) {
+          atomicExch(err, 3);
+          S.abort = 1;
         }
-        if (*(volatile int*)&S.abort) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        long long p, q0;
-        tile_of(tl, p, q0);
-        const long long q = q0 + erow;
+      }
+      if (__any_sync(0xffffffffu, *(volatile int*)&S.abort)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      long long p, q0;
+      tile_of(tl, p, q0);
+      for (int hf = 0; hf < 2; ++hf) {
+        if (q0 + hf * BM >= sh.Q) break;
+        const long long q = q0 + hf * BM + erow;
         float* orow = out + (size_t)p * sh.n * sh.Q + q;
 #pragma unroll 1
-        for (int cc = dh * 32; cc < (dh + 1) * 32; cc += 32) {
+        for (int cc = 0; cc < NJ && cc < sh.n; cc += 32) {
           uint32_t v[32];
-          const uint32_t taddr = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)cc;
+          const uint32_t taddr = tmem + (lanes << 16) + TM_ACC + (uint32_t)(ab * 2 + hf) * NJ + (uint32_t)cc;
           asm volatile(
               "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
               "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
@@ -328,12 +366,13 @@ __global__ void __launch_bounds__(NT, 1)
 #pragma unroll
             for (int j = 0; j < 32; ++j)
               if (cc + j < sh.n) orow[(size_t)(cc + j) * sh.Q] = __uint_as_float(v[j]);
+          __syncwarp();
         }
-        // every read of the accumulator is done before the next tile's products
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) arrive(&S.accfree);
       }
+      // every read of the accumulators is done before their next products
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) arrive(&S.accfree[ab]);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -347,7 +386,7 @@ __global__ void __launch_bounds__(NT, 1)
     if (mi > 0) wait_bar(&S.afree[(mi - 1) % AST], (uint32_t)((mi - 1) / AST) & 1u);
   }
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TMEM_COLS) : "memory");
 }
 
 typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -380,7 +419,7 @@ using namespace tfx;
 
 extern "C" int tfx_ttm_tc_supported(long long P, int D, long long Q, int n) {
   return P >= 1 && P <= 0x7fffffffLL && D >= ttc::BD && D <= ttc::DMAX && D % ttc::BD == 0 && n >= 1 &&
-         n <= ttc::NJ && Q >= ttc::BQ && Q % 4 == 0 && Q <= 0x7fffffffLL;
+         n <= ttc::NJ && Q >= ttc::BM && Q % 4 == 0 && Q <= 0x7fffffffLL;
 }
 
 // S: (P, D, Q) C-order FP32, 16-byte aligned; Ut: n x D row-major (U^T),
