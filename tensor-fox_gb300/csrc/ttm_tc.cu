@@ -32,7 +32,11 @@
 // Tensor memory: 4 accumulators and 2 x 2 operands (hi | lo) of 64 columns.
 // With A staged in shared memory as well the chunk of 128 rows moved 1340
 // wavefronts of 128 bytes (A written and read three times, B read three times)
-// and shared memory bound the kernel: MEASURED
+// and shared memory bound the kernel (512^3, n 50: 230 us, 2.5 TB/s).  From
+// tensor memory it takes 165 us (3.6 TB/s; 107 without any product): an
+// instruction takes about 117 cycles whether N is 32 or 64, three a K step.  Two
+// (A_hi with both parts of B at N = 128) ran in 148 us, but the separate sum of
+// the small terms moved the core by 1e-5 of its norm.
 // Every wait is bounded; a wait that runs out sets *err, the CTA stops, waits
 // (bounded) for its copies and products in flight and frees TMEM.
 #include <cuda.h>
