@@ -362,8 +362,38 @@ __device__ __forceinline__ void cg_matvec(const int L, const int R, const int nx
   ctick(3);
   // z_l = W_l Y_l + D_l P1_l over all owned outputs of all modes at once;
   // a thread takes one row i of one mode and four owned columns
-  // (FP64: one, as above)
-  constexpr int ZC = sizeof(T) == 8 ? 1 : 4;
+  // (FP64: one, its two sums on neighbouring lanes: twice the warps, half the
+  // chain on each)
+  if constexpr (sizeof(T) == 8) {
+    const int sd = nx / R, total = 2 * ncol * sd;
+    for (int e0 = tid & ~31; e0 < total; e0 += TFX_THREADS) {
+      const int e = min(e0 + (tid & 31), total - 1), h = e & 1, o = e >> 1, c = o / sd;
+      int l = 0, i = o - c * sd;
+      while (i >= d[l]) {
+        i -= d[l];
+        ++l;
+      }
+      const int dl = d[l], ol = off[l], ncp8 = (ncol + 3) & ~3;
+      const T* v = (h ? Din : Wr) + ol + i;
+      const T* q = h ? (STAGED ? sP1o + (size_t)l * R * ncp8 + c : P1g + (size_t)l * R * R + c0 + c)
+                     : sY + (size_t)l * R * ncp8 + c;
+      const int qs = (h && !STAGED) ? R : ncp8;
+      T a = T(0);
+#pragma unroll 4
+      for (int r = 0; r < R; ++r) a = fma(v[r * dl], q[r * qs], a);
+      const T b = __shfl_xor_sync(0xffffffffu, a, 1);
+      if (!h && e0 + (tid & 31) < total) {
+        if (zloc)
+          zloc[ncol * (ol / R) + c * dl + i] = a + b;
+        else
+          zout[ol + (c0 + c) * dl + i] = a + b;
+      }
+    }
+    __syncthreads();
+    ctick(4);
+    return;
+  }
+  constexpr int ZC = 4;
   const int sumd = nx / R;
   const int ncg = (ncol + ZC - 1) / ZC;
   for (int e = tid; e < ncg * sumd; e += TFX_THREADS) {
@@ -398,8 +428,6 @@ __device__ __forceinline__ void cg_matvec(const int L, const int R, const int nx
         a2[2] = fma(dd, (T)p4.z, a2[2]);
         a2[3] = fma(dd, (T)p4.w, a2[3]);
       }
-    } else if (ZC == 1) {
-      z_cols<T, 1>(R, dl, wrow, drow, yc, ncp, p1c, p1s, a1, a2);
     } else {
       switch (cn) {
         case 1: z_cols<T, 1>(R, dl, wrow, drow, yc, ncp, p1c, p1s, a1, a2); break;
@@ -507,13 +535,21 @@ __device__ __forceinline__ int cg_team(const Team tm, const int L, const int R, 
     // global memory.  (Measured alternatives: publishing through global
     // memory and copying the full vector back from L2, by threads or by one
     // multicast bulk copy, take as long as the push.)
-    for (int l = 0; l < L; ++l) {
-      const int dl = d[l], base = off[l] + c0 * dl, n = ncol * dl, lb = ncol * (off[l] / R);
-      for (int e = tid; e < n; e += TFX_THREADS) {
-        if (STAGED) {
-          const T q = vM[lb + e] * vP[lb + e];
-          for (int rr = 0; rr < tm.size; ++rr) tm.peer(sQf, rr)[base + e] = q;
-        } else {
+    if (STAGED) {
+      for (int e = tid; e < own; e += TFX_THREADS) {
+        int l = 0, i = e;
+        while (i >= ncol * d[l]) {
+          i -= ncol * d[l];
+          ++l;
+        }
+        const int g = off[l] + c0 * d[l] + i;
+        const T q = vM[e] * vP[e];
+        for (int rr = 0; rr < tm.size; ++rr) tm.peer(sQf, rr)[g] = q;
+      }
+    } else {
+      for (int l = 0; l < L; ++l) {
+        const int dl = d[l], base = off[l] + c0 * dl, n = ncol * dl;
+        for (int e = tid; e < n; e += TFX_THREADS) {
           const int c = e / dl;
           Q[base + e] = sM[l * ncol + c] * P[base + e];
         }
@@ -529,19 +565,28 @@ __device__ __forceinline__ int cg_team(const Team tm, const int L, const int R, 
     // reference's separate reduction of the updated residual
     constexpr bool MERGED = sizeof(T) == 4;
     Acc<T> w[3];
-    const T* Qs = STAGED ? (const T*)sQf : Q;
-    for (int l = 0; l < L; ++l) {
-      const int dl = d[l], base = off[l] + c0 * dl, n = ncol * dl, lb = ncol * (off[l] / R);
-      for (int e = tid; e < n; e += TFX_THREADS) {
-        if (STAGED) {
-          const T zz = vM[lb + e] * (vz[lb + e] + vDG[lb + e] * Qs[base + e]);
-          vz[lb + e] = zz;
-          w[0].fma_(vP[lb + e], zz);
-          if (MERGED) {
-            w[1].fma_(vr[lb + e], zz);
-            w[2].fma_(zz, zz);
-          }
-        } else {
+    if (STAGED) {
+      // the own slice as one run (all modes at once: with few owned elements a
+      // loop a mode keeps them on one warp; with z's split above a CG step of
+      // 10^3, R 10, FP64 went from 7.7 to 6.4 us, of 30^3, R 20, FP32 from 5.7 to 5.0)
+      for (int e = tid; e < own; e += TFX_THREADS) {
+        int l = 0, i = e;
+        while (i >= ncol * d[l]) {
+          i -= ncol * d[l];
+          ++l;
+        }
+        const T zz = vM[e] * (vz[e] + vDG[e] * sQf[off[l] + c0 * d[l] + i]);
+        vz[e] = zz;
+        w[0].fma_(vP[e], zz);
+        if (MERGED) {
+          w[1].fma_(vr[e], zz);
+          w[2].fma_(zz, zz);
+        }
+      }
+    } else {
+      for (int l = 0; l < L; ++l) {
+        const int dl = d[l], base = off[l] + c0 * dl, n = ncol * dl;
+        for (int e = tid; e < n; e += TFX_THREADS) {
           const int c = e / dl, g = base + e;
           const T zz = sM[l * ncol + c] * (z[g] + sDG[l * ncol + c] * Q[g]);
           z[g] = zz;
