@@ -49,6 +49,9 @@
 #include "tfx_common.cuh"
 
 namespace tfx {
+int ttm_tc_narrow(const float* S, long long P, int D, long long Q, const float* Ut, int n, float* out, int* err,
+                  cudaStream_t st);
+
 namespace ttc {
 
 constexpr int BM = 128, BQ = 2 * BM, BD = 32, NJ = 64, NCW = 8, NEW = 4, NT = 64 + 32 * (NCW + NEW);
@@ -436,6 +439,11 @@ extern "C" int tfx_ttm_tc(const float* S, long long P, int D, long long Q, const
     return tfx_set_error(TFX_STATUS_ERR_UNSUPPORTED, "ttm_tc: D % 32 == 0, n <= 64, Q >= 128, Q % 4 == 0");
   if (((uintptr_t)S & 15) != 0 || ((uintptr_t)Ut & 15) != 0)
     return tfx_set_error(TFX_STATUS_ERR_ARG, "ttm_tc needs 16-byte aligned operands");
+  // 128-wide tiles in one round of the SMs, or one chunk a tile: ttm_tc_narrow.cu
+  // (both sides measured there); beyond it 256-wide tiles (P 50, D 512, Q 512, n
+  // 50: 29 us, 35 there; P 1, D 64, Q 40000, n 10: 10.9 and 12.2)
+  if (P * ((Q + ttc::BM - 1) / ttc::BM) <= ttc::sms() || D < 2 * ttc::BD)
+    return ttm_tc_narrow(S, P, D, Q, Ut, n, out, err, (cudaStream_t)stream);
   ttc::EncodeFn enc = ttc::encode_fn();
   if (!enc) return tfx_set_error(TFX_STATUS_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled unavailable");
   CUtensorMap tmap, umap;

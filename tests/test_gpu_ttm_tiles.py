@@ -1,6 +1,6 @@
-"""The tensor-core mode product at the edges of its 256-wide tiles and 128-row
-halves, with several tiles a CTA (both pairs of accumulators reused) and every
-count of chunks from one, against FP64."""
+"""The tensor-core mode product at the edges of its 128- and 256-wide tiles, on
+either side of the rule between them, with several tiles a CTA (both pairs of
+accumulators reused) and chunk counts from one, against FP64."""
 import pytest
 import torch
 
@@ -11,7 +11,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("P,D,Q,n", [(1, 32, 128, 1), (1, 64, 132, 16), (2, 96, 252, 33), (3, 32, 256, 64),
                                      (3, 160, 260, 50), (2, 64, 384, 31), (1, 128, 388, 32), (1, 512, 1000, 50),
-                                     (500, 32, 128, 5), (310, 64, 300, 40), (7, 32, 25604, 64)])
+                                     (500, 32, 128, 5), (310, 64, 300, 40), (7, 32, 25604, 64),
+                                     (160, 64, 132, 16), (100, 96, 252, 33), (60, 160, 260, 50), (152, 64, 128, 7),
+                                     (153, 64, 128, 7), (1, 512, 19460, 64), (3, 64, 25604, 1)])
 def test_product(P, D, Q, n):
     assert _lib.load().tfx_ttm_tc_supported(P, D, Q, n)
     g = torch.Generator(device="cuda").manual_seed(P + D + Q + n)
