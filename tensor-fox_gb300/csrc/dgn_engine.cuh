@@ -1839,7 +1839,7 @@ struct Engine {
     if (nmy > 1) issue(1);
     // W0[i, :] of the next slab: lane r of every warp holds columns r and
     // r + 32 (one L2 latency a slab, where a load in the loop over r cost one
-    // every other column)
+    // every other column); columns from 64 on are read as they are needed
     const int lane = tid & 31;
     T an[2] = {T(0), T(0)};
     auto load_a = [&](int t) {
@@ -1848,6 +1848,7 @@ struct Engine {
       if (lane + 32 < R) an[1] = a[(lane + 32) * d0];
     };
     if (nmy > 0) load_a(0);
+    const int RL = min(R, 64);  // columns that the lanes hold
     const int nk4 = d2p >> 2, nj4 = d1p >> 2;
     const int j4 = tid / nk4, k4 = tid - j4 * nk4;
     const bool active = tid < nj4 * nk4;  // <= 16 x 16
@@ -1883,10 +1884,12 @@ struct Engine {
           const int e = min(e0 + lane, np - 1), j = e / d2, k = e - j * d2;
           T x = T(0);
 #pragma unroll 4
-          for (int r = 0; r < R; ++r) {
+          for (int r = 0; r < RL; ++r) {
             const T ai = __shfl_sync(0xffffffffu, r < 32 ? ac[0] : ac[1], r & 31);
             x = fma(ai * sBt[r * d1p + j], sCt[r * d2p + k], x);
           }
+          for (int r = RL; r < R; ++r)
+            x = fma(Wf[off[0] + r * d0 + first + t * step] * sBt[r * d1p + j], sCt[r * d2p + k], x);
           if (e0 + lane < np) {
             const T df = slab[e] - x;
             acc.fma_(df, df);
@@ -1900,9 +1903,7 @@ struct Engine {
           for (int v = 0; v < 4; ++v) x[u][v] = T(0);
         const T* pb = sBt + (active ? 4 * j4 : 0);
         const T* pc = sCt + (active ? 4 * k4 : 0);
-#pragma unroll 4
-        for (int r = 0; r < R; ++r) {
-          const T ai = __shfl_sync(0xffffffffu, r < 32 ? ac[0] : ac[1], r & 31);
+        auto column = [&](int r, T ai) {
           T b[4], c[4];
           lds4(pb + r * d1p, b);
           lds4(pc + r * d2p, c);
@@ -1912,7 +1913,11 @@ struct Engine {
 #pragma unroll
             for (int v = 0; v < 4; ++v) x[u][v] = fma(bu, c[v], x[u][v]);
           }
-        }
+        };
+#pragma unroll 4
+        for (int r = 0; r < RL; ++r) column(r, __shfl_sync(0xffffffffu, r < 32 ? ac[0] : ac[1], r & 31));
+#pragma unroll 1
+        for (int r = RL; r < R; ++r) column(r, Wf[off[0] + r * d0 + first + t * step]);
         if (active) {
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
