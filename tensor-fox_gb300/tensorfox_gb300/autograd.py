@@ -194,7 +194,15 @@ class CPFitLoss(torch.autograd.Function):
         R = int(factors[0].shape[1])
         grads = [None] * len(factors)
         wanted = ctx.needs_input_grad[1:]
-        if any(wanted):
+        if any(wanted) and torch.is_grad_enabled() and gl.requires_grad:
+            # differentiated again (``create_graph``): scaled in torch, which
+            # records that the gradients depend on ``gl``
+            g, s = fit_grad(T, W_flat, dims, R).mul_(gl.to(T.dtype)), 0
+            for l, d in enumerate(dims):
+                if wanted[l]:
+                    grads[l] = g[s:s + d * R].view(R, d).t().to(factors[l].dtype)
+                s += d * R
+        elif any(wanted):
             lib = _declare()
             L, dt, cd = len(dims), _dt(T), _cint(dims)
             nb = int(lib.tfx_cp_fit_grad_scratch_bytes(dt, L, cd, R))
