@@ -37,13 +37,14 @@ def _cint(v):
 def _flat(factors, dtype=None):
     """The factors as one flat vector of column-major blocks, of ``dtype`` (the
     factors' own by default): one launch that reads them where they lie, whatever
-    their strides."""
+    their strides (a view whose values are still to be negated goes through torch,
+    which does that)."""
     W0 = factors[0]
     dt = W0.dtype if dtype is None else dtype
     L, R, dev = len(factors), W0.shape[-1], W0.device
     if (1 < L <= _lib.MAX_ORDER and dev.type == "cuda" and dt in (torch.float32, torch.float64) and
-            all(W.dtype == dt and W.device == dev and W.dim() == 2 and W.shape[1] == R and W.shape[0] > 0 and R > 0
-                for W in factors)):
+            all(W.dtype == dt and W.device == dev and W.dim() == 2 and W.shape[1] == R and W.shape[0] > 0 and R > 0 and
+                not W.is_neg() for W in factors)):
         lib = _declare()
         dims = [W.shape[0] for W in factors]
         out = torch.empty(R * sum(dims), dtype=dt, device=dev)
