@@ -206,7 +206,8 @@ using namespace tfx;
 
 extern "C" size_t tfx_mttkrp_all_scratch_bytes(int dtype, int L, const int* dims, int R);
 
-// the FP32 model on register-tiled column pairs (dense_kernels.cu)
+// the FP32 model on register-tiled column pairs (dense_kernels.cu); -1 where the
+// 64 x 64 tiles here are the faster form
 int tfx_cp_full_f32(int L, const int* dims, int R, const float* W, float* out, cudaStream_t st);
 
 static int nsm() {
@@ -246,13 +247,17 @@ static size_t al256(size_t v) { return (v + 255) & ~(size_t)255; }
 extern "C" int tfx_cp_full(int dtype, int L, const int* dims, int R, const void* W, void* out, void* stream) {
   CpDims sh;
   if (cpdims(sh, L, dims, R) || !W || !out) return tfx_set_error(TFX_STATUS_ERR_ARG, "cp_full args");
-  if (dtype == TFX_F32) return tfx_cp_full_f32(L, dims, R, (const float*)W, (float*)out, (cudaStream_t)stream);
+  if (dtype == TFX_F32) {
+    const int r = tfx_cp_full_f32(L, dims, R, (const float*)W, (float*)out, (cudaStream_t)stream);
+    if (r >= 0) return r;
+  }
   long long Q0 = 1;
   for (int l = 1; l < L; ++l) Q0 *= dims[l];
   const long long tiles = ((dims[0] + 63) / 64) * ((Q0 + 63) / 64);
   const int blocks = (int)std::max<long long>(1, std::min<long long>(tiles, 8LL * nsm()));
   cudaStream_t st = (cudaStream_t)stream;
-  k_cp_full<double, 4><<<blocks, TFX_THREADS, 0, st>>>((const double*)W, sh, (double*)out);
+  if (dtype == TFX_F32) k_cp_full<float, 4><<<blocks, TFX_THREADS, 0, st>>>((const float*)W, sh, (float*)out);
+  else k_cp_full<double, 4><<<blocks, TFX_THREADS, 0, st>>>((const double*)W, sh, (double*)out);
   return done("cp_full");
 }
 

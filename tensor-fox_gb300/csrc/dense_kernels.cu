@@ -794,6 +794,7 @@ __global__ void __launch_bounds__(TFX_THREADS) k_cp_residual(const T* __restrict
   const long long ntiles = (long long)tm_ * ((Q0 + TL::BN - 1) / TL::BN);
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   double part = 0.0;
+  Acc<float> part32[TS];  // FP32: squares in float-float, a chain a row
   for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int m0 = (int)(t % tm_) * TL::BM;
     const long long q0 = (t / tm_) * TL::BN;
@@ -836,12 +837,20 @@ __global__ void __launch_bounds__(TFX_THREADS) k_cp_residual(const T* __restrict
         const long long q = q0 + tx + 16 * v;
         if (m < d0 && q < Q0) {
           const T df = Tt[(long long)m * Q0 + q] - acc[u][v];
-          ps = fma(df, df, ps);
+          if constexpr (sizeof(T) == 4) part32[u].fma_(df, df);
+          else ps = fma(df, df, ps);
         }
       }
-    part += (double)ps;
+    if constexpr (sizeof(T) == 8) part += ps;
   }
-  part = warp_sum(part);
+  if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int u = 1; u < TS; ++u) part32[0].add2_(part32[u]);
+    part32[0].warp_reduce();
+    part = part32[0].value();
+  } else {
+    part = warp_sum(part);
+  }
   if ((tid & 31) == 0) red[tid >> 5] = part;
   __syncthreads();
   if (tid == 0) {
@@ -1351,20 +1360,34 @@ int tfx_cp_residual_tc_launch(const float* T, const int* dims, int R, const floa
                               int max_partials, int* err, int* nblocks, cudaStream_t st);
 
 // ---------------------------------------------------------------------------
-// The FP32 model [[W]] as a register-tiled GEMM with the Khatri-Rao operand
-// generated on the fly: subtracted from the tensor and squared, or written
-// (FULL).  A block owns 32 TN columns q of the other modes: it forms their
-// Khatri-Rao rows (up to 64 ranks at a time, shared memory), then walks its row
-// tiles of mode 0 (blockIdx.y deals them): the model tile (8 rows per warp, 8 x
-// TN outputs per lane as column pairs, as in k_ttm_f32) = W_0 (rows x R) KR^T
-// (R x columns).  The residual accumulates squares in float-float; block
-// partials are summed in FP64 by k_final_sum.  A written tile goes out through
-// shared memory, whole lines a warp whatever the row's alignment.  Bound by the
-// FP32 FMA rate and, written, by HBM: 300 x 262 x 217 at R = 40 82 us (92 with 4 x
-// 4 outputs a thread on scalar reads); residual of 187 x 143 x 95 at R = 21 22 us
-// (40 with one block a column tile, 53 of them).
+// The FP32 model [[W]], R <= 64, as a register-tiled GEMM with the Khatri-Rao
+// operand generated on the fly: subtracted from the tensor and squared, or
+// written (FULL).  A block owns 32 TN columns q of the other modes: it forms
+// their Khatri-Rao rows once (shared memory), then walks its row tiles of mode 0
+// (blockIdx.y deals them): the model tile (8 rows per warp, 8 x TN outputs per
+// lane as column pairs, as in k_ttm_f32) = W_0 (rows x R) KR^T (R x columns).  The
+// residual accumulates squares in float-float; block partials are summed in FP64
+// by k_final_sum.  A written tile goes out through shared memory, whole lines a
+// warp whatever the row's alignment.  Bound by the FP32 FMA rate and, written, by
+// HBM: 300 x 262 x 217 at R = 40 82 us (92 with 4 x 4 outputs a thread on scalar
+// reads).  Where its blocks are few, or the rows of one block do not repay its
+// Khatri-Rao rows, the 64 x 64 tiles of k_cp_full and k_cp_residual are the
+// faster form: model_tiles().
 // ---------------------------------------------------------------------------
 constexpr int RES_RMAX = 64, RES_AKS = RES_RMAX + 4;
+
+// Whether the model kernel is the faster one, from both measured at leading modes
+// of 1 to 100000, 2 to 350000 columns and ranks 1 to 200 (us, 64 x 64 tiles |
+// here).  Written, R 7: 32 x 65536 11.7 | 9.8, 16 x 65536 11.9 | 12.8; R 20: 65 x
+// 65536 26.7 | 23.5, 64 x 65536 16.4 | 16.9, 512 x 900 7.2 | 8.2; R 40: 65 x 350000
+// 213 | 170; R 65: 128 x 65536 67 | 85; R 5: 1000000 x 2 51 | 120; a leading mode of 8, R 64, 65536 columns 33
+// | 150.  Residuals: 187 x 13585 R 21 21 | 25, 300 x 65535 R 50 150 | 137 and R 70
+// 194 | 261, 8 x 65535 R 64 41 | 183.
+static bool model_tiles(int d0, long long Q0, int R) {
+  const double n = (double)d0 * (double)Q0;
+  if (Q0 < 64 || R > RES_RMAX) return false;
+  return R <= 8 ? d0 >= 8 + 3 * R && n >= 1e6 : d0 > 64 && n >= 3e6;
+}
 
 template <int TN>
 constexpr size_t model_smem(bool full) {
@@ -1384,7 +1407,7 @@ __global__ void __launch_bounds__(256, 2) k_cp_model_f32(const float* __restrict
   __shared__ double red[8];
   const int nw = blockDim.x >> 5, nt = blockDim.x;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int L = sh.L, R = sh.R, d0 = sh.d[0];
+  const int L = sh.L, R = sh.R, Rp = (R + 3) & ~3, d0 = sh.d[0];
   const int BM = 8 * nw, mt = (d0 + BM - 1) / BM;
   const int mb = mt * blockIdx.y / gridDim.y, me = mt * (blockIdx.y + 1) / gridDim.y;
   const long long qt = (Q0 + BN - 1) / BN;
@@ -1408,28 +1431,25 @@ __global__ void __launch_bounds__(256, 2) k_cp_model_f32(const float* __restrict
       for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0ull;
-      for (int rb = 0; rb < R; rb += RES_RMAX) {
-        const int rn = min(RES_RMAX, R - rb), rp = (rn + 3) & ~3;
-        __syncthreads();  // indices ready / the previous readers are done
-        if (m == mb || R > RES_RMAX)
-          for (int e = tid; e < rp * BN; e += nt) {
-            const int r = e / BN, c = e - r * BN;
-            float v = 0.f;
-            if (r < rn) {
-              v = 1.f;
-              for (int l = 1; l < L; ++l) v *= __ldg(W + sh.off[l] + (size_t)(rb + r) * sh.d[l] + sIdx[c][l]);
-            }
-            sKR[r * BN + c] = v;
+      __syncthreads();  // indices ready / the previous readers are done
+      if (m == mb)
+        for (int e = tid; e < Rp * BN; e += nt) {
+          const int r = e / BN, c = e - r * BN;
+          float v = 0.f;
+          if (r < R) {
+            v = 1.f;
+            for (int l = 1; l < L; ++l) v *= __ldg(W + sh.off[l] + (size_t)r * sh.d[l] + sIdx[c][l]);
           }
-        for (int e = tid; e < BM * rp; e += nt) {  // rows along the lanes: W_0's columns lie together
-          const int r = e / BM, i = e - r * BM;
-          sA[i * RES_AKS + r] = (m0 + i < d0 && r < rn) ? __ldg(W + (size_t)(rb + r) * d0 + m0 + i) : 0.f;
+          sKR[r * BN + c] = v;
         }
-        __syncthreads();
-#pragma unroll 1
-        for (int k4 = 0; k4 < rp; k4 += 4)
-          rows8_fma4<TN>(acc, sA + wid * 8 * RES_AKS + k4, RES_AKS, sKR + k4 * BN + lane * 4, BN);
+      for (int e = tid; e < BM * Rp; e += nt) {  // rows along the lanes: W_0's columns lie together
+        const int r = e / BM, i = e - r * BM;
+        sA[i * RES_AKS + r] = (m0 + i < d0 && r < R) ? __ldg(W + (size_t)r * d0 + m0 + i) : 0.f;
       }
+      __syncthreads();
+#pragma unroll 1
+      for (int k4 = 0; k4 < Rp; k4 += 4)
+        rows8_fma4<TN>(acc, sA + wid * 8 * RES_AKS + k4, RES_AKS, sKR + k4 * BN + lane * 4, BN);
       if (FULL) {
         float* o = sO + wid * 8 * OST;  // the warp's own rows
 #pragma unroll
@@ -1515,7 +1535,8 @@ static int launch_model_f32(const float* T, const float* W, const CpShape& sh, l
   return (int)(bx * by);
 }
 
-// cp_full for FP32 (called from autograd_kernels.cu)
+// cp_full for FP32 where the model kernel is the faster form (called from
+// autograd_kernels.cu); -1 where it is not
 int tfx_cp_full_f32(int L, const int* dims, int R, const float* W, float* out, cudaStream_t st) {
   CpShape sh;
   sh.L = L;
@@ -1528,6 +1549,7 @@ int tfx_cp_full_f32(int L, const int* dims, int R, const float* W, float* out, c
     s += dims[l];
     if (l) Q0 *= dims[l];
   }
+  if (!model_tiles(dims[0], Q0, R)) return -1;
   const int r = launch_model_f32<true>(nullptr, W, sh, Q0, nullptr, out, st);
   return r < 0 ? -r : TFX_STATUS_OK;
 }
@@ -1565,7 +1587,7 @@ static int cp_residual(int dtype, const void* Tp, int L, const int* dims, int R,
     }
     if (r != TFX_STATUS_ERR_UNSUPPORTED) return r;
   }
-  if (dtype == TFX_F32) {
+  if (dtype == TFX_F32 && model_tiles(dims[0], Q0, R)) {
     const int nb = launch_model_f32<false>((const float*)Tp, (const float*)W, sh, Q0, partial, nullptr, st);
     if (nb < 0) return -nb;
     k_final_sum<T><<<1, 256, 0, st>>>(partial, nb, 1, nullptr, out, out_t);
@@ -1573,7 +1595,10 @@ static int cp_residual(int dtype, const void* Tp, int L, const int* dims, int R,
   }
   const long long tiles = ((dims[0] + 63) / 64) * ((Q0 + 63) / 64);
   const int blocks = (int)std::max<long long>(1, std::min<long long>(tiles, 8LL * num_sms()));
-  k_cp_residual<double, 4><<<blocks, TFX_THREADS, 0, st>>>((const double*)Tp, (const double*)W, sh, partial);
+  if (dtype == TFX_F32)
+    k_cp_residual<float, 4><<<blocks, TFX_THREADS, 0, st>>>((const float*)Tp, (const float*)W, sh, partial);
+  else
+    k_cp_residual<double, 4><<<blocks, TFX_THREADS, 0, st>>>((const double*)Tp, (const double*)W, sh, partial);
   int r = check_launch("cp_residual");
   if (r) return r;
   k_final_sum<T><<<1, 256, 0, st>>>(partial, blocks, 1, nullptr, out, out_t);
