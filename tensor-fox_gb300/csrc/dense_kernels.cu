@@ -1582,7 +1582,7 @@ static int cp_residual(int dtype, const void* Tp, int L, const int* dims, int R,
     int nb = 0;
     const int r = tfx_cp_residual_tc_launch((const float*)Tp, dims, R, (const float*)W, partial, 8 * 1024, err, &nb, st);
     if (r == TFX_STATUS_OK) {
-      k_final_sum<T><<<1, 256, 0, st>>>(partial, nb, 1, err, out, out_t);
+      k_final_sum<T><<<1, final_sum_threads(nb), 0, st>>>(partial, nb, 1, err, out, out_t);
       return check_launch("final_sum");
     }
     if (r != TFX_STATUS_ERR_UNSUPPORTED) return r;
@@ -1590,7 +1590,7 @@ static int cp_residual(int dtype, const void* Tp, int L, const int* dims, int R,
   if (dtype == TFX_F32 && model_tiles(dims[0], Q0, R)) {
     const int nb = launch_model_f32<false>((const float*)Tp, (const float*)W, sh, Q0, partial, nullptr, st);
     if (nb < 0) return -nb;
-    k_final_sum<T><<<1, 256, 0, st>>>(partial, nb, 1, nullptr, out, out_t);
+    k_final_sum<T><<<1, final_sum_threads(nb), 0, st>>>(partial, nb, 1, nullptr, out, out_t);
     return check_launch("final_sum");
   }
   const long long tiles = ((dims[0] + 63) / 64) * ((Q0 + 63) / 64);
@@ -1601,7 +1601,7 @@ static int cp_residual(int dtype, const void* Tp, int L, const int* dims, int R,
     k_cp_residual<double, 4><<<blocks, TFX_THREADS, 0, st>>>((const double*)Tp, (const double*)W, sh, partial);
   int r = check_launch("cp_residual");
   if (r) return r;
-  k_final_sum<T><<<1, 256, 0, st>>>(partial, blocks, 1, nullptr, out, out_t);
+  k_final_sum<T><<<1, final_sum_threads(blocks), 0, st>>>(partial, blocks, 1, nullptr, out, out_t);
   return check_launch("final_sum");
 }
 
@@ -1632,7 +1632,7 @@ extern "C" int tfx_tensor_norms(int dtype, const void* T, long long N, double* o
     k_tensor_norms<double><<<blocks, TFX_THREADS, 0, st>>>((const double*)T, N, partial);
   int r = check_launch("tensor_norms");
   if (r) return r;
-  k_final_sum<double><<<1, 256, 0, st>>>(partial, blocks, 2, nullptr, out2, nullptr);
+  k_final_sum<double><<<1, final_sum_threads(blocks), 0, st>>>(partial, blocks, 2, nullptr, out2, nullptr);
   return check_launch("final_sum");
 }
 

@@ -842,7 +842,7 @@ static int sparse_residual(int dtype, const int* idx32, const void* vals, long l
     k_sparse_residual<double><<<blocks, 256, 0, st>>>(idx32, (const double*)vals, nnz, sh,
                                                       row_ptrs<double>(W_host, W_dev, sh.L), partial);
   if (int s = launched("sparse_residual")) return s;
-  k_final_sum<double><<<1, 256, 0, st>>>(partial, blocks, 1, nullptr, out, nullptr);
+  k_final_sum<double><<<1, final_sum_threads(blocks), 0, st>>>(partial, blocks, 1, nullptr, out, nullptr);
   return launched("final_sum");
 }
 

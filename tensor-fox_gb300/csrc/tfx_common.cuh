@@ -435,31 +435,40 @@ __device__ __forceinline__ void tile_zero(T (&acc)[TM][TN]) {
     for (int v = 0; v < TN; ++v) acc[u][v] = T(0);
 }
 
-// The sum of n partials of `stride` interleaved values each, by one CTA of 256
-// threads: thread t takes partials t, t + 256, ..., warps and then the eight
-// warp sums are added in a fixed order.  out[j] (double) and, where given,
-// out_t (the first value in the working type); *err != 0 makes them NaN.  One
-// thread walking the partials took 4 us for 300 of them and 65 us for 1216.
+// The sum of n partials of `stride` interleaved values each, by one CTA of
+// final_sum_threads(n) threads: thread t takes partials t, t + threads, ..., warps
+// and then their sums are added in a fixed order.  out[j] (double) and, where
+// given, out_t (the first value in the working type); *err != 0 makes them NaN.
+// One thread walking the partials took 4 us for 300 of them and 65 us for 1216;
+// few partials take one warp, whose FP64 adds do not queue behind idle warps'.
+inline int final_sum_threads(int n) { return n <= 128 ? 32 : 256; }
+
 template <class T>
 __global__ void __launch_bounds__(256) k_final_sum(const double* __restrict__ partial, int n, int stride,
                                                    const int* __restrict__ err, double* __restrict__ out,
                                                    T* __restrict__ out_t) {
   __shared__ double red[8];
+  const int nt = blockDim.x;
   for (int j = 0; j < stride; ++j) {
     double s = 0.0;
-    for (int i = threadIdx.x; i < n; i += 256) s += partial[(size_t)i * stride + j];
+    for (int i = threadIdx.x; i < n; i += nt) s += partial[(size_t)i * stride + j];
     s = warp_sum(s);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
+    if (nt > 32) {
+      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+      __syncthreads();
+    }
     if (threadIdx.x == 0) {
-      double t = red[0];
+      double t = s;
+      if (nt > 32) {
+        t = red[0];
 #pragma unroll
-      for (int w = 1; w < 8; ++w) t += red[w];
+        for (int w = 1; w < 8; ++w) t += red[w];
+      }
       if (err && *err) t = nan("");
       if (out) out[j] = t;
       if (out_t && j == 0) *out_t = (T)t;
     }
-    __syncthreads();
+    if (nt > 32) __syncthreads();
   }
 }
 
