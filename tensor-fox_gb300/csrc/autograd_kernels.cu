@@ -73,32 +73,39 @@ __global__ void __launch_bounds__(TFX_THREADS) k_cp_full(const T* __restrict__ W
 }
 
 // The factors as a caller has them (any strides) into the flat column-major
-// layout: 32 x 32 tiles through shared memory, read along whichever stride is
-// the shorter.
+// layout: tiles of 1024 entries through shared memory, read along whichever
+// stride is the shorter.  A tile has 2^LC columns, the fewest that hold R (up to
+// 32): with 32 x 32 tiles 27 of 32 lanes idled at R = 5 (1000000 x 5 and 2 x 5, FP32:
+// 17 us, 58 that way).
 struct PackArgs {
   const void* p[TFX_MAX_ORDER];
   long long rs[TFX_MAX_ORDER], cs[TFX_MAX_ORDER];
 };
 
-template <class T>
+template <class T, int LC>
 __global__ void __launch_bounds__(256) k_pack(const __grid_constant__ PackArgs a, const __grid_constant__ CpDims sh,
                                               T* __restrict__ out) {
-  __shared__ T tile[32][33];
-  const int R = sh.R, nr = (R + 31) / 32;
+  constexpr int TC = 1 << LC, TR = 1024 >> LC, ST = TR + (32 >> LC);
+  __shared__ T tile[TC * ST];  // [column][row]; the pad keeps a warp's rows and columns on their own banks
+  const int R = sh.R, nr = (R - 1) / TC + 1;
   int t = blockIdx.x, m = 0;
-  while (t >= (sh.d[m] + 31) / 32 * nr) t -= (sh.d[m++] + 31) / 32 * nr;
-  const int i0 = t / nr * 32, r0 = t % nr * 32, d = sh.d[m];
+  while (t >= ((sh.d[m] - 1) / TR + 1) * nr) t -= ((sh.d[m++] - 1) / TR + 1) * nr;
+  const int i0 = t / nr * TR, r0 = t % nr * TC, d = sh.d[m];
   const T* w = (const T*)a.p[m];
   const long long rs = a.rs[m], cs = a.cs[m];
-  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
   const bool along_r = cs <= rs;
-  for (int u = y; u < 32; u += 8) {
-    const int i = along_r ? u : x, r = along_r ? x : u;
-    if (i0 + i < d && r0 + r < R) tile[i][r] = w[(i0 + i) * rs + (r0 + r) * cs];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int e = threadIdx.x + 256 * u;
+    const int i = along_r ? e >> LC : e % TR, r = along_r ? e & (TC - 1) : e / TR;
+    if (i < d - i0 && r0 + r < R) tile[r * ST + i] = w[(long long)(i0 + i) * rs + (r0 + r) * cs];
   }
   __syncthreads();
-  for (int u = y; u < 32; u += 8)
-    if (i0 + x < d && r0 + u < R) out[sh.off[m] + (long long)(r0 + u) * d + i0 + x] = tile[x][u];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int e = threadIdx.x + 256 * u, i = e % TR, r = e / TR;
+    if (i < d - i0 && r0 + r < R) out[sh.off[m] + (long long)(r0 + r) * d + i0 + i] = tile[r * ST + i];
+  }
 }
 
 // Gramians of every mode, G_m = W_m^T W_m (FP64, compensated sums of the
@@ -261,21 +268,38 @@ extern "C" int tfx_cp_full(int dtype, int L, const int* dims, int R, const void*
   return done("cp_full");
 }
 
+template <class T>
+static void launch_pack(int lc, unsigned g, const PackArgs& a, const CpDims& sh, T* out, cudaStream_t st) {
+  switch (lc) {
+    case 0: k_pack<T, 0><<<g, 256, 0, st>>>(a, sh, out); break;
+    case 1: k_pack<T, 1><<<g, 256, 0, st>>>(a, sh, out); break;
+    case 2: k_pack<T, 2><<<g, 256, 0, st>>>(a, sh, out); break;
+    case 3: k_pack<T, 3><<<g, 256, 0, st>>>(a, sh, out); break;
+    case 4: k_pack<T, 4><<<g, 256, 0, st>>>(a, sh, out); break;
+    default: k_pack<T, 5><<<g, 256, 0, st>>>(a, sh, out); break;
+  }
+}
+
 extern "C" int tfx_factors_pack(int dtype, int L, const int* dims, int R, const void* const* W, const long long* rs,
                                 const long long* cs, void* out, void* stream) {
   CpDims sh;
   if (cpdims(sh, L, dims, R) || !W || !rs || !cs || !out) return tfx_set_error(TFX_STATUS_ERR_ARG, "factors_pack args");
   PackArgs a;
+  int lc = 0;
+  while (lc < 5 && (1 << lc) < R) ++lc;
+  const int tc = 1 << lc, tr = 1024 >> lc;
   long long nb = 0;
   for (int l = 0; l < L; ++l) {
     if (!W[l]) return tfx_set_error(TFX_STATUS_ERR_ARG, "factors_pack pointer");
     a.p[l] = W[l];
     a.rs[l] = rs[l];
     a.cs[l] = cs[l];
-    nb += (long long)((dims[l] + 31) / 32) * ((R + 31) / 32);
+    nb += (long long)((dims[l] - 1) / tr + 1) * ((R - 1) / tc + 1);
   }
-  if (dtype == TFX_F64) k_pack<double><<<(unsigned)nb, 256, 0, (cudaStream_t)stream>>>(a, sh, (double*)out);
-  else k_pack<float><<<(unsigned)nb, 256, 0, (cudaStream_t)stream>>>(a, sh, (float*)out);
+  const unsigned g = (unsigned)nb;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (dtype == TFX_F64) launch_pack<double>(lc, g, a, sh, (double*)out, st);
+  else launch_pack<float>(lc, g, a, sh, (float*)out, st);
   return done("factors_pack");
 }
 
