@@ -112,7 +112,9 @@ __global__ void __launch_bounds__(256) k_pack(const __grid_constant__ PackArgs a
 // working-type products).  A CTA takes a 16 x 16 block on or above the diagonal
 // of one Gramian: 32 rows of its 32 columns at a time through shared memory
 // (coalesced), four groups of threads a quarter of the rows each, added in
-// order.  512 rows, R = 50: 67 us with one thread an entry walking two columns.
+// order.  512 rows, R = 50: 17 us, 67 with one thread an entry walking two columns.
+// Rows past the end and warps past the rank are left out: the FP64 pipe takes as
+// long for zeros (4 x 4 x 4, R = 3, FP64 with the product below: 7 us, 15 with them).
 template <class T>
 __global__ void __launch_bounds__(1024) k_cp_grams(const T* __restrict__ W, CpDims sh, double* __restrict__ gram) {
   __shared__ T sa[16][129], sb[16][129];
@@ -125,6 +127,7 @@ __global__ void __launch_bounds__(1024) k_cp_grams(const T* __restrict__ W, CpDi
   }
   const int a0 = ba * 16, b0 = (ba + t) * 16, m = blockIdx.y, d = sh.d[m];
   const int tid = threadIdx.x, z = tid >> 8, a = (tid >> 4) & 15, b = tid & 15;
+  const bool on = a0 + (a & ~1) < R;  // a warp has two values of a
   const T* w = W + sh.off[m];
   Acc<T> s[2];
   for (int i0 = 0; i0 < d; i0 += 128) {
@@ -136,10 +139,19 @@ __global__ void __launch_bounds__(1024) k_cp_grams(const T* __restrict__ W, CpDi
       else sb[c - 16][i] = v;
     }
     __syncthreads();
+    const int n = on ? min(32, d - i0 - 32 * z) : 0;
+    const T *pa = sa[a] + 32 * z, *pb = sb[b] + 32 * z;
+    if (n == 32) {
 #pragma unroll 4
-    for (int i = 32 * z; i < 32 * z + 32; i += 2) {
-      s[0].fma_(sa[a][i], sb[b][i]);
-      s[1].fma_(sa[a][i + 1], sb[b][i + 1]);
+      for (int i = 0; i < 32; i += 2) {
+        s[0].fma_(pa[i], pb[i]);
+        s[1].fma_(pa[i + 1], pb[i + 1]);
+      }
+    } else {
+      for (int i = 0; i < n; i += 2) {  // an odd end takes one zero
+        s[0].fma_(pa[i], pb[i]);
+        s[1].fma_(pa[i + 1], pb[i + 1]);
+      }
     }
   }
   double v = s[0].value() + s[1].value();
