@@ -55,7 +55,10 @@ struct Plan {
 // of the least; FP64 32, its warps past the last row idle.
 // F: every other mode if they lie together and the block stays within 8 MB;
 // else the one beside the rows, and those next to it while the chunks' padding
-// is above 1/8 and the block within 4096 rows.
+// is above 1/8 and the block within 4096 rows.  Where that still pads every
+// chunk to four times its steps or more, every other mode if they lie together
+// and the block stays within 64 MB (10 x 200000 x 3 at R = 8, the first mode:
+// chunks of 3 steps took 339 us in FP32 and 458 in FP64; so 58 and 183).
 // Splits: one wave of the resident CTAs, in FP32 at least 4 chunks each.
 inline Plan plan(int es, const CpDims& sh, int g0, int g1, int sms) {
   Plan p;
@@ -76,14 +79,17 @@ inline Plan plan(int es, const CpDims& sh, int g0, int g1, int sms) {
   p.last = Q == 1;
   const int lo = p.last ? 0 : g1, hi = p.last ? g0 : L;  // the modes F may take
   const long long K = p.last ? P : Q;
-  long long dF;
-  if ((p.last || P == 1) && K * p.w.ldp * es <= (8LL << 20)) {
-    p.f0 = lo;
-    dF = K;
-  } else {
+  const bool together = p.last || P == 1;
+  long long dF = K;
+  p.f0 = lo;
+  if (!together || K * p.w.ldp * es > (8LL << 20)) {
     p.f0 = hi - 1;
     dF = sh.d[hi - 1];
     while (p.f0 > lo && ((dF + BK - 1) / BK * BK - dF) * 8 > dF && dF * sh.d[p.f0 - 1] <= 4096) dF *= sh.d[--p.f0];
+    if (together && (dF + BK - 1) / BK * BK >= 4 * dF && K * p.w.ldp * es <= (64LL << 20)) {
+      p.f0 = lo;
+      dF = K;
+    }
   }
   p.f1 = hi;
   p.w.dF = (int)dF;
