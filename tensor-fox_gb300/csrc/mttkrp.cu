@@ -204,7 +204,10 @@ struct Group {
 
 // Microseconds of the GEMM and of the contractions, from the rates measured on
 // GB300 (40 and 0.9 TFLOP/s on padded work; Khatri-Rao blocks written at 1 TB/s,
-// partials and X read at 2 TB/s; about 3 us a launch).
+// partials and X read at 2 TB/s; about 3 us a launch).  The contractions' CTAs, one
+// an index and 32 columns, take 1.5 us each however few their positions, 608 at a
+// time: beyond a few thousand they count (39 x 51351 x 4 at R = 14, the middle mode
+// from the last two 164 us, by itself 78).
 static double gemm_us(const Plan& p, int es, double N) {
   const double dp = es == 4 ? (double)p.tilesM * 32 * p.WM : (double)((p.w.D + 7) / 8 * 8);
   const double flop = 2.0 * N / p.w.D * dp * ((double)p.rowsF / p.w.dF) * p.w.ldp;
@@ -221,14 +224,16 @@ static Group group(int es, const CpDims& sh, int g0, int g1, int only, int sms) 
   g.x_bytes = g.w_bytes = 0;
   if (g1 - g0 > 1) {
     const long long D = g.p.w.D;
-    long long rows = 0, least = D;
+    long long rows = 0, idx = 0, least = D;
     for (int m = g0; m < g1; ++m)
       if (only < 0 || only == m) {
         rows += D / sh.d[m];
+        idx += sh.d[m];
         least = std::min<long long>(least, sh.d[m]);
       }
     const double per = (double)D * g.p.w.ldp * es, steps = (double)(D / least) / MY;
-    g.us += 6.0 + ((only < 0 ? g1 - g0 : 1) + 1) * per / 2e6 + 0.1 * steps;
+    const double ctas = (double)idx * ((g.p.w.ldp + 31) / 32);
+    g.us += 6.0 + ((only < 0 ? g1 - g0 : 1) + 1) * per / 2e6 + 0.1 * steps + std::max(0.0, ctas - 4096.0) * (1.5 / 608);
     if (D > 0x7fffffffLL / g.p.w.ldp) g.us = 1e30;
     g.x_bytes = (size_t)((D * g.p.w.ldp * es + 255) & ~255LL);
     g.w_bytes = (size_t)((rows * g.p.w.ldp * es + 255) & ~255LL);
