@@ -96,7 +96,8 @@ inline Plan plan(int es, const CpDims& sh, int g0, int g1, int sms) {
   p.w.nc = (int)((dF + BK - 1) / BK);
   p.rowsF = (long long)p.w.nc * BK;
   p.w.nO = P * Q / dF;
-  p.fold = p.w.nO > 1;
+  // some mode is outside, if only of size 1: its factor's row scales all the same
+  p.fold = L - (g1 - g0) - (p.f1 - p.f0) > 0;
   p.w.Q1 = p.last ? 1 : Q / dF;
   p.w.sP = p.last ? dF * D : D * Q;
   p.w.sQ = dF;
