@@ -54,6 +54,9 @@ struct Cfg {
   static constexpr int BM = 32 * WM, BN = 4 * TN;
   static constexpr int WK = 4 / WM, KW = BK / WK;
   static constexpr int CTAS = TN > 8 ? 2 : 3;
+  // chunks a chain: 512 steps a lane, and 32 where the rows are few, so that long
+  // contractions of short modes are summed in chains no longer than theirs
+  static constexpr int FC = WM == 1 ? 4 : 512 / KW;
   static constexpr int ASZ = LAST ? BK * BM : BM * AST;
   static constexpr int STG = ASZ + BK * BN + BN;  // A, KR_F rows, KR_O row
   static constexpr size_t SMEM = (size_t)STAGES * STG * 4;
@@ -219,7 +222,7 @@ __global__ void __launch_bounds__(NT, Cfg<TN, WM, LAST, FOLD>::CTAS)
           add2(sum[i][j], acc[i][j]);
           acc[i][j] = 0ull;
         }
-    } else if (++cc == nc || c + 1 == ce) {
+    } else if (++cc == nc || c + 1 == ce || cc % C::FC == 0) {
       if (cc == nc) cc = 0;
       const float* sp = A + C::ASZ + BK * C::BN;
 #pragma unroll

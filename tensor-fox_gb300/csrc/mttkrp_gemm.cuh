@@ -6,9 +6,10 @@
 // global memory (L2-resident), and the outer rest O:
 //   M[d, r] = sum_o KR_O[o, r] (sum_f T[d, o, f] KR_F[f, r]).
 // So the inner loop is a plain GEMM whose operands both arrive by cp.async, and
-// every dF steps the sums are scaled by KR_O's row and folded into a second set
-// (none in FP64 when F holds every other mode; FP32 then adds chunk by chunk).  Forming Khatri-Rao rows in the loop
-// instead cost as many instructions as the FMAs.
+// every dF steps, in FP32 at the latest after a chain's length, the sums are
+// scaled by KR_O's row and folded into a second set (none in FP64 when F holds
+// every other mode; FP32 then adds chunk by chunk).  Forming Khatri-Rao rows in
+// the loop instead cost as many instructions as the FMAs.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
