@@ -1218,18 +1218,30 @@ static void launch_ttm_f64(const double* S, long long P, int D, long long Q, con
     k_ttm_f64<TN, 4><<<dim3((unsigned)((rows + 7) / 8), by, nblk), TD_NT, 0, st>>>(S, Ut, out, n, D, Q, P, va, vb);
 }
 
+// Whether the tiles of k_ttm_f32 fill the GPU well enough for its element-wise
+// copies (shapes and pointers that 16-byte copies cannot take); else the general
+// GEMM is the faster form.  Both measured at P 1 to 400, D 3 to 394, Q 128 to 20003,
+// n 1 to 130 (us, GEMM | here): 3 x 394 x 202 n 6 8.8 | 52, 50 x 394 x 129 n 10 16
+// | 35, 1 x 33 x 5001 n 64 10.8 | 7.2, 50 x 101 x 128 n 130 24 | 12, 400 x 33 x 1943
+// n 16 272 | 79.
+static bool ttm_f32_fills(long long P, int D, long long Q, int n) {
+  const int nw = ((n < 64 ? n : 64) + 7) / 8;  // warps a CTA
+  const double t = (double)P * (double)Q / 128 * std::max(1.0, n / (8.0 * nw)), sms = num_sms();
+  return t >= sms || (t >= 0.4 * sms && (D < 32 || nw >= 2)) || (t >= 0.2 * sms && D <= 64 && nw >= 5);
+}
+
 extern "C" int tfx_ttm(int dtype, const void* S, long long P, int D, long long Q, const void* Ut, int n, void* out,
                        void* stream) {
   if (!S || !Ut || !out || P < 1 || D < 1 || Q < 1 || n < 1) return tfx_set_error(TFX_STATUS_ERR_ARG, "ttm args");
   cudaStream_t st = (cudaStream_t)stream;
   const bool vec = D % 4 == 0 && Q % 4 == 0 && ((uintptr_t)S & 15) == 0 && ((uintptr_t)Ut & 15) == 0 &&
                    ((uintptr_t)out & 15) == 0;
-  if (dtype == TFX_F32 && Q >= 128) {
+  if (dtype == TFX_F32 && Q >= 128 && (vec || ttm_f32_fills(P, D, Q, n))) {
     const int rows = n < 64 ? n : 64;
     const int nw = (rows + 7) / 8;
     const int mt = (n + 8 * nw - 1) / (8 * nw);
     // wide tiles when there are enough of them to fill the GPU twice over
-    const bool wide = ((Q + 255) / 256) * P * mt >= 2LL * num_sms();
+    const bool wide = ((Q + 255) / 256) * P * mt >= 2LL * num_sms() && (vec || Q > 128);
     const long long tq = wide ? (Q + 255) / 256 : (Q + 127) / 128;
     if (tq > 2147483647LL) return tfx_set_error(TFX_STATUS_ERR_UNSUPPORTED, "ttm too wide");
     dim3 grid((unsigned)tq, (unsigned)(P < 65535 ? P : 65535), (unsigned)mt);
