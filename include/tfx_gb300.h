@@ -152,7 +152,8 @@ int tfx_gemm(int dtype, const void* A, const void* B, void* C, long long M, long
  * for S of shape (P, D, Q) and Ut (n x D), all row-major (Compression.py:153-156,
  * the multilin_mult of MultilinearAlgebra.py:72-105 with U_l^T).  FP32 with
  * Q >= 128 and FP64 with Q = 1 or Q >= 8 run dedicated register-tiled kernels
- * (any D and n, any alignment); other shapes use tfx_gemm. */
+ * (any D, n and alignment) where they are the faster form; other shapes use
+ * tfx_gemm. */
 int tfx_ttm(int dtype, const void* S, long long P, int D, long long Q, const void* Ut, int n, void* out,
             void* stream);
 /* The same product on the tensor cores for precision 'mixed' (3xTF32: both

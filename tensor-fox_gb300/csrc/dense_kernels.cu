@@ -1218,6 +1218,26 @@ static void launch_ttm_f64(const double* S, long long P, int D, long long Q, con
     k_ttm_f64<TN, 4><<<dim3((unsigned)((rows + 7) / 8), by, nblk), TD_NT, 0, st>>>(S, Ut, out, n, D, Q, P, va, vb);
 }
 
+// Columns a lane of k_ttm_f64 (blocks of 4 TN, all as narrow as n allows), or 0
+// where the general GEMM is the faster form.  Both measured at P 1 to 3000, D 3 to
+// 300, Q 1 to 8000, n 1 to 100 (us, GEMM | 32-column blocks | 8-column blocks).
+// With 32-row tiles for two CTAs a SM: 3000 x 14 x 16 n 14 318 | 23; but few rows a
+// position against many columns, 200 x 300 x 8 n 64 61 | 104.  With fewer, the
+// columns are spread over more CTAs: 3 x 300 x 100 n 100 24 | 48 | 25, 1 x 300 x 100 n
+// 64 31 | 32 | 19; and below 32 steps the GEMM's latency is the shorter, 1 x 5 x 15 n
+// 64 2.7 | 5.7.
+static int ttm_f64_columns(long long P, int D, long long Q, int n) {
+  const long long rows = Q == 1 ? P : Q, batch = Q == 1 ? 1 : P;
+  if ((Q > 1 && Q < 8) || rows > 0x7fffffffLL) return 0;
+  const int per = (n + (n + 31) / 32 - 1) / ((n + 31) / 32);  // columns a block, at most 32
+  const int tn = per <= 8 ? 2 : per <= 16 ? 4 : per <= 24 ? 6 : 8;
+  const long long nblk = (n + 4 * tn - 1) / (4 * tn), sms = num_sms(), ctas8 = (rows + 7) / 8 * batch * nblk;
+  if ((rows + 31) / 32 * batch * nblk >= 2 * sms)
+    return Q > 1 && n > 32 && batch < 1024 && (rows <= 8 || (rows < 16 && n <= 48)) ? 0 : tn;
+  if (D < 32) return tn == 2 && ctas8 >= sms ? 2 : 0;
+  return 5 * ctas8 < 6 * sms ? 2 : tn;
+}
+
 // Whether the tiles of k_ttm_f32 fill the GPU well enough for its element-wise
 // copies (shapes and pointers that 16-byte copies cannot take); else the general
 // GEMM is the faster form.  Both measured at P 1 to 400, D 3 to 394, Q 128 to 20003,
@@ -1255,11 +1275,11 @@ extern "C" int tfx_ttm(int dtype, const void* S, long long P, int D, long long Q
     }
     return check_launch("ttm");
   }
-  if (dtype == TFX_F64 && (Q == 1 || Q >= 8) && (Q == 1 ? P : Q) <= 0x7fffffffLL) {
-    const int per = (n + (n + 31) / 32 - 1) / ((n + 31) / 32);  // columns a block, at most 32
-    if (per <= 8) launch_ttm_f64<2>((const double*)S, P, D, Q, (const double*)Ut, n, (double*)out, st);
-    else if (per <= 16) launch_ttm_f64<4>((const double*)S, P, D, Q, (const double*)Ut, n, (double*)out, st);
-    else if (per <= 24) launch_ttm_f64<6>((const double*)S, P, D, Q, (const double*)Ut, n, (double*)out, st);
+  const int tn = dtype == TFX_F64 ? ttm_f64_columns(P, D, Q, n) : 0;
+  if (tn) {
+    if (tn == 2) launch_ttm_f64<2>((const double*)S, P, D, Q, (const double*)Ut, n, (double*)out, st);
+    else if (tn == 4) launch_ttm_f64<4>((const double*)S, P, D, Q, (const double*)Ut, n, (double*)out, st);
+    else if (tn == 6) launch_ttm_f64<6>((const double*)S, P, D, Q, (const double*)Ut, n, (double*)out, st);
     else launch_ttm_f64<8>((const double*)S, P, D, Q, (const double*)Ut, n, (double*)out, st);
     return check_launch("ttm_f64");
   }
