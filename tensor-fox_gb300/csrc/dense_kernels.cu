@@ -1232,6 +1232,7 @@ static int ttm_f64_columns(long long P, int D, long long Q, int n) {
   const int per = (n + (n + 31) / 32 - 1) / ((n + 31) / 32);  // columns a block, at most 32
   const int tn = per <= 8 ? 2 : per <= 16 ? 4 : per <= 24 ? 6 : 8;
   const long long nblk = (n + 4 * tn - 1) / (4 * tn), sms = num_sms(), ctas8 = (rows + 7) / 8 * batch * nblk;
+  if (nblk > 65535) return 0;  // a grid's third dimension
   if ((rows + 31) / 32 * batch * nblk >= 2 * sms)
     return Q > 1 && n > 32 && batch < 1024 && (rows <= 8 || (rows < 16 && n <= 48)) ? 0 : tn;
   if (D < 32) return tn == 2 && ctas8 >= sms ? 2 : 0;
@@ -1256,10 +1257,11 @@ extern "C" int tfx_ttm(int dtype, const void* S, long long P, int D, long long Q
   cudaStream_t st = (cudaStream_t)stream;
   const bool vec = D % 4 == 0 && Q % 4 == 0 && ((uintptr_t)S & 15) == 0 && ((uintptr_t)Ut & 15) == 0 &&
                    ((uintptr_t)out & 15) == 0;
-  if (dtype == TFX_F32 && Q >= 128 && (vec || ttm_f32_fills(P, D, Q, n))) {
-    const int rows = n < 64 ? n : 64;
-    const int nw = (rows + 7) / 8;
-    const int mt = (n + 8 * nw - 1) / (8 * nw);
+  const int rows = n < 64 ? n : 64;
+  const int nw = (rows + 7) / 8;
+  const int mt = (n + 8 * nw - 1) / (8 * nw);
+  // (row tiles are a grid's third dimension, whose limit the GEMM does not have)
+  if (dtype == TFX_F32 && Q >= 128 && mt <= 65535 && (vec || ttm_f32_fills(P, D, Q, n))) {
     // wide tiles when there are enough of them to fill the GPU twice over
     const bool wide = ((Q + 255) / 256) * P * mt >= 2LL * num_sms() && (vec || Q > 128);
     const long long tq = wide ? (Q + 255) / 256 : (Q + 127) / 128;
