@@ -28,6 +28,7 @@ __device__ __forceinline__ void cp(void* s, const void* g, bool ok) {
                  : "memory");
 }
 __device__ __forceinline__ void fma2(f2& c, f2 a, f2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
+__device__ __forceinline__ void add2(f2& c, f2 a) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(c) : "l"(a)); }
 __device__ __forceinline__ f2 dup2(float a) {
   f2 d;
   asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(a));
@@ -160,12 +161,28 @@ __global__ void __launch_bounds__(NT, 2) k_gram_f32(const float* __restrict__ S,
     la.load(gsm + s * 2 * SZ);
     if (!diag) lb.load(gsm + s * 2 * SZ + SZ);
   };
-  // LAST: pairs of columns, 8 rows x 4 pairs; else pairs of k, 8 x 8
-  f2 acc[8][LAST ? 4 : 8];
+  // LAST: pairs of columns, 8 rows x 4 pairs, and a second set into which they
+  // are added every 512 steps of a lane (its chain would be half the split; that
+  // of a pair of k is a quarter); else pairs of k, 8 x 8
+  constexpr int FC = 32;  // chunks
+  f2 acc[8][LAST ? 4 : 8], sum[8][LAST ? 4 : 1];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < (LAST ? 4 : 8); ++j) acc[i][j] = 0ull;
+    for (int j = 0; j < (LAST ? 4 : 8); ++j) {
+      acc[i][j] = 0ull;
+      if (LAST) sum[i][j & 3] = 0ull;
+    }
+  auto fold = [&]() {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        add2(sum[i][LAST ? j : 0], acc[i][j]);
+        acc[i][j] = 0ull;
+      }
+  };
+  int left = FC;
 #pragma unroll
   for (int s = 0; s < FSTAGES - 1; ++s) {
     if (cb + s < ce) load(s);
@@ -198,6 +215,10 @@ __global__ void __launch_bounds__(NT, 2) k_gram_f32(const float* __restrict__ S,
           fma2(acc[i][3], a, b1.y);
         }
       }
+      if (--left == 0) {
+        fold();
+        left = FC;
+      }
     } else {
       const float* ap = A + (wm * 32 + lm) * FST + wk * 16;
       const float* bp = B + ln * FST + wk * 16;
@@ -219,13 +240,14 @@ __global__ void __launch_bounds__(NT, 2) k_gram_f32(const float* __restrict__ S,
     if (++stage == FSTAGES) stage = 0;
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  if (LAST) fold();
   // the second k half's sums into the first's
   float v[8][8];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int j = 0; j < (LAST ? 4 : 8); ++j) {
-      const float2 t = unpack2(acc[i][j]);
+      const float2 t = unpack2(LAST ? sum[i][j & 3] : acc[i][j]);
       if (LAST) {
         v[i][2 * (j & 3)] = t.x;
         v[i][2 * (j & 3) + 1] = t.y;
@@ -372,8 +394,8 @@ static long long tiles(int dtype, int D) {
 }
 
 // Splits: whole waves of the resident CTAs (2 a SM in FP32, 5 in FP64), at
-// least 2 (FP32) or 1 (FP64) chunks each; in FP32 a second wave where a lane's
-// chain (a quarter of the split: two k halves, two of a pair) is above 4096.
+// least 2 (FP32) or 1 (FP64) chunks each; in FP32 a second wave where a quarter of
+// the split, a lane's chain but in the last mode's form, is above 4096.
 static long long splits(int dtype, long long K, int D) {
   const long long t = tiles(dtype, D), slots = (long long)sms() * (dtype == TFX_F64 ? 5 : 2);
   long long ks = std::max<long long>(1, slots / t);
