@@ -164,7 +164,7 @@ DENSE_MTTKRP_MIN = 1 << 22
 def _engine_launch(Td, x0, R, options, prec, aliased=False, fix_mode=-1):
     """Queues one engine solve on the current stream; nothing is read back."""
     b = _Batch([Td], [x0], [R], options, prec, aliased=aliased, fix_mode=fix_mode)
-    b.launch(options.cluster or auto_cluster(tuple(Td.shape), R))
+    b.launch(options.cluster or auto_cluster(tuple(Td.shape), R), auto=not options.cluster)
     return b
 
 

@@ -66,9 +66,27 @@ def auto_cluster(dims, R, problems=1):
     return int(max(1, min(16, R, alone, share)))
 
 
-def _cluster_candidates(c, R):
-    cands = [c] + [x for x in (1, 2, 4, 8, 12, 16) if x > c and x <= max(R, 1)]
-    return [x for x in cands if x <= max(R, 1)] or [1]
+def _cluster_candidates(c, R, auto=False):
+    """Cluster sizes to try in turn: ``c``, then wider ones, whose CTAs need less
+    shared memory, and for a size that ``auto_cluster`` chose (``auto``) also
+    narrower ones, for a device that cannot schedule that many CTAs together."""
+    R = max(R, 1)
+    if auto:
+        c = max(1, min(c, R))
+    cands = [c] + [x for x in (1, 2, 4, 8, 12, 16) if x > c]
+    if auto:
+        cands += [x for x in (12, 8, 4, 2, 1) if x < c]
+    return [x for x in cands if x <= R] or [1]
+
+
+def _first_that_fits(cands, launch):
+    """The first size that ``launch`` does not refuse as unsupported."""
+    for c in cands:
+        status = launch(c)
+        if status != 5:
+            break
+    _lib.check(status)
+    return c
 
 
 class _Batch:
@@ -159,20 +177,15 @@ class _Batch:
         h = self._out[:n * (2 + 4 * self.maxiter)].cpu().numpy()
         return h[:2 * n].view(np.int32).reshape(n, 4), h[2 * n:].reshape(n, -1)
 
-    def launch(self, cluster, stream=None):
+    def launch(self, cluster, stream=None, auto=False):
+        """``auto``: ``cluster`` is auto_cluster's choice, not the caller's."""
         lib = _lib.load()
         st = _dev.stream() if stream is None else stream
-        cands = _cluster_candidates(cluster, min(self.R))
-        last = None
-        for c in cands:
-            status = lib.tfx_dgn_solve(_dev.lib_dtype(self.precision), self.desc, ctypes.c_void_p(_dev.ptr(self.d_desc)),
-                                       self.n, ctypes.byref(self.opts), c, ctypes.c_void_p(st))
-            if status == 5:      # does not fit: retry with a wider cluster
-                last = status
-                continue
-            _lib.check(status)
-            return c
-        _lib.check(last)
+        return _first_that_fits(
+            _cluster_candidates(cluster, min(self.R), auto),
+            lambda c: lib.tfx_dgn_solve(_dev.lib_dtype(self.precision), self.desc,
+                                        ctypes.c_void_p(_dev.ptr(self.d_desc)), self.n, ctypes.byref(self.opts), c,
+                                        ctypes.c_void_p(st)))
 
 
 def _precision_of(T, options):
@@ -191,8 +204,8 @@ def _precision_of(T, options):
 def dGN_device(Td, x0d, R, options, precision, cluster=None, aliased=False, fix_mode=-1):
     """Runs the engine on device-resident inputs; returns device results."""
     b = _Batch([Td], [x0d], [R], options, precision, aliased=aliased, fix_mode=fix_mode)
-    c = cluster if cluster is not None else (options.cluster or auto_cluster(Td.shape, R))
-    b.launch(c)
+    c = cluster if cluster is not None else options.cluster
+    b.launch(c or auto_cluster(Td.shape, R), auto=not c)
     return b
 
 
@@ -236,6 +249,12 @@ def _vp(t):
     return ctypes.c_void_p(_dev.ptr(t) if t is not None else None)
 
 
+def _single_candidates(cluster, dims, R):
+    if cluster is not None:
+        return [int(cluster)]
+    return _cluster_candidates(auto_cluster(dims, R), int(R), auto=True)
+
+
 def jtj_matvec(T, factors, R, v=None, damp=1.0, cluster=None, precision=None, gradient=True):
     """The solver's per-iteration products at one point, computed by the same
     device code as the solve (``tfx_jtj_matvec``): the gradient ``g`` of
@@ -251,9 +270,10 @@ def jtj_matvec(T, factors, R, v=None, damp=1.0, cluster=None, precision=None, gr
     vd = s.vec(v) if v is not None else None
     jv = torch.empty_like(s.x) if v is not None else None
     g = torch.empty_like(s.x) if gradient else None
-    c = cluster if cluster is not None else auto_cluster(s.dims, R)
-    _lib.call("tfx_jtj_matvec", _dev.lib_dtype(precision), ctypes.byref(s.desc), _vp(s.d_desc),
-              ctypes.byref(s.opts), int(c), float(damp), _vp(vd), _vp(jv), _vp(g), ctypes.c_void_p(_dev.stream()))
+    lib = _lib.load()
+    _first_that_fits(_single_candidates(cluster, s.dims, R), lambda c: lib.tfx_jtj_matvec(
+        _dev.lib_dtype(precision), ctypes.byref(s.desc), _vp(s.d_desc), ctypes.byref(s.opts), c, float(damp), _vp(vd),
+        _vp(jv), _vp(g), ctypes.c_void_p(_dev.stream())))
     s.check()
     return g, jv
 
@@ -272,10 +292,10 @@ def dogleg_steps(T, x, y, grad, jtj, error, damp, R, cluster=None, precision=Non
     yd, gd, jd = s.vec(y), s.vec(grad), s.vec(jtj)
     bx, by, bw = torch.empty_like(s.x), torch.empty_like(s.x), torch.empty_like(s.x)
     be = torch.empty(1, dtype=torch.float64, device=s.x.device)
-    c = cluster if cluster is not None else auto_cluster(s.dims, R)
-    _lib.call("tfx_dgn_dogleg", _dev.lib_dtype(precision), ctypes.byref(s.desc), _vp(s.d_desc), ctypes.byref(s.opts),
-              int(c), float(damp), float(error), _vp(yd), _vp(gd), _vp(jd), _vp(bx), _vp(by), _vp(bw), _vp(be),
-              ctypes.c_void_p(_dev.stream()))
+    lib = _lib.load()
+    _first_that_fits(_single_candidates(cluster, s.dims, R), lambda c: lib.tfx_dgn_dogleg(
+        _dev.lib_dtype(precision), ctypes.byref(s.desc), _vp(s.d_desc), ctypes.byref(s.opts), c, float(damp),
+        float(error), _vp(yd), _vp(gd), _vp(jd), _vp(bx), _vp(by), _vp(bw), _vp(be), ctypes.c_void_p(_dev.stream())))
     s.check()
     return bw, bx, by, float(be.item())
 

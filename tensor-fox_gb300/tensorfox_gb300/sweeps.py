@@ -126,7 +126,7 @@ class _Dense:
             b = _Batch([p[0] for p in problems], [p[4] for p in problems], [p[3] for p in problems], o, self.prec,
                        budgets=list(caps), aliased=alias)
             c = o.cluster or min(auto_cluster(tuple(p[2]), p[3], n) for p in problems)
-            b.launch(c)
+            b.launch(c, auto=not o.cluster)
             res = b.result.cpu().numpy()
             from . import _lib
             _lib.check_solve_status(res)
@@ -143,7 +143,7 @@ class _Dense:
                 return out
             caps = _draw_caps(o, L, n)
             b2 = _Batch([self.Td] * n, full, [p[3] for p in problems], o, self.prec, budgets=list(caps))
-            b2.launch(o.cluster or auto_cluster(self.dims, max(p[3] for p in problems), n))
+            b2.launch(o.cluster or auto_cluster(self.dims, max(p[3] for p in problems), n), auto=not o.cluster)
             res2 = b2.result.cpu().numpy()
             st2 = b2.stats.cpu().numpy()
             m = int(o.maxiter)
