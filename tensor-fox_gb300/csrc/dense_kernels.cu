@@ -931,7 +931,6 @@ __global__ void k_tensor_norms(const T* __restrict__ Tt, long long N, double* __
   }
 }
 
-// fixed-order sum of `n` partials with stride `stride` into out[0..stride)
 }  // namespace tfx
 
 // ============================================================================

@@ -759,7 +759,7 @@ struct Engine {
   int* sIdx;
   RedScratch<4>* rs4;
   RedScratch<TFX_MAX_ORDER>* rs12;
-  int flip4, flip12, flip1, flipw;
+  int flip4, flip12, flipw;
   T* sScale;
   double damp, Tsize;
   tfx_dgn_options op;
@@ -1265,7 +1265,8 @@ struct Engine {
   // columns past the end are computed all the same.  A gradient of 10^3, R 10, FP64
   // on 8 CTAs: 10 us, where columns shared out took 63; 30^3, R 20, FP32 on 16:
   // 8.4 and 27; 50^3, R 50 (in 64 x 64 tiles of both products on all 256 threads
-  // in turn, partials read row by row from the peers): 27 and 44.  // -------------------------------------------------------------------------
+  // in turn, partials read row by row from the peers): 27 and 44.
+  // -------------------------------------------------------------------------
   template <bool STAGED, int UR, int UC>
   __device__ __noinline__ void gradient_l3s() {
     long long gt = gprof ? clock64() : 0;
@@ -2240,7 +2241,6 @@ __device__ __forceinline__ void engine_setup(Engine<T, TS>& E, const tfx_dgn_pro
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   __syncthreads();
-  E.flip1 = 0;
   E.flip4 = 0;
   E.flip12 = 0;
   E.flipw = 0;

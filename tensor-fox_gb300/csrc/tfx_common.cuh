@@ -305,7 +305,8 @@ __device__ __forceinline__ void team_push_sum3_max(const Team& tm, Acc<T> (&v)[3
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   S* wslot = reinterpret_cast<S*>(&ps->warp[0][0]);
   S* tslot = reinterpret_cast<S*>(&ps->team[flip][0][0]);
-  // lanes l < n hold partials; sums and maximum over them in every lane
+  // lanes l < n hold partials; lane 0 (and those below the power of two at or
+  // above n) gets their sums and maximum
   auto fold = [&](Acc<T>(&a)[3], T& mm, int n) {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
