@@ -59,7 +59,9 @@ def auto_cluster(dims, R, problems=1):
     FP32 1.04 -> 0.71; 30^3 R 30 FP64 28.7 -> 3.7, FP32 4.3 -> 0.96 (two CTAs:
     15.8 and 2.4); 4^3 R 4 FP32 0.65 -> 0.64.  ``problems`` solved in one launch
     share the GPU's 152 SMs: no more CTAs than those, but about one CTA per 1.2
-    million multiply-adds of per-iteration MTTKRP work."""
+    million multiply-adds of per-iteration MTTKRP work.  It knows nothing of solves
+    in flight on other streams: a program that keeps the GPU full of small ones
+    sets ``options.cluster`` (one CTA is the least SM time)."""
     n = int(np.prod(dims))
     alone = 16 if n * R >= 100000 else 8
     share = max(152 // problems, n * R * len(dims) // 1200000)
