@@ -395,11 +395,15 @@ static long long tiles(int dtype, int D) {
 
 // Splits: whole waves of the resident CTAs (2 a SM in FP32, 5 in FP64), at
 // least 2 (FP32) or 1 (FP64) chunks each; in FP32 a second wave where a quarter of
-// the split, a lane's chain but in the last mode's form, is above 4096.
+// the split, a lane's chain but in the last mode's form, is above 4096; in FP64 at
+// least 4 while the tiles are within 16 waves, so that the SMs' shares of them
+// come out even (1805 x 1464: 1081 tiles 4.63 ms in one split, 3.28 in four; 3000 x
+// 1250 4.65 and 4.02, 5000 x 900 3.74 and 3.58).
 static long long splits(int dtype, long long K, int D) {
   const long long t = tiles(dtype, D), slots = (long long)sms() * (dtype == TFX_F64 ? 5 : 2);
   long long ks = std::max<long long>(1, slots / t);
   if (dtype != TFX_F64 && K / ks > 4 * 4096) ks = std::max<long long>(ks, 2 * slots / t);
+  if (dtype == TFX_F64 && t <= 16 * slots) ks = std::max<long long>(ks, 4);
   ks = std::min(ks, std::max<long long>(1, K / (BK * (dtype == TFX_F64 ? 1 : 2))));
   return std::min<long long>(ks, 1024);
 }
