@@ -1247,7 +1247,7 @@ static int ttm_f64_columns(long long P, int D, long long Q, int n) {
 static bool ttm_f32_fills(long long P, int D, long long Q, int n) {
   const int nw = ((n < 64 ? n : 64) + 7) / 8;  // warps a CTA
   const double t = (double)P * (double)Q / 128 * std::max(1.0, n / (8.0 * nw)), sms = num_sms();
-  return t >= sms || (t >= 0.4 * sms && (D < 32 || nw >= 2)) || (t >= 0.2 * sms && D <= 64 && nw >= 5);
+  return t >= sms || (t >= 0.4 * sms && nw >= 2) || (t >= 0.5 * sms && D < 32) || (t >= 0.2 * sms && D <= 64 && nw >= 5);
 }
 
 extern "C" int tfx_ttm(int dtype, const void* S, long long P, int D, long long Q, const void* Ut, int n, void* out,
