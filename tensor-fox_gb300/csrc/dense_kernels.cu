@@ -1109,10 +1109,14 @@ extern "C" int tfx_gemm(int dtype, const void* A, const void* B, void* C, long l
 // ---------------------------------------------------------------------------
 // Mode product in FP64: out[p] (n x Q) = Ut (n x D) S[p] (D x Q); Q == 1: out
 // (P x n) = S (P x D) Ut^T.  Bound by the FP64 pipe, so no padded FMAs: a warp
-// holds 8 rows (q, or p) x 4 TN columns, one output a lane and column group,
-// over the valid k only.  WK = 4: the four warps share 8 rows and take a quarter
-// of each k chunk, where 32-row CTAs would leave SMs idle.  20 x 150 x 18330: 124
-// us; 542 us when 20 of the 64 rows of the short-left-factor GEMM did work.
+// holds 8 rows (q, or p) x 8 columns, two outputs a lane, over the valid k only;
+// wider blocks pad n (predicated-off FMAs take the pipe) and leave fewer CTAs to
+// deal out (20 x 150 x 18330 123 us against 124 at 24 columns and 172 at 32, 20 x
+// 141 x 130 with 20 22 against 26, 60 x 87 x 127 with 104 118 against 211).  The
+// strips of 8 rows are dealt to the warps in turn, CTA by CTA, so that ragged
+// tiles use the SM's quarters evenly.  WK = 4: the four warps share 8 rows and
+// take a quarter of each k chunk, where 32-row CTAs would leave SMs idle.  542 us
+// for the first when 20 of the 64 rows of the short-left-factor GEMM did work.
 // ---------------------------------------------------------------------------
 constexpr int TD_BK = 32, TD_ST = TD_BK + 2, TD_NT = 128;
 
@@ -1122,11 +1126,11 @@ __device__ __forceinline__ void cp_async_bytes(void* sdst, const void* gsrc, int
   else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gsrc) : "memory");
 }
 
-template <int TN, int WK>
+template <int WK>
 __global__ void __launch_bounds__(TD_NT) k_ttm_f64(const double* __restrict__ S, const double* __restrict__ Ut,
                                                    double* __restrict__ out, int n, int D, long long Q, long long P,
                                                    int vec_a, int vec_b) {
-  constexpr int BM = 32 / WK, BN = 4 * TN;
+  constexpr int TN = 2, BM = 32 / WK, BN = 4 * TN;
   __shared__ __align__(16) double sA[2][32 * TD_ST];  // [k][BM] or, Q == 1, [row][TD_ST]
   __shared__ __align__(16) double sB[2][BN * TD_ST];  // [column][TD_ST]
   __shared__ double red[WK > 1 ? 3 * BN * 8 : 1];
@@ -1134,7 +1138,7 @@ __global__ void __launch_bounds__(TD_NT) k_ttm_f64(const double* __restrict__ S,
   const bool rowk = Q == 1;
   const long long rows = rowk ? P : Q, m0 = (long long)blockIdx.x * BM;
   const int n0 = blockIdx.z * BN, nn = min(BN, n - n0);
-  const int strip = WK > 1 ? 0 : ((warp + blockIdx.x) & 3);
+  const int strip = WK > 1 ? 0 : ((warp + blockIdx.x + blockIdx.y + blockIdx.z) & 3);
   const bool on = m0 + 8 * strip < rows;
   const int nch = (D + TD_BK - 1) / TD_BK;
   for (long long p = blockIdx.y; p < (rowk ? 1 : P); p += gridDim.y) {
@@ -1204,38 +1208,25 @@ __global__ void __launch_bounds__(TD_NT) k_ttm_f64(const double* __restrict__ S,
   }
 }
 
-template <int TN>
-static void launch_ttm_f64(const double* S, long long P, int D, long long Q, const double* Ut, int n, double* out,
-                           cudaStream_t st) {
-  const long long rows = Q == 1 ? P : Q, batch = Q == 1 ? 1 : P;
-  const int nblk = (n + 4 * TN - 1) / (4 * TN);
-  const int va = ((uintptr_t)S & 15) == 0 && (Q == 1 ? D : Q) % 2 == 0, vb = ((uintptr_t)Ut & 15) == 0 && D % 2 == 0;
-  const unsigned by = (unsigned)std::min<long long>(batch, 65535);
-  if ((rows + 31) / 32 * batch * nblk >= 2LL * num_sms())
-    k_ttm_f64<TN, 1><<<dim3((unsigned)((rows + 31) / 32), by, nblk), TD_NT, 0, st>>>(S, Ut, out, n, D, Q, P, va, vb);
-  else
-    k_ttm_f64<TN, 4><<<dim3((unsigned)((rows + 7) / 8), by, nblk), TD_NT, 0, st>>>(S, Ut, out, n, D, Q, P, va, vb);
-}
-
-// Columns a lane of k_ttm_f64 (blocks of 4 TN, all as narrow as n allows), or 0
-// where the general GEMM is the faster form.  Both measured at P 1 to 3000, D 3 to
-// 300, Q 1 to 8000, n 1 to 100 (us, GEMM | 32-column blocks | 8-column blocks).
-// With 32-row tiles for two CTAs a SM: 3000 x 14 x 16 n 14 318 | 23; but few rows a
-// position against many columns, 200 x 300 x 8 n 64 61 | 104.  With fewer, the
-// columns are spread over more CTAs: 3 x 300 x 100 n 100 24 | 48 | 25, 1 x 300 x 100 n
-// 64 31 | 32 | 19; and below 32 steps the GEMM's latency is the shorter, 1 x 5 x 15 n
-// 64 2.7 | 5.7.
-static int ttm_f64_columns(long long P, int D, long long Q, int n) {
-  const long long rows = Q == 1 ? P : Q, batch = Q == 1 ? 1 : P;
-  if ((Q > 1 && Q < 8) || rows > 0x7fffffffLL) return 0;
-  const int per = (n + (n + 31) / 32 - 1) / ((n + 31) / 32);  // columns a block, at most 32
-  const int tn = per <= 8 ? 2 : per <= 16 ? 4 : per <= 24 ? 6 : 8;
-  const long long nblk = (n + 4 * tn - 1) / (4 * tn), sms = num_sms(), ctas8 = (rows + 7) / 8 * batch * nblk;
-  if (nblk > 65535) return 0;  // a grid's third dimension
-  if ((rows + 31) / 32 * batch * nblk >= 2 * sms)
-    return Q > 1 && n > 32 && batch < 1024 && (rows <= 8 || (rows < 16 && n <= 48)) ? 0 : tn;
-  if (D < 32) return tn == 2 && ctas8 >= sms ? 2 : 0;
-  return 5 * ctas8 < 6 * sms ? 2 : tn;
+// WK of k_ttm_f64, or 0 where the general GEMM is the faster form.  Both measured
+// at P 1 to 3000, D 3 to 300, Q 1 to 9000, n 1 to 160 (us, GEMM | here).  32-row
+// tiles for two CTAs a SM: 3000 x 14 x 16 n 14 318 | 23, 60 x 87 x 127 n 104 162 |
+// 118; but few rows a position against many columns, 200 x 300 x 8 n 64 61 | 104.
+// 8-row ones where those leave SMs idle (1 x 300 x 100 n 64 31 | 19) or are ragged,
+// from 32 steps on, which the warps share (60 x 150 x 33 n 20 21, 37 in 32-row
+// ones; 2000 x 10 x 33 n 100 161 in 32-row ones, 375); with few CTAs and below 32
+// steps the GEMM's latency is the shorter, 1 x 5 x 15 n 64 2.7 | 5.7.
+static int ttm_f64_form(long long P, int D, long long Q, int n) {
+  const long long rows = Q == 1 ? P : Q, batch = Q == 1 ? 1 : P, nblk = (n + 7) / 8, sms = num_sms();
+  if ((Q > 1 && Q < 8) || rows > 0x7fffffffLL || nblk > 65535) return 0;
+  const long long r32 = (rows + 31) / 32, r8 = (rows + 7) / 8;
+  if (r32 * batch * ((n + 31) / 32) >= 2 * sms) {
+    if (Q > 1 && n > 32 && batch < 1024 && (rows <= 12 || (rows < 16 && n <= 48))) return 0;
+  } else if (D < 32 && (n > 8 || r8 * batch < sms)) {
+    return 0;
+  }
+  const bool ragged = rows > 32 && r32 * 20 > r8 * 6;  // a fifth more rows than 8-row tiles have
+  return r32 * batch * nblk >= 2 * sms && !(ragged && D >= 32) ? 1 : 4;
 }
 
 // Whether the tiles of k_ttm_f32 fill the GPU well enough for its element-wise
@@ -1276,12 +1267,15 @@ extern "C" int tfx_ttm(int dtype, const void* S, long long P, int D, long long Q
     }
     return check_launch("ttm");
   }
-  const int tn = dtype == TFX_F64 ? ttm_f64_columns(P, D, Q, n) : 0;
-  if (tn) {
-    if (tn == 2) launch_ttm_f64<2>((const double*)S, P, D, Q, (const double*)Ut, n, (double*)out, st);
-    else if (tn == 4) launch_ttm_f64<4>((const double*)S, P, D, Q, (const double*)Ut, n, (double*)out, st);
-    else if (tn == 6) launch_ttm_f64<6>((const double*)S, P, D, Q, (const double*)Ut, n, (double*)out, st);
-    else launch_ttm_f64<8>((const double*)S, P, D, Q, (const double*)Ut, n, (double*)out, st);
+  if (const int wk = dtype == TFX_F64 ? ttm_f64_form(P, D, Q, n) : 0) {
+    const double *u = (const double*)Ut, *x = (const double*)S;
+    const long long rows64 = Q == 1 ? P : Q;
+    const unsigned by = (unsigned)std::min<long long>(Q == 1 ? 1 : P, 65535), bz = (unsigned)((n + 7) / 8);
+    const int va = ((uintptr_t)S & 15) == 0 && (Q == 1 ? D : Q) % 2 == 0, vb = ((uintptr_t)Ut & 15) == 0 && D % 2 == 0;
+    if (wk == 1)
+      k_ttm_f64<1><<<dim3((unsigned)((rows64 + 31) / 32), by, bz), TD_NT, 0, st>>>(x, u, (double*)out, n, D, Q, P, va, vb);
+    else
+      k_ttm_f64<4><<<dim3((unsigned)((rows64 + 7) / 8), by, bz), TD_NT, 0, st>>>(x, u, (double*)out, n, D, Q, P, va, vb);
     return check_launch("ttm_f64");
   }
   // general shapes: strided batched GEMM, batched over p (Q >= 16) or over q

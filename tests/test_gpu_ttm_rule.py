@@ -31,7 +31,8 @@ def test_f32(P, D, Q, n, shift):
 
 F64 = [(3, 5, 15, 18), (1, 14, 15, 40), (1, 31, 33, 70), (1, 32, 33, 70), (200, 14, 24, 1), (60, 14, 8, 8),
        (200, 40, 8, 33), (200, 40, 8, 32), (200, 40, 15, 48), (200, 40, 15, 49), (1100, 33, 8, 64), (3, 300, 100, 100),
-       (20, 300, 33, 64), (3000, 33, 1, 14), (5, 100, 1, 64), (1, 7, 1, 1), (1, 40, 9000, 9)]
+       (20, 300, 33, 64), (3000, 33, 1, 14), (300, 40, 12, 33), (300, 40, 13, 49), (300, 40, 33, 9), (60, 40, 100, 30),
+       (60, 87, 127, 104), (5, 100, 1, 64), (1, 7, 1, 1), (1, 40, 9000, 9)]
 
 
 @pytest.mark.parametrize("shift", [0, 1])
